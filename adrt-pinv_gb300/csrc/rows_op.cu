@@ -1,0 +1,326 @@
+// Row operators: one pass G (the op lists [B_1] P M [B_1^*] of the hybrid's G_h and of the L_p frame operator,
+// fastops.py:277-281, 325-331) on the packed rows as one small real matrix per frequency instead of d_k fused Gram
+// passes.
+//
+// The operator of frequency k is T_k = B_1^* M p_k(M) B_1 (or M p_k(M)), M = A^* A with A_{s,c} = z_k^{off(s,c)} over
+// the digital lines. A line of slope s and its complement N-1-s have offsets that add up to c, so conjugating T_k with
+// the half-shift phases D = diag(z_k^{c/2}) makes it REAL: T_k = D^* R_k D. Reversing a line, off(s, N-1-c) =
+// s - off(s, c), makes R_k centro-symmetric: R_k(N-1-c, N-1-j) = R_k(c, j). So with H = N/2, a = D y,
+//     E_j = a_j + a_{N-1-j},  O_j = a_j - a_{N-1-j},   e = T_e E,  o = T_o O   (two real H x H matrices)
+//     z_c = conj(D_c) (e_c + o_c),   z_{N-1-c} = conj(D_{N-1-c}) (e_c - o_c)        (c, j < H)
+// and R_{-k} = R_k with D conjugated, so the rows k and L-k of both quadrant pairs of every image share one pair of
+// matrices: 4 B complex vectors per frequency 0 < k < N (2 B at k = 0 and N, which are their own negatives). A row
+// costs N^2/2 complex-by-real multiply-adds (N^2 real FMAs) whatever its degree; the polynomial needs
+// 4 N (n - 1) FMAs per Gram and d_k of them (mean degree 7 at N = 256: 100 k against 66 k), and the filter's
+// ill-conditioned rows lose nothing to the recurrence, because the matrices are evaluated in FP64 when the plan's
+// tables are built.
+//
+// Two kernels, both in place (a CTA reads whole rows before it writes them):
+//  rows_op_small  few vectors (and FP64): bounded by reading the matrices (N^2/2 values per frequency, 34 MB in FP32
+//                 at N = 256, L2 resident) and by latency, so a CTA takes a frequency and at most 8 vectors, its
+//                 256 threads split the sum over j, every matrix value is read once per CTA straight into registers
+//                 (coalesced over c) and the partial sums meet in shared memory.
+//  rows_op_tile   many vectors (FP32): bounded by the FP32 pipe; a CTA keeps E and O of 4096 / H vectors in shared
+//                 memory, streams the matrices through a cp.async ring and each thread owns an 8 x 8 tile of both
+//                 products (128 FMAs per eight 16-byte shared loads), so e_c and o_c meet in registers.
+#include "common.cuh"
+#include "launch.h"
+
+namespace adrt {
+
+template <int n> struct OpCfg {
+    static constexpr int N = 1 << n, H = N / 2, L = 2 * N;
+};
+
+// vector v of frequency k: image, packed row and whether the row is that of -k (its phases are conjugated)
+struct OpVec {
+    int img, row;
+    bool neg;
+};
+template <int n> __device__ __forceinline__ OpVec op_vec(int k, int v) {
+    constexpr int N = 1 << n, L = 2 * N;
+    OpVec r;
+    const bool self = (k == 0 || k == N);
+    r.img = self ? v >> 1 : v >> 2;
+    r.neg = !self && (v & 2);
+    r.row = (v & 1) * L + (r.neg ? L - k : k);
+    return r;
+}
+
+template <typename C> __device__ __forceinline__ C conj_if(C a, bool c) {
+    if (c) a.y = -a.y;
+    return a;
+}
+
+// E and O of VT vectors (zero beyond nv) into shared memory as [j][vector] complex, row stride RS complex
+template <typename real, int n, int VT, int THREADS, int RS>
+__device__ __forceinline__ void op_load(const cplx<real>* __restrict__ Y, long long img_stride,
+                                        const cplx<real>* __restrict__ half, int k, int v0, int nv, cplx<real>* E,
+                                        cplx<real>* O) {
+    using C = cplx<real>;
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H, MASK = 2 * OpCfg<n>::L - 1;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < VT * H; e += THREADS) {
+        const int v = e / H, c = e % H;
+        C a = mk<real>(0, 0), b = mk<real>(0, 0);
+        if (v0 + v < nv) {
+            const OpVec w = op_vec<n>(k, v0 + v);
+            const C* y = Y + (long long)w.img * img_stride + (long long)w.row * N;
+            a = cmul(conj_if(half[(k * c) & MASK], w.neg), y[c]);
+            b = cmul(conj_if(half[(k * (N - 1 - c)) & MASK], w.neg), y[N - 1 - c]);
+        }
+        E[c * RS + v] = cadd(a, b);
+        O[c * RS + v] = csub(a, b);
+    }
+}
+
+// ------------------------------------------------------------------ few vectors, or FP64
+template <typename real, int n, int VT>
+__global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __restrict__ T, cplx<real>* Y,
+                                                     long long img_stride, const cplx<real>* __restrict__ half) {
+    using C = cplx<real>;
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H, MASK = 2 * OpCfg<n>::L - 1;
+    constexpr int CG = H / 4;              // groups of four outputs c
+    constexpr int KS = CG >= 256 ? 1 : 256 / CG;  // slices of the sum over j
+    constexpr int VB = VT < 4 ? VT : 4;    // vectors per reduction round
+    static_assert(CG * KS == 256, "256 threads");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* E = reinterpret_cast<C*>(smem_raw);  // [H][VT]
+    C* O = E + H * VT;
+    C* red = O + H * VT;                    // [KS][2][VB][H]
+    const int k = blockIdx.y, v0 = blockIdx.x * VT;
+    const int nv = nimg * ((k == 0 || k == N) ? 2 : 4);
+    if (v0 >= nv) return;
+    op_load<real, n, VT, 256, VT>(Y, img_stride, half, k, v0, nv, E, O);
+    __syncthreads();
+
+    const int cg = threadIdx.x % CG, ks = threadIdx.x / CG;
+    const real* Te = T + (size_t)k * 2 * H * H + 4 * cg;
+    const real* To = Te + (size_t)H * H;
+    C ae[4][VT], ao[4][VT];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int v = 0; v < VT; ++v) ae[q][v] = ao[q][v] = mk<real>(0, 0);
+    struct alignas(4 * sizeof(real)) R4 { real q[4]; };
+#pragma unroll 4
+    for (int j = ks; j < H; j += KS) {
+        const R4 te = *reinterpret_cast<const R4*>(Te + (size_t)j * H), to = *reinterpret_cast<const R4*>(To + (size_t)j * H);
+#pragma unroll
+        for (int v = 0; v < VT; ++v) {
+            const C ev = E[j * VT + v], ov = O[j * VT + v];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                ae[q][v].x = fma(te.q[q], ev.x, ae[q][v].x);
+                ae[q][v].y = fma(te.q[q], ev.y, ae[q][v].y);
+                ao[q][v].x = fma(to.q[q], ov.x, ao[q][v].x);
+                ao[q][v].y = fma(to.q[q], ov.y, ao[q][v].y);
+            }
+        }
+    }
+#pragma unroll
+    for (int vb = 0; vb < VT; vb += VB) {
+        if (vb) __syncthreads();
+#pragma unroll
+        for (int v = 0; v < VB; ++v)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                red[((ks * 2 + 0) * VB + v) * H + 4 * cg + q] = ae[q][vb + v];
+                red[((ks * 2 + 1) * VB + v) * H + 4 * cg + q] = ao[q][vb + v];
+            }
+        __syncthreads();
+        for (int e = threadIdx.x; e < VB * H; e += 256) {
+            const int v = e / H, c = e % H;
+            if (v0 + vb + v >= nv) break;
+            C se = red[v * H + c], so = red[(VB + v) * H + c];
+#pragma unroll
+            for (int s = 1; s < KS; ++s) {
+                se = cadd(se, red[((s * 2 + 0) * VB + v) * H + c]);
+                so = cadd(so, red[((s * 2 + 1) * VB + v) * H + c]);
+            }
+            const OpVec w = op_vec<n>(k, v0 + vb + v);
+            C* y = Y + (long long)w.img * img_stride + (long long)w.row * N;
+            y[c] = cmul(conj_if(half[(k * c) & MASK], !w.neg), cadd(se, so));
+            y[N - 1 - c] = cmul(conj_if(half[(k * (N - 1 - c)) & MASK], !w.neg), csub(se, so));
+        }
+    }
+}
+
+// ------------------------------------------------------------------ many vectors, FP32
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+template <int n> struct OpTile {
+    static constexpr int H = OpCfg<n>::H;
+    static constexpr int VT = 4096 / H;      // vectors per CTA (2 VT real columns)
+    static constexpr int CGS = H / 8;        // groups of 8 outputs (two runs of 4, H/2 apart)
+    static constexpr int VGS = VT / 4;       // groups of 4 vectors (two pairs, VT/2 apart)
+    static constexpr int THREADS = CGS * VGS;
+    static constexpr int RS = VT + 2;        // row stride of E and O (complex)
+    static constexpr int KC = 8;             // matrix rows per stage
+    static constexpr int STAGES = 3;
+    static constexpr int STAGE = 2 * KC * H;  // floats: KC rows of T_e, then of T_o
+    static constexpr size_t smem = (size_t)2 * H * RS * sizeof(float2) + (size_t)STAGES * STAGE * sizeof(float);
+};
+
+template <int n>
+__global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
+    rows_op_tile(int nimg, const float* __restrict__ T, float2* Y, long long img_stride, const float2* __restrict__ half) {
+    using W = OpTile<n>;
+    constexpr int N = OpCfg<n>::N, H = W::H, VT = W::VT, RS = W::RS, KC = W::KC, S = W::STAGES;
+    constexpr int MASK = 2 * OpCfg<n>::L - 1, NCH = H / KC;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* ring = reinterpret_cast<float*>(smem_raw);
+    float2* E = reinterpret_cast<float2*>(ring + S * W::STAGE);
+    float2* O = E + H * RS;
+    const int k = blockIdx.y, v0 = blockIdx.x * VT;
+    const int nv = nimg * ((k == 0 || k == N) ? 2 : 4);
+    if (v0 >= nv) return;
+    const float* Tk = T + (size_t)k * 2 * H * H;
+    auto fetch = [&](int ch) {
+        if (ch < NCH) {
+            float* st = ring + (ch % S) * W::STAGE;
+            for (int e = 4 * threadIdx.x; e < W::STAGE; e += 4 * W::THREADS) {
+                const int par = e / (KC * H), r = e % (KC * H);
+                cp16(st + e, Tk + (size_t)par * H * H + (size_t)ch * KC * H + r);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int ch = 0; ch < S - 1; ++ch) fetch(ch);
+    op_load<float, n, VT, W::THREADS, RS>(Y, img_stride, half, k, v0, nv, E, O);
+
+    const int cg = threadIdx.x % W::CGS, vg = threadIdx.x / W::CGS;
+    const int c0 = 4 * cg, u0 = 2 * vg;
+    float2 ae[8][4], ao[8][4];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) ae[q][v] = ao[q][v] = make_float2(0.f, 0.f);
+    for (int ch = 0; ch < NCH; ++ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        __syncthreads();  // stage ch has landed for every thread; stage ch - 1 may be refilled
+        fetch(ch + S - 1);
+        const float* st = ring + (ch % S) * W::STAGE;
+#pragma unroll
+        for (int jj = 0; jj < KC; ++jj) {
+            const int j = ch * KC + jj;
+            float te[8], to[8];
+            *reinterpret_cast<float4*>(te) = *reinterpret_cast<const float4*>(st + jj * H + c0);
+            *reinterpret_cast<float4*>(te + 4) = *reinterpret_cast<const float4*>(st + jj * H + H / 2 + c0);
+            *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(st + (KC + jj) * H + c0);
+            *reinterpret_cast<float4*>(to + 4) = *reinterpret_cast<const float4*>(st + (KC + jj) * H + H / 2 + c0);
+            float2 ev[4], ov[4];
+            *reinterpret_cast<float4*>(ev) = *reinterpret_cast<const float4*>(E + j * RS + u0);
+            *reinterpret_cast<float4*>(ev + 2) = *reinterpret_cast<const float4*>(E + j * RS + VT / 2 + u0);
+            *reinterpret_cast<float4*>(ov) = *reinterpret_cast<const float4*>(O + j * RS + u0);
+            *reinterpret_cast<float4*>(ov + 2) = *reinterpret_cast<const float4*>(O + j * RS + VT / 2 + u0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    ae[q][v].x = fmaf(te[q], ev[v].x, ae[q][v].x);
+                    ae[q][v].y = fmaf(te[q], ev[v].y, ae[q][v].y);
+                    ao[q][v].x = fmaf(to[q], ov[v].x, ao[q][v].x);
+                    ao[q][v].y = fmaf(to[q], ov[v].y, ao[q][v].y);
+                }
+        }
+    }
+    // z_c and z_{N-1-c}: two runs of four consecutive outputs per vector, 16-byte stores
+#pragma unroll
+    for (int run = 0; run < 2; ++run) {
+        const int cr = run * (H / 2) + c0;
+        float2 pa[4], pb[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            pa[q] = half[(k * (cr + q)) & MASK];
+            pb[q] = half[(k * (N - 1 - cr - q)) & MASK];
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const int vec = v0 + (v >> 1) * (VT / 2) + u0 + (v & 1);
+            if (vec >= nv) continue;
+            const OpVec w = op_vec<n>(k, vec);
+            float2* y = Y + (long long)w.img * img_stride + (long long)w.row * N;
+            float2 za[4], zb[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                za[q] = cmul(conj_if(pa[q], !w.neg), cadd(ae[run * 4 + q][v], ao[run * 4 + q][v]));
+                zb[q] = cmul(conj_if(pb[q], !w.neg), csub(ae[run * 4 + q][v], ao[run * 4 + q][v]));
+            }
+            float4* lo = reinterpret_cast<float4*>(y + cr);
+            lo[0] = make_float4(za[0].x, za[0].y, za[1].x, za[1].y);
+            lo[1] = make_float4(za[2].x, za[2].y, za[3].x, za[3].y);
+            float4* hi = reinterpret_cast<float4*>(y + (N - 4 - cr));
+            hi[0] = make_float4(zb[3].x, zb[3].y, zb[2].x, zb[2].y);
+            hi[1] = make_float4(zb[1].x, zb[1].y, zb[0].x, zb[0].y);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ dispatch
+template <typename real, int n, int VT>
+static int launch_small(int nimg, const void* T, void* Y, long long img_stride, const void* half, cudaStream_t st) {
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H;
+    constexpr int KS = 1024 / H, VB = VT < 4 ? VT : 4;
+    const size_t smem = (size_t)(2 * H * VT + KS * 2 * VB * H) * sizeof(cplx<real>);
+    auto kern = rows_op_small<real, n, VT>;
+    if (int rc = ensure_smem((const void*)kern, smem)) return rc;
+    kern<<<dim3((4 * nimg + VT - 1) / VT, N + 1), 256, smem, st>>>(nimg, reinterpret_cast<const real*>(T),
+                                                                   reinterpret_cast<cplx<real>*>(Y), img_stride,
+                                                                   reinterpret_cast<const cplx<real>*>(half));
+    return launch_status("rows_op_small");
+}
+
+template <int n>
+static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, const void* half, cudaStream_t st) {
+    using W = OpTile<n>;
+    auto kern = rows_op_tile<n>;
+    if (int rc = ensure_smem((const void*)kern, W::smem)) return rc;
+    kern<<<dim3((4 * nimg + W::VT - 1) / W::VT, W::H * 2 + 1), W::THREADS, W::smem, st>>>(
+        nimg, reinterpret_cast<const float*>(T), reinterpret_cast<float2*>(Y), img_stride,
+        reinterpret_cast<const float2*>(half));
+    return launch_status("rows_op_tile");
+}
+
+template <int n>
+static int rows_operator_n(int dtype, int nimg, const void* T, void* Y, long long img_stride, const void* half,
+                           cudaStream_t st) {
+    if (dtype == ADRT_F64) {
+        if (nimg == 1) return launch_small<double, n, 2>(nimg, T, Y, img_stride, half, st);
+        return launch_small<double, n, 4>(nimg, T, Y, img_stride, half, st);
+    }
+    if (nimg == 1) return launch_small<float, n, 4>(nimg, T, Y, img_stride, half, st);
+    if (4 * nimg <= OpTile<n>::VT / 2) return launch_small<float, n, 8>(nimg, T, Y, img_stride, half, st);
+    return launch_tile<n>(nimg, T, Y, img_stride, half, st);
+}
+
+int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride, const void* half,
+                  cudaStream_t st) {
+    if ((dtype != ADRT_F32 && dtype != ADRT_F64) || n < 6 || n > 9 || nimg < 0 || nimg > 65535 ||
+        (nimg && (!T || !Y || !half))) {
+        set_error("rows_operator: bad arguments (dtype=%d n=%d nimg=%d; n must be 6..9)", dtype, n, nimg);
+        return ADRT_EINVAL;
+    }
+    if ((reinterpret_cast<uintptr_t>(Y) & 15) || (reinterpret_cast<uintptr_t>(T) & 15) || (img_stride & 1)) {
+        set_error("rows_operator: T and Y must be 16-byte aligned with an even image stride");
+        return ADRT_EINVAL;
+    }
+    if (!nimg) return ADRT_OK;
+    switch (n) {
+        case 6: return rows_operator_n<6>(dtype, nimg, T, Y, img_stride, half, st);
+        case 7: return rows_operator_n<7>(dtype, nimg, T, Y, img_stride, half, st);
+        case 8: return rows_operator_n<8>(dtype, nimg, T, Y, img_stride, half, st);
+        default: return rows_operator_n<9>(dtype, nimg, T, Y, img_stride, half, st);
+    }
+}
+
+}  // namespace adrt
+
+extern "C" int adrt_rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride,
+                                  const void* half_roots, void* stream) {
+    return adrt::rows_operator(dtype, n, nimg, T, Y, img_stride, half_roots, adrt::as_stream(stream));
+}

@@ -91,6 +91,10 @@ class RowTables:
         # polynomial rows (FP64 is accurate enough there)
         self.high_poly = getattr(plan, "high_rows", "dense") == "ff" and len(plan.dense_freqs) > 0
         self.high_ff = self.high_poly and real == torch.float32
+        # one pass G as a real operator per frequency (op_table), where the plan and the size allow it
+        self.row_ops = row_operators_for(plan)
+        self._g_ops = fuse_ops(_op_lists(plan)["G"])
+        self._op_dev = self._half = None
         if self.high_ff:
             # the compensated rows read the roots of unity and the filter constants in FP64
             self.roots64 = torch.from_numpy(roots_of_unity(plan.L)).to(device=device, dtype=torch.complex128)
@@ -121,15 +125,49 @@ class RowTables:
         j.grid = self.row_grid
         return j
 
-    def _timed_main(self, Y, ops, st):
+    def _timed(self, ops, fn):
         if self.timer is None:
-            C.call("adrt_rows_run", ctypes.byref(self.job(Y, ops, self.rows_main)), st)
+            fn()
             return
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
-        C.call("adrt_rows_run", ctypes.byref(self.job(Y, ops, self.rows_main)), st)
+        fn()
         e1.record()
         self.timer.append((e0, e1, ops))
+
+    def _timed_main(self, Y, ops, st):
+        self._timed(ops, lambda: C.call("adrt_rows_run", ctypes.byref(self.job(Y, ops, self.rows_main)), st))
+
+    def runs_operators(self, ops):
+        """Whether run() applies this op list as one real operator per frequency (the G list of the plan)."""
+        return self.row_ops and fuse_ops(ops) == self._g_ops
+
+    def op_table(self):
+        """The plan's row operators (row_operator_table) in the row precision, shared by the plan's pipelines of that
+        precision while any of them holds it; None during a stream capture that finds it not built (the polynomial
+        rows run instead)."""
+        if self._op_dev is None:
+            shared = self.plan.__dict__.setdefault("_dense_shared", weakref.WeakValueDictionary())
+            key = (str(self.device), str(self.real), "row_ops")
+            T = shared.get(key)
+            if T is None:
+                if torch.cuda.is_current_stream_capturing():
+                    return None
+                T = row_operator_table(self, self.real)
+                torch.cuda.current_stream(self.device).synchronize()  # complete before another stream shares it
+                shared[key] = T
+            self._op_dev = T
+        if self._half is None:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            self._half = torch.from_numpy(roots_of_unity(2 * self.plan.L)).to(device=self.device, dtype=_cdtype(self.real))
+        return self._op_dev
+
+    def run_operators(self, Y, T):
+        """Y[b, r] <- T_k Y[b, r] for every packed row (adrt_rows_operator), in place."""
+        B, R, N = Y.shape
+        C.call("adrt_rows_operator", self.code, self.plan.n, B, C.ptr(T), C.ptr(Y), R * N, C.ptr(self._half),
+               C.stream_handle())
 
     def main_level_rows(self, ops):
         """Level-rows processed by the polynomial-row launch of one op list (the dense rows excluded)."""
@@ -233,11 +271,18 @@ class RowTables:
         filter (fastops.py:100-117), fused with the butterflies around it (adjoint levels before, Gram levels and
         the level-1 butterflies of the hybrid around it) into one precomputed operator per row; with compensated
         high rows (plan.high_rows == "ff") they keep the polynomial filter in float-float arithmetic instead.
-        skip_main: the polynomial rows (main_job) were run by the caller; only the rest is done here."""
+        skip_main: the polynomial rows (main_job) were run by the caller; only the rest is done here.
+        The plan's own G list runs as one real operator per frequency, dense rows included, where row_ops is set."""
         ops = fuse_ops(ops)
         B = Y.shape[0]
         if not ops:
             return
+        if not skip_main and self.row_ops and ops == self._g_ops:
+            T = self.op_table()
+            if T is not None:
+                self._timed(ops, lambda: self.run_operators(Y, T))
+                self.count += B * self.plan.level_rows(ops_unfused(ops))
+                return
         st = C.stream_handle()
         pidx = [i for i, o in enumerate(ops) if o[0] == "P"]
         if len(pidx) > 1:
@@ -306,6 +351,82 @@ def _rows_apply_f64(X, z_rows, ops, n, counter):
         j.op[i], j.lo[i], j.hi[i] = OPCODE[op], lo, hi
     j.counter, j.grid = counter.data_ptr(), 0
     C.call("adrt_rows_run", ctypes.byref(j), st)
+
+
+# sizes whose G pass runs as row operators: above, the operators outgrow what a lane should hold (17 GB at N = 2048);
+# below, the polynomial rows are a few microseconds of latency
+ROW_OPS_MIN, ROW_OPS_MAX = 6, 9
+
+
+def row_operators_for(plan: Plan):
+    """Whether a pass G of this plan runs as one real operator per frequency: the operators of k and -k are conjugates
+    only if the bounds and degrees are symmetric, and plans that asked for no operator memory (compensated high rows)
+    keep the polynomial."""
+    idx = (-np.arange(plan.L)) % plan.L
+    return (ROW_OPS_MIN <= plan.n <= ROW_OPS_MAX and getattr(plan, "high_rows", "dense") == "dense"
+            and np.array_equal(plan.deg, plan.deg[idx]) and np.array_equal(plan.lam_max, plan.lam_max[idx]))
+
+
+def row_operator_bytes(plan: Plan, real):
+    """Device bytes of a plan's row operators and of their half-shift phases in one precision."""
+    return (plan.N + 1) * plan.N * plan.N // 2 * real.itemsize + 4 * plan.N * 2 * real.itemsize
+
+
+def row_operator_table(tables, real):
+    """The operators of one pass G, (N + 1, 2, H, H) real, H = N/2, frequencies k = 0..N: with D = diag(z_k^(c/2)) the
+    operator T_k of an op list is D^* R_k D with R_k real and centro-symmetric (csrc/rows_op.cu), and the two blocks are
+    (P + Q)/2 and (P - Q)/2, P(c, j) = R_k(c, j), Q(c, j) = R_k(N-1-c, j), stored [j][c]. Evaluated in FP64: the columns
+    T_k e_j, j < H, by the FP64 row kernels on unit vectors (polynomial rows), or from the exact dense operators."""
+    plan, dev = tables.plan, tables.device
+    n, N, L, H = plan.n, plan.N, plan.L, plan.N // 2
+    out = torch.empty((N + 1, 2, H, H), dtype=real, device=dev)
+    half = torch.from_numpy(roots_of_unity(2 * L)).to(dev)
+
+    def phases(k):  # z_k^(c/2) for frequencies k (K,) and every c
+        return half[(k[:, None] * torch.arange(N, device=dev)[None, :]) % (2 * L)]
+
+    def store(k, j0, cols):  # cols (J, K, N): T_k e_j for j = j0.. and frequencies k
+        D = phases(k)
+        R = (cols * D[None] * D[:, j0:j0 + cols.shape[0]].T.conj()[:, :, None]).real
+        P, Q = R[..., :H], R[..., H:].flip(-1)
+        out[k, 0, j0:j0 + cols.shape[0]] = (0.5 * (P + Q)).transpose(0, 1).to(real)
+        out[k, 1, j0:j0 + cols.shape[0]] = (0.5 * (P - Q)).transpose(0, 1).to(real)
+
+    dense = plan.dense_freqs[plan.dense_freqs <= N]
+    poly = np.setdiff1d(np.arange(N + 1), dense)
+    poly = poly[np.argsort(-plan.deg[poly], kind="stable")]  # costliest rows first
+    if len(poly):
+        t64 = tables if tables.real == torch.float64 else RowTables(plan, torch.float64, dev)
+        kp = torch.from_numpy(poly).to(dev)
+        rows = torch.arange(len(poly), dtype=torch.int32, device=dev)
+        # the rows of a unit vector are stored by position in `poly`: frequency tables in that order
+        deg, coef = t64.deg[kp], t64.coef.reshape(L, -1)[kp].contiguous()
+        tab = torch.empty((len(poly), N // 2 + 1), dtype=torch.complex128, device=dev)
+        z = torch.from_numpy(roots_of_unity(L)[poly]).to(dev)
+        C.call("adrt_twiddle_table", C.F64, n, len(poly), C.ptr(z), C.ptr(tab), C.stream_handle())
+        step = max(1, min(H, (1 << 28) // (len(poly) * N * 16)))  # about 256 MB of rows at a time
+        for j0 in range(0, H, step):
+            J = min(step, H - j0)
+            X = torch.zeros((J, len(poly), N), dtype=torch.complex128, device=dev)
+            X[torch.arange(J, device=dev), :, torch.arange(j0, j0 + J, device=dev)] = 1
+            job = t64.job(X, tables._g_ops, rows)
+            job.freq_mod, job.roots, job.twtab = len(poly), None, tab.data_ptr()
+            job.deg, job.coef = deg.data_ptr(), coef.data_ptr()
+            C.call("adrt_rows_run", ctypes.byref(job), C.stream_handle())
+            store(kp, j0, X)
+    if len(dense):
+        b1 = plan.method == "hybrid"
+        sel = torch.from_numpy(np.nonzero(plan.dense_freqs <= N)[0]).to(dev)
+        freqs = torch.from_numpy(plan.dense_freqs).to(dev)
+        if n >= 9 and dev.type == "cuda":
+            chunks = dense_row_operator_device(plan, False, True, b1, b1, dev)
+        else:
+            chunks = [(0, torch.from_numpy(np.ascontiguousarray(plan.dense_row_operator(False, True, b1, b1))).to(dev))]
+        for c0, T in chunks:
+            hit = sel[(sel >= c0) & (sel < c0 + T.shape[0])]
+            if len(hit):
+                store(freqs[hit], 0, T[hit - c0][:, :, :H].permute(2, 0, 1))
+    return out
 
 
 def _load_torch_linalg():
@@ -431,7 +552,7 @@ class Pipeline:
         q.__dict__.update(self.__dict__)
         q.B = b
         t = RowTables(self.plan, self.real, self.device)
-        for k in ("stream_dense", "use_tc", "split_dense", "row_grid", "dense_tile"):
+        for k in ("stream_dense", "use_tc", "split_dense", "row_grid", "dense_tile", "row_ops"):
             setattr(t, k, getattr(self.tables, k))
         q.tables = t
         q.Y = self.Y[:b]
@@ -578,6 +699,7 @@ class Pipeline:
         bufs += [T._adrt_split for T in t._dense_dev.values() if getattr(T, "_adrt_split", None) is not None]
         if t.high_ff:
             bufs += [t.roots64, t.coef64]
+        bufs += [x for x in (t._op_dev, t._half) if x is not None]
         if t._zd is not None:
             bufs.append(t._zd)
         for name in ("b_in", "b_in2"):
@@ -594,8 +716,8 @@ class Pipeline:
     @staticmethod
     def estimate_bytes(plan: Plan, batch, precision="fp32", stencil_precision=None, captured=True):
         """Device bytes a pipeline for (plan, batch, precision) holds once it has run apply (and capture, which adds
-        the two input buffers): the buffers of __init__, the two folded dense-row tables (filter of G and of the
-        backprojection) and the dense-row staging, computed without allocating anything."""
+        the two input buffers): the buffers of __init__, the row operators of G (or its folded dense-row table), the
+        back-projection's folded dense-row table and the dense-row staging, computed without allocating anything."""
         N, L, B = plan.N, plan.L, int(batch)
         rs = PRECISIONS[precision].itemsize
         ss = STENCIL_PRECISIONS[stencil_precision or precision].itemsize
@@ -608,9 +730,12 @@ class Pipeline:
         if ff:  # FP64 roots and coefficients of the compensated rows instead of dense operators
             total += L * 16 + plan.coef.size * 8
         else:
-            total += 2 * nd * N * N * 2 * rs + nd * B * N * 2 * rs
+            lists = 1 if row_operators_for(plan) else 2  # op lists with dense tables: G has its row operators instead
+            total += lists * nd * N * N * 2 * rs + nd * B * N * 2 * rs
             if precision == "fp32" and B > 16 and 7 <= plan.n <= 10:  # their pre-split tensor-core form (in place)
-                total += 2 * nd * N * N * 16 - nd * B * N * 2 * rs
+                total += lists * nd * N * N * 16 - nd * B * N * 2 * rs
+            if lists == 1:
+                total += row_operator_bytes(plan, PRECISIONS[precision])
         total += L * 2 * rs + 3 * L * 4 + plan.coef.size * rs  # roots; deg and the row lists; coefficients
         if captured:  # the two input buffers of the captured graphs
             total += 2 * B * 4 * (2 * N - 1) * N * 8
@@ -762,10 +887,10 @@ class Pipeline:
         C.call("adrt_pack_fft", self._codes(), p.n, self.B, 1 if sino else 0, C.dtype_code(src.dtype), C.ptr(src),
                stride, C.ptr(self.Y), C.ptr(self.tables.roots), self.fft_cols, st)
 
-    def finish_pass(self, ops):
+    def finish_pass(self, ops, skip_main=True):
         """Everything of a packed pass after the polynomial-row launch: the dense (or compensated) rows, the inverse
-        FFT and the unpack into the partial images."""
-        self.tables.run(self.Y, ops, skip_main=True)
+        FFT and the unpack into the partial images (skip_main=False: the polynomial rows or row operators too)."""
+        self.tables.run(self.Y, ops, skip_main=skip_main)
         self._unpack(C.stream_handle())
 
 

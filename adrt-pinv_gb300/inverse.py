@@ -113,6 +113,8 @@ class _GpuInverse:
             outer = self._outer_interval(eps)
         self.plan.set_outer(outer)
         self.lo, self.hi, self.outer_deg = self.plan.lo, self.plan.hi, self.plan.outer_deg
+        if precision == "fp32":
+            self._pipes.pop((1, "fp64"), None)  # the setup's FP64 pipeline and its tables are not kept
         self.eng.count = [0]
 
     # ---------------------------------------------------------------- device pipelines

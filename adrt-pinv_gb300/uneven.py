@@ -68,7 +68,8 @@ class UnevenBatch:
 
 
 class PersistentUnevenBatch:
-    """Uneven batch whose polynomial rows run in ONE persistent launch per outer step.
+    """Uneven batch whose polynomial rows run in ONE persistent launch per outer step (the back-projection of every class,
+    and the G passes of the classes that do not run them as row operators).
 
     All classes step through the outer iteration together (class c takes D_c steps; it drops out once they are
     done): at every step each class packs its images (or, at step 0, its sinograms) on its own stream, then one
@@ -123,11 +124,13 @@ class PersistentUnevenBatch:
             return (raw, torch.tensor(codes, dtype=torch.int32, device=self.device),
                     torch.tensor(starts, dtype=torch.int32, device=self.device), len(jobs))
 
+        # classes whose G pass runs as row operators launch it themselves; the others share the persistent launch
+        self.own_rows = [p.tables.runs_operators(p.ops["G"]) for p in self.pipes]
         self.counter = torch.zeros(4, dtype=torch.int32, device=self.device)
         self.job_sets = {("BP", None): job_set("BP", self.order)}
         for s in range(1, max(self.D)):
-            act = tuple(i for i in self.order if self.D[i] > s)
-            if ("G", act) not in self.job_sets:
+            act = tuple(i for i in self.order if self.D[i] > s and not self.own_rows[i])
+            if act and ("G", act) not in self.job_sets:
                 self.job_sets[("G", act)] = job_set("G", act)
         self.streams = [torch.cuda.Stream(device=self.device) for _ in self.pipes]
         cap = torch.cuda.Stream(device=self.device)
@@ -187,7 +190,7 @@ class PersistentUnevenBatch:
             def finish_g(i, s=s):
                 p = self.pipes[i]
                 x, xp, free = state[i]
-                p.finish_pass(p.ops["G"])
+                p.finish_pass(p.ops["G"], skip_main=not self.own_rows[i])
                 om_a, om_1 = self.coeffs[i][2][s - 1]
                 xn = free.pop(0)
                 p.next_step(p.y, x, xp, xn, om_a, om_1)
@@ -196,7 +199,9 @@ class PersistentUnevenBatch:
                 state[i] = [xn, x, free]
 
             self._fork(cap, act, pack_g)
-            self._rows(("G", act), cap)
+            shared = tuple(i for i in act if not self.own_rows[i])
+            if shared:
+                self._rows(("G", shared), cap)
             self._fork(cap, act, finish_g)
         return [self.pipes[i].result(state[i][0]) for i in range(len(self.pipes))]
 

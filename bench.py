@@ -11,9 +11,9 @@ stencil and FP64 with the others. Metric: whole-job reconstructions per second. 
           an instrumented eager pass before it gives the per-kernel timings, the launch count and `eager`.
   e2e   : the public API FastHybridGpu.apply on pinned host sinograms into a pinned host result every step (H2D + D2H
           inside the timed region; consecutive calls overlap a batch's copy with the previous batch's graph).
-  roofline : the row engine (rows_prog_kernel), the dominant kernel, timed live with CUDA events on its stream;
-          algorithmic FLOPs = level-rows x 8N (the reference's cost unit, fastops.py:166); peak = FP32 FMA
-          throughput measured in this run by the library's probe kernel.
+  roofline : the row engine's G_h launch, the dominant kernel, timed live with CUDA events on its stream; algorithmic
+          FLOPs = 2 N^2 per packed row (row operators) or level-rows x 8N (polynomial rows, the reference's cost unit,
+          fastops.py:166); peak = FP32 FMA throughput measured in this run by the library's probe kernel.
   cpu_baseline : the reference's C++-engine path (FastHybridCpp semantics: C row kernels + NumPy) timed on this
           host's cores on one image of the same workload, same plan.
   extras (one-GPU runs, --no-extras to skip): preconditioner_ff / _fp32 (the other preconditioner precision),
@@ -372,7 +372,9 @@ def run_ours(args):
 
     g_ms = [a.elapsed_time(b) for a, b, ops in timer if ops == fuse_ops(pipe.ops["G"])]
     rows_launch_ms = float(np.mean(g_ms)) if g_ms else None
-    flops_per_launch = pipe.tables.main_level_rows(pipe.ops["G"]) * B * 8 * N
+    # row operators: N^2 real FMAs per packed row (two half-size real matrices on complex rows); polynomial rows: 8N per level-row
+    operators = pipe.tables.runs_operators(pipe.ops["G"])
+    flops_per_launch = B * 4 * N * 2 * N * N if operators else pipe.tables.main_level_rows(pipe.ops["G"]) * B * 8 * N
 
     # ---- end to end through the public API with pinned host buffers
     b_host = torch.empty(b_dev.shape, dtype=b_dev.dtype, pin_memory=True)
@@ -416,8 +418,9 @@ def run_ours(args):
     if rows_launch_ms:
         achieved = flops_per_launch / (rows_launch_ms * 1e-3) / 1e12
         tr = traffic_per_launch()  # captured at N=256, batch 64; rows scale with the batch
-        tr = tr * B / 64 if tr is not None and n == 8 else None
-        line["roofline"] = {"bound": "fp32", "kernel": "rows_prog_kernel (G_h op list, polynomial rows)",
+        tr = tr * B / 64 if tr is not None and n == 8 and not operators else None
+        line["roofline"] = {"bound": "fp32", "kernel": "rows_op_tile (G_h as one real operator per frequency)" if operators
+                            else "rows_prog_kernel (G_h op list, polynomial rows)",
                             "achieved": achieved, "peak": peak / 1e12, "unit": "TFLOP/s", "frac": achieved * 1e12 / peak,
                             "peak_source": "measured in this run: FP32 FMA probe kernel",
                             "flop_per_launch": flops_per_launch, "launch_ms": rows_launch_ms,

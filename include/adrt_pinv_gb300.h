@@ -124,6 +124,14 @@ int adrt_rows_lanes_per_row(int n);
 int adrt_rows_run_multi(const adrt_row_job* jobs, const int32_t* code, const int32_t* wstart, int njobs,
                         int32_t* counter, int grid, void* stream);
 
+/* One pass G on every packed row (2L rows per image, copies of the L frequencies stacked) as one real operator per
+ * frequency: T (N+1 x 2 x N/2 x N/2, dtype) holds for k = 0..N the blocks (P + Q)/2 and (P - Q)/2, [j][c], of the
+ * centro-symmetric R_k = D T_k D^*, D = diag(z_k^(c/2)), P(c,j) = R_k(c,j), Q(c,j) = R_k(N-1-c,j), c, j < N/2;
+ * half_roots: 4N roots exp(2 pi i j / 4N) (dtype). Rows k and L-k share T_k. In place on Y (16-byte aligned, img_stride
+ * even, complex elements). 6 <= n <= 9. */
+int adrt_rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride,
+                       const void* half_roots, void* stream);
+
 /* Per-row twiddle table tab[k*(N/2+1) + t] = z_k^t (t = 0..N/2) from K complex z (FP64 in, dtype out),
  * by binary powering in FP64. */
 int adrt_twiddle_table(int dtype, int n, int K, const double* z, void* tab, void* stream);
