@@ -1,19 +1,37 @@
-// Spatial ADRT levels in the reference's layout (adrtcore.py:29-137). Level m maps data on E^n_{m-1}
-// (stored (N + 2^(m-1) - 1) x N, row = h + 2^(m-1) - 1) to E^n_m ((N + 2^m - 1) x N):
+// Spatial ADRT levels in the reference's layout (adrtcore.py:29-137). Level m maps data on E^n_{m-1} to E^n_m
+// (rows h = -(2^m - 1)..N-1):
 //   g(h, l*2w + 2t + b) = f(h, l*2w + t) [h >= -t] + f(h + t + b, l*2w + w + t) [h + t + b in [-t, N)],  w = 2^(m-1).
-// Forward: one pass per level over all images and quadrants, the quadrant permutation T_q folded into level 1.
-// Adjoint: the scatter-add of S_m^T is evaluated as a gather (two terms per output), and the last level also applies
-// T_q^T and sums the four quadrants. Additions only, so integer dtypes are exact.
+// Additions only, so integer dtypes are exact.
+//
+// Several levels per pass. Levels m0+1..m0+G combine, for one slope index t (< 2^m0) of level m0, the 2^G consecutive
+// blocks b of a group. Shifting block b by b t rows (f~_b(h) = f_b(h + b t)) turns them into a plain ADRT of 2^G columns
+// without t: with sigma the slope gained so far, sub-level u pairs blocks at a relative shift of sigma + b only. So a CTA
+// takes 32 columns (32 / 2^G such groups) and a band of rows plus a halo of 2^G - 1 through G levels in shared memory,
+// two levels at a time in registers, and HBM sees one read and one write per pass: 1 pass up to N = 16, 2 up to N = 256,
+// 3 up to N = 4096, instead of one per level. The guards of the formula need no code: data outside [-t, N) is zero
+// (forward), and values inside the domain only ever depend on values inside it (adjoint).
+//   * The band is 32 R rows, a lane owning R consecutive ones (R odd: conflict-free), so a two-level step costs
+//     4 R + 6 shared loads and 4 R stores for 4 R results; it touches four columns only and runs in place in one warp
+//     (results of slope digits b at bit position of their level: columns end up bit-reversed, undone by the addressing
+//     of the copy out).
+//   * Between passes the data lie as [slope t][block][row], rows contiguous, so the sheared reads stay coalesced; the
+//     first pass reads the T_q strips straight from the image, the last writes the sinogram's rows (32 columns, 128
+//     bytes in 4-byte types, at a time).
+//   * The adjoint runs the same passes backwards; its last pass leaves the four quadrants' images, which
+//     adrt_quadrant_sum adds (T_q^T).
+// Bounded by HBM (each pass reads and writes its level's data once). 64 int32 images at N = 256: forward 129 us, adjoint
+// 199 us (one pass per level above the fourth: 359 and 527 us); 3 FP32 images at N = 1024, adjoint: 137 us (624 us).
 #include "common.cuh"
 #include "launch.h"
 
 namespace adrt {
 
-static int grid_of(size_t total) {
-    size_t g = (total + 255) / 256;
-    if (g > 65535u * 16) g = 65535u * 16;
-    return (int)(g ? g : 1);
-}
+constexpr int AW_COLS = 32;      // columns per CTA
+constexpr int AW_THREADS = 256;  // 8 warps, one 4-column group each at 2^G columns per group of blocks
+constexpr int AW_PAD = 17;       // rows past the band that a step may touch (at most 3 sigma + 3 <= 15), pitch odd
+
+__host__ __device__ constexpr int aw_pitch(int R) { return 32 * R + AW_PAD; }
+template <int G> __host__ __device__ constexpr int aw_rows(int R) { return 32 * R - ((1 << G) - 1); }  // rows kept
 
 // (T_q x)(i, j) (adrtcore.py:29-39)
 template <typename T> __device__ __forceinline__ T tq_read(const T* x, int N, int q, int i, int j) {
@@ -25,337 +43,408 @@ template <typename T> __device__ __forceinline__ T tq_read(const T* x, int N, in
     }
 }
 
-// one forward level for every (image, quadrant); level 1 reads T_q x, later levels read src; slot stride S elements.
-// active (nullable): images with active[img] == 0 are skipped (their output is left as it was)
-template <typename T>
-__global__ void adrt_fwd_level(int n, int m, int nimg, const T* __restrict__ src, T* __restrict__ dst, size_t S,
-                               const int* __restrict__ active) {
-    const int N = 1 << n, w = 1 << (m - 1);
-    const int Hout = N + 2 * w - 1;
-    const size_t per = (size_t)Hout * N;
-    const size_t total = per * 4 * nimg;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const size_t slot = e / per;
-        if (active && !active[slot >> 2]) continue;
-        const size_t rem = e - slot * per;
-        const int row = (int)(rem >> n), s = (int)(rem & (N - 1));
-        const int h = row - (2 * w - 1);
-        const int l = s / (2 * w), rr = s - l * 2 * w, t = rr >> 1, b = rr & 1;
-        const int c0 = l * 2 * w + t, c1 = c0 + w;
-        T acc = 0;
-        if (m == 1) {
-            const int q = (int)(slot & 3);
-            const T* x = src + (slot >> 2) * (size_t)N * N;
-            if (h >= 0 && h < N) acc += tq_read(x, N, q, h, c0);
-            const int h1 = h + b;
-            if (h1 >= 0 && h1 < N) acc += tq_read(x, N, q, h1, c1);
+// what one CTA of a pass works on: levels m0+1..m0+G of image quadrant `slot`, groups slice0..slice0+nt-1 (group =
+// block group l' and slope t, group index l' 2^m0 + t, so the columns at level m0+G are group * 2^G + slope), rows
+// r0..r0+TR-1 of the level-(m0+G) layout
+struct AwPass {
+    int n, m0;
+    int bands, groups;  // CTAs along the rows and along the columns, per slot
+    int nt;             // groups per CTA
+    size_t S;           // elements per slot in the scratch and in the sinogram
+};
+
+// sub-levels u+1, u+2 (or u+1 alone) on the columns of a group, in place; fwd: shifts towards larger rows
+template <typename T, int G, int R, int U, bool FWD>
+__device__ __forceinline__ void aw_step4(T* tile, int ncols, int warp, int lane) {
+    constexpr int P = aw_pitch(R), LOW = (1 << U) - 1;
+    for (int task = warp; task < ncols / 4; task += AW_THREADS / 32) {
+        const int grp = task / ((1 << G) / 4), w = task % ((1 << G) / 4);
+        const int phi = (w & LOW) | ((w >> U) << (U + 2));
+        const int sg = U ? (int)(__brev((unsigned)(phi & LOW)) >> (32 - (U ? U : 1))) : 0;
+        T* c0 = tile + (size_t)(grp * (1 << G) + phi) * P + lane * R;
+        T* c1 = c0 + (size_t)P * (1 << U);
+        T* c2 = c1 + (size_t)P * (1 << U);
+        T* c3 = c2 + (size_t)P * (1 << U);
+        if (FWD) {
+            // blocks 0..3 with block j shifted by j sigma; slopes b (first level), b' (second)
+            T p0[2][R], p1[2][R + 2];
+            {
+                T a[R], b[R + 1];
+#pragma unroll
+                for (int i = 0; i < R; ++i) a[i] = c0[i];
+#pragma unroll
+                for (int i = 0; i < R + 1; ++i) b[i] = c1[sg + i];
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    p0[0][i] = a[i] + b[i];
+                    p0[1][i] = a[i] + b[i + 1];
+                }
+            }
+            {
+                T a[R + 2], b[R + 3];
+#pragma unroll
+                for (int i = 0; i < R + 2; ++i) a[i] = c2[2 * sg + i];
+#pragma unroll
+                for (int i = 0; i < R + 3; ++i) b[i] = c3[3 * sg + i];
+#pragma unroll
+                for (int i = 0; i < R + 2; ++i) {
+                    p1[0][i] = a[i] + b[i];
+                    p1[1][i] = a[i] + b[i + 1];
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                c0[i] = p0[0][i] + p1[0][i];          // b = 0, b' = 0
+                c2[i] = p0[0][i] + p1[0][i + 1];      // b = 0, b' = 1
+                c1[i] = p0[1][i] + p1[1][i + 1];      // b = 1, b' = 0
+                c3[i] = p0[1][i] + p1[1][i + 2];      // b = 1, b' = 1
+            }
         } else {
-            const T* f = src + slot * S;
-            const int off = w - 1;
-            if (h >= -t && h < N) acc += f[(size_t)(h + off) * N + c0];
-            const int h1 = h + t + b;
-            if (h1 >= -t && h1 < N) acc += f[(size_t)(h1 + off) * N + c1];
+            // o(b, b') in columns b + 2 b'; rows r-3..r (the rows above the band's first are never kept)
+            T f0[R], f1[R], f2[R], f3[R];
+            auto at = [&](const T* c, int i) -> T { return (i >= 0 || lane > 0) ? c[i] : (T)0; };
+            {
+                T s0[R], s1[R + 1], t0[R], t1[R + 1];
+                T x[R + 1], y[R + 2];
+                // b = 0: p0(r, 0) = o00(r) + o01(r), P1(r, 0) = o00(r) + o01(r - 1)
+#pragma unroll
+                for (int i = 0; i < R; ++i) x[i] = c0[i];
+#pragma unroll
+                for (int i = 0; i < R + 1; ++i) y[i] = at(c2, i - 1);
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    s0[i] = x[i] + y[i + 1];
+                    t0[i] = x[i] + y[i];
+                }
+                // b = 1: p0(r, 1) = o10(r) + o11(r), P1(r, 1) = o10(r - 1) + o11(r - 2); rows r - 1 and r
+                T xx[R + 2], yy[R + 3];
+#pragma unroll
+                for (int i = 0; i < R + 2; ++i) xx[i] = at(c1, i - 2);
+#pragma unroll
+                for (int i = 0; i < R + 3; ++i) yy[i] = at(c3, i - 3);
+#pragma unroll
+                for (int i = 0; i < R + 1; ++i) {
+                    s1[i] = xx[i + 1] + yy[i + 2];  // p0(r - 1 + i, 1)
+                    t1[i] = xx[i] + yy[i];          // P1(r - 1 + i, 1) = o10(r - 2 + i) + o11(r - 3 + i)
+                }
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    f0[i] = s0[i] + s1[i + 1];
+                    f1[i] = s0[i] + s1[i];
+                    f2[i] = t0[i] + t1[i + 1];
+                    f3[i] = t0[i] + t1[i];
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                c0[i] = f0[i];
+                c1[sg + i] = f1[i];
+                c2[2 * sg + i] = f2[i];
+                c3[3 * sg + i] = f3[i];
+            }
         }
-        dst[slot * S + rem] = acc;
+        __syncwarp();
     }
 }
 
-// adjoint value of level m at input position (h, col) from level-m data g (rows h_out + 2w - 1)
-template <typename T> __device__ __forceinline__ T adj_at(const T* g, int N, int m, int h, int col) {
-    const int w = 1 << (m - 1);
-    const int l = col / (2 * w), r = col - l * 2 * w, c = r / w, t = r - c * w;
-    if (h < -t || h >= N) return 0;
-    const int base = l * 2 * w + 2 * t, off = 2 * w - 1;
-    if (c == 0) return g[(size_t)(h + off) * N + base] + g[(size_t)(h + off) * N + base + 1];
-    return g[(size_t)(h - t + off) * N + base] + g[(size_t)(h - t - 1 + off) * N + base + 1];
-}
-
-template <typename T>
-__global__ void adrt_adj_level(int n, int m, int nimg, const T* __restrict__ src, T* __restrict__ dst, size_t S,
-                               const int* __restrict__ active) {
-    const int N = 1 << n, w = 1 << (m - 1);
-    const int Hin = N + w - 1;
-    const size_t per = (size_t)Hin * N;
-    const size_t total = per * 4 * nimg;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const size_t slot = e / per;
-        if (active && !active[slot >> 2]) continue;
-        const size_t rem = e - slot * per;
-        const int row = (int)(rem >> n), col = (int)(rem & (N - 1));
-        dst[slot * S + rem] = adj_at(src + slot * S, N, m, row - (w - 1), col);
-    }
-}
-
-// ------------------------------------------------------------------ tiled level passes (N >= 32, level m >= 2)
-// The per-element kernels above read the second term f(h + t + b, c1) along a shear: neighbouring output columns
-// read different rows, so a warp's loads touch many rows. The tiled passes stage the input rows a tile of 32 output
-// columns x ADRT_TR output rows needs in shared memory with row-contiguous (coalesced) loads, then gather from there;
-// the arithmetic and the guards are those of adrt_fwd_level / adj_at.
-constexpr int ADRT_TR = 32;  // output rows per tile
-
-template <typename T>
-__global__ void __launch_bounds__(256) adrt_fwd_level_tiled(int n, int m, const T* __restrict__ src,
-                                                            T* __restrict__ dst, size_t S,
-                                                            const int* __restrict__ active) {
-    const int N = 1 << n, w = 1 << (m - 1);
-    const int Hout = N + 2 * w - 1, off = w - 1;
-    const int s0 = blockIdx.x * 32, row0 = blockIdx.y * ADRT_TR;
-    const size_t slot = blockIdx.z;
-    if (active && !active[slot >> 2]) return;
-    const T* f = src + slot * S;
-    T* g = dst + slot * S;
-    const int h0 = row0 - (2 * w - 1);  // h of the tile's first output row
-    __shared__ T tA[ADRT_TR + 16][33];
-    __shared__ T tB[ADRT_TR + 16][17];
-    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    auto ld = [&](int h, int c) -> T { return (h >= -(w - 1) && h < N) ? f[(size_t)(h + off) * N + c] : (T)0; };
-    const bool small = 2 * w <= 32;
-    int cA = s0, cB = 0, hB = h0, t0 = 0;
-    if (small) {
-        // the 32 output columns read input columns of the same window, rows h0 .. h0 + TR + w - 1
-        for (int e = threadIdx.x; e < (ADRT_TR + w) * 32; e += 256) {
-            const int r = e >> 5, c = e & 31;
-            tA[r][c] = ld(h0 + r, s0 + c);
+template <typename T, int G, int R, int U, bool FWD>
+__device__ __forceinline__ void aw_step2(T* tile, int ncols, int warp, int lane) {
+    constexpr int P = aw_pitch(R), LOW = (1 << U) - 1;
+    for (int task = warp; task < ncols / 2; task += AW_THREADS / 32) {
+        const int grp = task / ((1 << G) / 2), w = task % ((1 << G) / 2);
+        const int phi = (w & LOW) | ((w >> U) << (U + 1));
+        const int sg = U ? (int)(__brev((unsigned)(phi & LOW)) >> (32 - (U ? U : 1))) : 0;
+        T* c0 = tile + (size_t)(grp * (1 << G) + phi) * P + lane * R;
+        T* c1 = c0 + (size_t)P * (1 << U);
+        T x[R], y[R + 1], f0[R], f1[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = c0[i];
+#pragma unroll
+        for (int i = 0; i < R + 1; ++i) y[i] = FWD ? c1[sg + i] : ((i > 0 || lane > 0) ? c1[i - 1] : (T)0);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            if (FWD) {
+                f0[i] = x[i] + y[i];
+                f1[i] = x[i] + y[i + 1];
+            } else {
+                f0[i] = x[i] + y[i + 1];  // g(h, 2t) + g(h, 2t + 1)
+                f1[i] = x[i] + y[i];      // g(h - t, 2t) + g(h - t - 1, 2t + 1), stored t rows further
+            }
         }
-    } else {
-        const int l = s0 / (2 * w);
-        t0 = (s0 - l * 2 * w) >> 1;
-        cA = l * 2 * w + t0;  // c0 columns cA .. cA + 15
-        cB = cA + w;          // c1 columns cB .. cB + 15
-        hB = h0 + t0;         // c1 rows h + t + b start at h0 + t0
-        for (int e = threadIdx.x; e < ADRT_TR * 16; e += 256) {
-            const int r = e >> 4, c = e & 15;
-            tA[r][c] = ld(h0 + r, cA + c);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            c0[i] = f0[i];
+            c1[(FWD ? 0 : sg) + i] = f1[i];
         }
-        for (int e = threadIdx.x; e < (ADRT_TR + 16) * 16; e += 256) {
-            const int r = e >> 4, c = e & 15;
-            tB[r][c] = ld(hB + r, cB + c);
-        }
-    }
-    __syncthreads();
-    const int s = s0 + lane;
-    const int l = s / (2 * w), rr = s - l * 2 * w, t = rr >> 1, b = rr & 1;
-    const int c0 = l * 2 * w + t, c1 = c0 + w;
-    for (int i = grp; i < ADRT_TR; i += 8) {
-        const int row = row0 + i;
-        if (row >= Hout) break;
-        const int h = h0 + i;
-        T acc = 0;
-        if (h >= -t && h < N) acc += small ? tA[i][c0 - s0] : tA[i][c0 - cA];
-        const int h1 = h + t + b;
-        if (h1 >= -t && h1 < N) acc += small ? tA[h1 - h0][c1 - s0] : tB[h1 - hB][c1 - cB];
-        g[(size_t)row * N + s] = acc;
+        __syncwarp();
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) adrt_adj_level_tiled(int n, int m, const T* __restrict__ src,
-                                                            T* __restrict__ dst, size_t S,
-                                                            const int* __restrict__ active) {
-    const int N = 1 << n, w = 1 << (m - 1);
-    const int Hin = N + w - 1, off = 2 * w - 1;  // output rows (level m-1 layout); input row offset (level m)
-    const int col0 = blockIdx.x * 32, row0 = blockIdx.y * ADRT_TR;
-    const size_t slot = blockIdx.z;
-    if (active && !active[slot >> 2]) return;
-    const T* g = src + slot * S;
-    T* o = dst + slot * S;
-    const int h0 = row0 - (w - 1);
-    __shared__ T tg[ADRT_TR + 32][65];
-    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    const int Hg = N + 2 * w - 1;
-    auto ld = [&](int h, int c) -> T {
-        const int r = h + off;
-        return (r >= 0 && r < Hg) ? g[(size_t)r * N + c] : (T)0;
-    };
-    const bool small = 2 * w <= 32;
-    const int l = col0 / (2 * w), r0 = col0 - l * 2 * w, half = small ? 0 : r0 / w;
-    const int t0 = small ? 0 : r0 - half * w;
-    int gc0, gh0, ncols;
-    if (small) {
-        gc0 = col0;      // the window's own columns
-        gh0 = h0 - w;    // rows h - t - 1 >= h0 - w
-        ncols = 32;
-    } else {
-        gc0 = l * 2 * w + 2 * t0;                // base columns of t0 .. t0 + 31, and base + 1
-        gh0 = half == 0 ? h0 : h0 - t0 - 32;     // second half reads rows h - t, h - t - 1
-        ncols = 64;
-    }
-    const int nrows = small ? ADRT_TR + w : (half == 0 ? ADRT_TR : ADRT_TR + 32);
-    for (int e = threadIdx.x; e < nrows * ncols; e += 256) {
-        const int r = e / ncols, c = e - r * ncols;
-        tg[r][c] = ld(gh0 + r, gc0 + c);
-    }
-    __syncthreads();
-    const int col = col0 + lane;
-    const int cl = col / (2 * w), r = col - cl * 2 * w, c = r / w, t = r - c * w;
-    const int base = cl * 2 * w + 2 * t - gc0;
-    for (int i = grp; i < ADRT_TR; i += 8) {
-        const int row = row0 + i;
-        if (row >= Hin) break;
-        const int h = h0 + i;
-        T v = 0;
-        if (h >= -t && h < N) {
-            if (c == 0) v = tg[h - gh0][base] + tg[h - gh0][base + 1];
-            else v = tg[h - t - gh0][base] + tg[h - t - 1 - gh0][base + 1];
-        }
-        o[(size_t)row * N + col] = v;
-    }
-}
+template <int G> __device__ __forceinline__ int aw_rev(int x) { return (int)(__brev((unsigned)x) >> (32 - G)); }
 
-// ------------------------------------------------------------------ the first four levels in shared memory
-// Levels 1..4 only combine columns within blocks of 16 (level m pairs the halves of blocks of 2^m columns), so a CTA
-// can take one 16-column block of one quadrant through all four levels in shared memory: the forward pass reads the
-// T_q strip once and writes level 4; the adjoint reads level 4 and writes level 1 (the quadrant sum stays with
-// adrt_adj_final). Rows in shared memory have a stride of 17 elements (conflict-free column walks).
-constexpr int F4_SP = 17;
-
-template <typename T> static size_t f4_smem(int N) { return 2 * (size_t)(N + 15) * F4_SP * sizeof(T); }
-
-template <typename T>
-__global__ void __launch_bounds__(256) adrt_fwd_levels14(int n, const T* __restrict__ x, T* __restrict__ dst, size_t S,
-                                                         const int* __restrict__ active) {
-    const int N = 1 << n;
-    const int c0 = blockIdx.x * 16, q = blockIdx.y, img = blockIdx.z;
-    if (active && !active[img]) return;
+// forward levels m0+1..m0+G: src is the image (m0 = 0) or the level-m0 layout [t][block][row]; dst the level-(m0+G)
+// layout, or the sinogram's rows where m0 + G = n. active (nullable): images with active[img] == 0 are skipped
+template <typename T, int G, int R>
+__global__ void __launch_bounds__(AW_THREADS) adrt_fwd_pass(const AwPass A, const T* __restrict__ src,
+                                                            T* __restrict__ dst, const int* __restrict__ active) {
+    constexpr int C = 1 << G, P = aw_pitch(R), RT = 32 * R, TR = aw_rows<G>(R);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* a = reinterpret_cast<T*>(smem_raw);
-    T* b = a + (size_t)(N + 15) * F4_SP;
-    const T* xi = x + (size_t)img * N * N;
-    // level 0: the T_q strip (rows h = 0..N-1); quadrants 0 and 3 read image rows, so there consecutive threads take
-    // consecutive h, the others consecutive columns
-    for (int e = threadIdx.x; e < N * 16; e += 256) {
-        int h, c;
-        if (q == 1 || q == 2) {
-            h = e >> 4;
-            c = e & 15;
+    T* tile = reinterpret_cast<T*>(smem_raw);
+    const int N = 1 << A.n, M0 = 1 << A.m0, M1 = M0 << G;
+    const int slice0 = (int)(blockIdx.x % A.groups) * A.nt;
+    const int band = (int)(blockIdx.x / A.groups % A.bands);
+    const size_t slot = blockIdx.x / A.groups / A.bands;
+    if (active && !active[slot >> 2]) return;
+    const int ncols = A.nt * C, HO = N + M1 - 1, r0 = band * TR, h0 = r0 - (M1 - 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool last = A.m0 + G == A.n;
+    // the largest slope of this CTA's columns: rows below it are structurally zero
+    int smax = 0;
+    for (int i = 0; i < A.nt; ++i) smax = max(smax, ((slice0 + i) & (M0 - 1)) * C + C - 1);
+    const bool zero = h0 + TR - 1 < -smax;
+    if (zero && !last) return;
+    if (!zero) {
+        if (A.m0 == 0) {
+            const T* x = src + (slot >> 2) * (size_t)N * N;
+            const int q = (int)(slot & 3), c0 = slice0 * C;
+            if (q == 1 || q == 2) {  // image rows along the columns
+#pragma unroll 4
+                for (int e = threadIdx.x; e < RT * AW_COLS; e += AW_THREADS) {
+                    const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + r;
+                    if (c < ncols) tile[c * P + r] = (h >= 0 && h < N) ? tq_read(x, N, q, h, c0 + c) : (T)0;
+                }
+            } else {
+                for (int c = warp; c < ncols; c += AW_THREADS / 32)
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        const int r = i * 32 + lane, h = h0 + r;
+                        tile[c * P + r] = (h >= 0 && h < N) ? tq_read(x, N, q, h, c0 + c) : (T)0;
+                    }
+            }
         } else {
-            c = e >> n;
-            h = e & (N - 1);
-        }
-        a[h * F4_SP + c] = tq_read(xi, N, q, h, c0 + c);
-    }
-    __syncthreads();
-    int off = 0;  // row offset of the level held in a (level m-1 data: 2^(m-1) - 1)
-    for (int m = 1; m <= 4; ++m) {
-        const int w = 1 << (m - 1), Hout = N + 2 * w - 1;
-        for (int e = threadIdx.x; e < Hout * 16; e += 256) {
-            const int row = e >> 4, cc = e & 15;
-            const int h = row - (2 * w - 1);
-            const int l = cc / (2 * w), rr = cc - l * 2 * w, t = rr >> 1, bb = rr & 1;
-            const int ca = l * 2 * w + t, cb = ca + w;
-            T acc = 0;
-            if (h >= -t && h < N) acc += a[(h + off) * F4_SP + ca];
-            const int h1 = h + t + bb;
-            if (h1 >= -t && h1 < N) acc += a[(h1 + off) * F4_SP + cb];
-            b[row * F4_SP + cc] = acc;
+            const int P0 = N + M0 - 1;
+            const T* f = src + slot * A.S;
+            for (int c = warp; c < ncols; c += AW_THREADS / 32) {
+                const int sl = slice0 + c / C, t = sl & (M0 - 1), b = c % C;
+                const T* col = f + ((size_t)t * (N / M0) + (size_t)(sl >> A.m0) * C + b) * P0 + (M0 - 1);
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int r = i * 32 + lane, h = h0 + r + b * t;
+                    tile[c * P + r] = (h >= -t && h < N) ? col[h] : (T)0;
+                }
+            }
         }
         __syncthreads();
-        T* tmp = a;
-        a = b;
-        b = tmp;
-        off = 2 * w - 1;
+        if constexpr (G >= 2) aw_step4<T, G, R, 0, true>(tile, ncols, warp, lane);
+        else aw_step2<T, G, R, 0, true>(tile, ncols, warp, lane);
+        __syncthreads();
+        if constexpr (G == 4) {
+            aw_step4<T, G, R, 2, true>(tile, ncols, warp, lane);
+            __syncthreads();
+        } else if constexpr (G == 3) {
+            aw_step2<T, G, R, 2, true>(tile, ncols, warp, lane);
+            __syncthreads();
+        }
     }
-    T* g = dst + ((size_t)img * 4 + q) * S;
-    for (int e = threadIdx.x; e < (N + 15) * 16; e += 256) {
-        const int row = e >> 4, cc = e & 15;
-        g[(size_t)row * N + c0 + cc] = a[row * F4_SP + cc];
+    if (last) {
+        T* g = dst + slot * A.S + slice0 * C;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < TR * AW_COLS; e += AW_THREADS) {
+            const int r = e / AW_COLS, c = e % AW_COLS;
+            if (c < ncols && r0 + r < HO)
+                g[(size_t)(r0 + r) * N + c] = zero ? (T)0 : tile[((c & ~(C - 1)) | aw_rev<G>(c & (C - 1))) * P + r];
+        }
+    } else {
+        const int P1 = N + M1 - 1;
+        T* g = dst + slot * A.S;
+        for (int c = warp; c < ncols; c += AW_THREADS / 32) {
+            const int sl = slice0 + c / C, t = (sl & (M0 - 1)) * C + aw_rev<G>(c % C);
+            T* col = g + ((size_t)t * (N / M1) + (sl >> A.m0)) * P1;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = i * 32 + lane;
+                if (r < TR && r0 + r < HO) col[r0 + r] = tile[c * P + r];
+            }
+        }
     }
 }
 
+// adjoint levels m0+G..m0+1: src is the sinogram (m0 + G = n) or the level-(m0+G) layout; dst the level-m0 layout, or
+// (m0 = 0) the quadrant's image, [h][column] for quadrants 1 and 2 and [column][h] for 0 and 3
+template <typename T, int G, int R>
+__global__ void __launch_bounds__(AW_THREADS) adrt_adj_pass(const AwPass A, const T* __restrict__ src,
+                                                            T* __restrict__ dst, const int* __restrict__ active) {
+    constexpr int C = 1 << G, P = aw_pitch(R), RT = 32 * R, TR = aw_rows<G>(R), HALO = C - 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* tile = reinterpret_cast<T*>(smem_raw);
+    const int N = 1 << A.n, M0 = 1 << A.m0, M1 = M0 << G;
+    const int slice0 = (int)(blockIdx.x % A.groups) * A.nt;
+    const int band = (int)(blockIdx.x / A.groups % A.bands);
+    const size_t slot = blockIdx.x / A.groups / A.bands;
+    if (active && !active[slot >> 2]) return;
+    // tile row i holds row h0 + i of the inputs (and of the blocks shifted by b t); rows i >= HALO are kept. The kept
+    // rows cover -(M1 - C)..N-1, or 0..N-1 in the last pass
+    const int ncols = A.nt * C, hbase = -(M1 - C), h0 = hbase + band * TR - HALO;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int tmax = 0;
+    for (int i = 0; i < A.nt; ++i) tmax = max(tmax, (slice0 + i) & (M0 - 1));
+    if (h0 + RT - 1 < -C * tmax) return;  // no block has a row of its domain here
+    if (A.m0 + G == A.n) {
+        const T* g = src + slot * A.S + slice0 * C;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < RT * AW_COLS; e += AW_THREADS) {
+            const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + r;
+            if (c < ncols)
+                tile[((c & ~(C - 1)) | aw_rev<G>(c & (C - 1))) * P + r] =
+                    (h > -N && h < N) ? g[(size_t)(h + N - 1) * N + c] : (T)0;
+        }
+    } else {
+        const int P1 = N + M1 - 1;
+        const T* g = src + slot * A.S;
+        for (int c = warp; c < ncols; c += AW_THREADS / 32) {
+            const int sl = slice0 + c / C, t = (sl & (M0 - 1)) * C + aw_rev<G>(c % C);
+            const T* col = g + ((size_t)t * (N / M1) + (sl >> A.m0)) * P1 + (M1 - 1);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = i * 32 + lane, h = h0 + r;
+                tile[c * P + r] = (h >= -t && h < N) ? col[h] : (T)0;
+            }
+        }
+    }
+    __syncthreads();
+    if constexpr (G == 4) {
+        aw_step4<T, G, R, 2, false>(tile, ncols, warp, lane);
+        __syncthreads();
+    } else if constexpr (G == 3) {
+        aw_step2<T, G, R, 2, false>(tile, ncols, warp, lane);
+        __syncthreads();
+    }
+    if constexpr (G >= 2) aw_step4<T, G, R, 0, false>(tile, ncols, warp, lane);
+    else aw_step2<T, G, R, 0, false>(tile, ncols, warp, lane);
+    __syncthreads();
+    T* o = dst + slot * A.S;
+    if (A.m0 == 0) {
+        const int q = (int)(slot & 3), c0 = slice0 * C;
+        if (q == 1 || q == 2) {
+#pragma unroll 4
+            for (int e = threadIdx.x; e < TR * AW_COLS; e += AW_THREADS) {
+                const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + HALO + r;
+                if (c < ncols && h < N) o[(size_t)h * N + c0 + c] = tile[c * P + HALO + r];
+            }
+        } else {
+            for (int c = warp; c < ncols; c += AW_THREADS / 32)
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int r = i * 32 + lane, h = h0 + HALO + r;
+                    if (r < TR && h < N) o[(size_t)(c0 + c) * N + h] = tile[c * P + HALO + r];
+                }
+        }
+    } else {
+        const int P0 = N + M0 - 1;
+        for (int c = warp; c < ncols; c += AW_THREADS / 32) {
+            const int sl = slice0 + c / C, t = sl & (M0 - 1), b = c % C;
+            T* col = o + ((size_t)t * (N / M0) + (size_t)(sl >> A.m0) * C + b) * P0 + (M0 - 1);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int r = i * 32 + lane, h = h0 + HALO + r + b * t;
+                if (r < TR && h >= -t && h < N) col[h] = tile[c * P + HALO + r];
+            }
+        }
+    }
+}
+
+// x[a, b] = sum_q (T_q^T f_q)[a, b] (adrtcore.py:131-137): q0 f(N-1-b, a), q1 f(N-1-a, b), q2 f(a, b), q3 f(N-1-b, N-1-a)
 template <typename T>
-__global__ void __launch_bounds__(256) adrt_adj_levels42(int n, const T* __restrict__ src, T* __restrict__ dst,
+__global__ void __launch_bounds__(256) adrt_quadrant_sum(int n, size_t total, const T* __restrict__ f, T* __restrict__ x,
                                                          size_t S, const int* __restrict__ active) {
     const int N = 1 << n;
-    const int c0 = blockIdx.x * 16;
-    const size_t slot = blockIdx.y;
-    if (active && !active[slot >> 2]) return;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* a = reinterpret_cast<T*>(smem_raw);
-    T* b = a + (size_t)(N + 15) * F4_SP;
-    const T* g = src + slot * S;
-    for (int e = threadIdx.x; e < (N + 15) * 16; e += 256) {
-        const int row = e >> 4, cc = e & 15;
-        a[row * F4_SP + cc] = g[(size_t)row * N + c0 + cc];
-    }
-    __syncthreads();
-    for (int m = 4; m >= 2; --m) {
-        // level-m data in a (rows h + 2w - 1) -> level m-1 data in b (rows h + w - 1), as adj_at
-        const int w = 1 << (m - 1), Hin = N + w - 1, goff = 2 * w - 1;
-        for (int e = threadIdx.x; e < Hin * 16; e += 256) {
-            const int row = e >> 4, col = e & 15;
-            const int h = row - (w - 1);
-            const int l = col / (2 * w), r = col - l * 2 * w, c = r / w, t = r - c * w;
-            T v = 0;
-            if (h >= -t && h < N) {
-                const int base = l * 2 * w + 2 * t;
-                if (c == 0) v = a[(h + goff) * F4_SP + base] + a[(h + goff) * F4_SP + base + 1];
-                else v = a[(h - t + goff) * F4_SP + base] + a[(h - t - 1 + goff) * F4_SP + base + 1];
-            }
-            b[row * F4_SP + col] = v;
-        }
-        __syncthreads();
-        T* tmp = a;
-        a = b;
-        b = tmp;
-    }
-    T* o = dst + slot * S;
-    for (int e = threadIdx.x; e < (N + 1) * 16; e += 256) {  // level 1: N + 1 rows
-        const int row = e >> 4, cc = e & 15;
-        o[(size_t)row * N + c0 + cc] = a[row * F4_SP + cc];
-    }
-}
-
-// level-1 adjoint of the four quadrants, T_q^T and the quadrant sum (adrtcore.py:131-137)
-template <typename T>
-__global__ void adrt_adj_final(int n, int nimg, const T* __restrict__ src, T* __restrict__ x, size_t S,
-                               const int* __restrict__ active) {
-    const int N = 1 << n;
-    const size_t per = (size_t)N * N;
-    const size_t total = per * nimg;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const size_t img = e / per;
+        const size_t img = e >> (2 * n);
         if (active && !active[img]) continue;
-        const size_t rem = e - img * per;
-        const int a = (int)(rem >> n), b = (int)(rem & (N - 1));
-        const T* g = src + img * 4 * S;
-        // x[a, b] = sum_q (T_q^T f_q)[a, b]: q0 f(N-1-b, a); q1 f(N-1-a, b); q2 f(a, b); q3 f(N-1-b, N-1-a)
-        T acc = adj_at(g + 0 * S, N, 1, N - 1 - b, a);
-        acc += adj_at(g + 1 * S, N, 1, N - 1 - a, b);
-        acc += adj_at(g + 2 * S, N, 1, a, b);
-        acc += adj_at(g + 3 * S, N, 1, N - 1 - b, N - 1 - a);
+        const int rem = (int)(e & (((size_t)1 << (2 * n)) - 1)), a = rem >> n, b = rem & (N - 1);
+        const T* g = f + img * 4 * S;
+        T acc = g[(size_t)a * N + (N - 1 - b)];
+        acc += g[S + (size_t)(N - 1 - a) * N + b];
+        acc += g[2 * S + (size_t)a * N + b];
+        acc += g[3 * S + (size_t)(N - 1 - a) * N + (N - 1 - b)];
         x[e] = acc;
     }
 }
 
+template <typename T, int G, int R>
+static int launch_pass(bool fwd, AwPass A, int nslots, int rows, const void* src, void* dst, const int* active,
+                       cudaStream_t st) {
+    constexpr int C = 1 << G;
+    const int slices = (1 << A.n) / C;
+    A.nt = slices < AW_COLS / C ? slices : AW_COLS / C;
+    A.groups = slices / A.nt;
+    A.bands = (rows + aw_rows<G>(R) - 1) / aw_rows<G>(R);
+    const long long ctas = (long long)nslots * A.bands * A.groups;
+    if (ctas > 0x7fffffffLL) {
+        set_error("adrt: %lld thread blocks exceed the grid limit", ctas);
+        return ADRT_EINVAL;
+    }
+    const size_t smem = (size_t)AW_COLS * aw_pitch(R) * sizeof(T);
+    auto kern = fwd ? adrt_fwd_pass<T, G, R> : adrt_adj_pass<T, G, R>;
+    if (int rc = ensure_smem((const void*)kern, smem)) return rc;
+    kern<<<(unsigned)ctas, AW_THREADS, smem, st>>>(A, reinterpret_cast<const T*>(src), reinterpret_cast<T*>(dst), active);
+    return launch_status(fwd ? "adrt_fwd_pass" : "adrt_adj_pass");
+}
+
+// the band height: the one that computes the fewest rows (halo and remainder included); the smaller one where equal, for
+// more CTAs. Nine rows of 8-byte values per lane would leave one CTA per SM (registers), so those types stop at five
+template <typename T, int G>
+static int launch_pass_g(bool fwd, const AwPass& A, int nslots, int rows, const void* src, void* dst, const int* active,
+                         cudaStream_t st) {
+    auto cost = [&](int R) {
+        const int tr = 32 * R - ((1 << G) - 1);
+        return (rows + tr - 1) / tr * 32 * R;
+    };
+    const int c3 = cost(3), c5 = cost(5);
+    if constexpr (sizeof(T) == 4) {
+        if (cost(9) < c3 && cost(9) < c5) return launch_pass<T, G, 9>(fwd, A, nslots, rows, src, dst, active, st);
+    }
+    if (c3 <= c5) return launch_pass<T, G, 3>(fwd, A, nslots, rows, src, dst, active, st);
+    return launch_pass<T, G, 5>(fwd, A, nslots, rows, src, dst, active, st);
+}
+
+template <typename T>
+static int run_pass(bool fwd, int n, int m0, int G, int nimg, const void* src, void* dst, const int* active,
+                    cudaStream_t st) {
+    const int N = 1 << n, M1 = 1 << (m0 + G);
+    AwPass A = {};
+    A.n = n;
+    A.m0 = m0;
+    A.S = (size_t)(2 * N - 1) * N;
+    const int rows = fwd ? N + M1 - 1 : N + M1 - (1 << G);  // rows of the level written, or of the blocks produced
+    switch (G) {
+        case 1: return launch_pass_g<T, 1>(fwd, A, 4 * nimg, rows, src, dst, active, st);
+        case 2: return launch_pass_g<T, 2>(fwd, A, 4 * nimg, rows, src, dst, active, st);
+        case 3: return launch_pass_g<T, 3>(fwd, A, 4 * nimg, rows, src, dst, active, st);
+        default: return launch_pass_g<T, 4>(fwd, A, 4 * nimg, rows, src, dst, active, st);
+    }
+}
+
+// the passes of n levels: at most four levels each, the wider ones first; returns their number
+static int pass_levels(int n, int* G) {
+    const int np = (n + 3) / 4;
+    for (int p = 0; p < np; ++p) G[p] = n / np + (p < n % np ? 1 : 0);
+    return np;
+}
+
 template <typename T>
 static int fwd_t(int n, int nimg, const void* x, void* b, void* scratch, const int* active, cudaStream_t st) {
-    const int N = 1 << n;
-    const size_t S = (size_t)(2 * N - 1) * N;
+    const size_t S = ((size_t)(2 << n) - 1) << n;
     T* bufs[2] = {reinterpret_cast<T*>(scratch), reinterpret_cast<T*>(scratch) + S * 4 * nimg};
-    const T* src = reinterpret_cast<const T*>(x);
-    int m0 = 1;
-    if (n >= 4 && f4_smem<T>(N) <= 200 * 1024 && nimg <= 65535) {
-        // levels 1..4 in one pass per 16-column block and quadrant
-        T* dst = (n == 4) ? reinterpret_cast<T*>(b) : bufs[0];
-        const size_t smem = f4_smem<T>(N);
-        if (int rc = ensure_smem((const void*)adrt_fwd_levels14<T>, smem)) return rc;
-        adrt_fwd_levels14<T><<<dim3(N / 16, 4, nimg), 256, smem, st>>>(n, src, dst, S, active);
-        if (int rc = launch_status("adrt_fwd_levels14")) return rc;
-        src = dst;
-        m0 = 5;
-    }
-    for (int m = m0; m <= n; ++m) {
-        T* dst = (m == n) ? reinterpret_cast<T*>(b) : bufs[m & 1];
-        const int Hout = N + (1 << m) - 1;
-        const size_t total = (size_t)Hout * N * 4 * nimg;
-        if (m >= 2 && N >= 32 && 4L * nimg <= 65535) {
-            dim3 grid(N / 32, (Hout + ADRT_TR - 1) / ADRT_TR, 4 * nimg);
-            adrt_fwd_level_tiled<T><<<grid, 256, 0, st>>>(n, m, src, dst, S, active);
-        } else {
-            adrt_fwd_level<T><<<grid_of(total), 256, 0, st>>>(n, m, nimg, src, dst, S, active);
-        }
-        int rc = launch_status("adrt_fwd_level");
-        if (rc) return rc;
+    int G[4];
+    const int np = pass_levels(n, G);
+    const void* src = x;
+    for (int p = 0, m0 = 0; p < np; m0 += G[p], ++p) {
+        void* dst = p == np - 1 ? b : bufs[p & 1];
+        if (int rc = run_pass<T>(true, n, m0, G[p], nimg, src, dst, active, st)) return rc;
         src = dst;
     }
     return ADRT_OK;
@@ -363,36 +452,23 @@ static int fwd_t(int n, int nimg, const void* x, void* b, void* scratch, const i
 
 template <typename T>
 static int adj_t(int n, int nimg, const void* b, void* x, void* scratch, const int* active, cudaStream_t st) {
-    const int N = 1 << n;
-    const size_t S = (size_t)(2 * N - 1) * N;
+    const size_t S = ((size_t)(2 << n) - 1) << n;
     T* bufs[2] = {reinterpret_cast<T*>(scratch), reinterpret_cast<T*>(scratch) + S * 4 * nimg};
-    const T* src = reinterpret_cast<const T*>(b);
-    const bool fuse = n >= 4 && f4_smem<T>(N) <= 200 * 1024 && 4L * nimg <= 65535;
-    for (int m = n; m >= (fuse ? 5 : 2); --m) {
-        T* dst = bufs[m & 1];
-        const int Hin = N + (1 << (m - 1)) - 1;
-        const size_t total = (size_t)Hin * N * 4 * nimg;
-        if (N >= 32 && 4L * nimg <= 65535) {
-            dim3 grid(N / 32, (Hin + ADRT_TR - 1) / ADRT_TR, 4 * nimg);
-            adrt_adj_level_tiled<T><<<grid, 256, 0, st>>>(n, m, src, dst, S, active);
-        } else {
-            adrt_adj_level<T><<<grid_of(total), 256, 0, st>>>(n, m, nimg, src, dst, S, active);
-        }
-        int rc = launch_status("adrt_adj_level");
-        if (rc) return rc;
-        src = dst;
+    int G[4];
+    const int np = pass_levels(n, G);
+    const void* src = b;
+    int m0 = n;
+    for (int p = np - 1; p >= 0; --p) {
+        m0 -= G[p];
+        if (int rc = run_pass<T>(false, n, m0, G[p], nimg, src, bufs[p & 1], active, st)) return rc;
+        src = bufs[p & 1];
     }
-    if (fuse) {
-        // levels 4..2 in one pass per 16-column block and quadrant: level 4 in, level 1 out
-        T* dst = (src == bufs[0]) ? bufs[1] : bufs[0];
-        const size_t smem = f4_smem<T>(N);
-        if (int rc = ensure_smem((const void*)adrt_adj_levels42<T>, smem)) return rc;
-        adrt_adj_levels42<T><<<dim3(N / 16, 4 * nimg), 256, smem, st>>>(n, src, dst, S, active);
-        if (int rc = launch_status("adrt_adj_levels42")) return rc;
-        src = dst;
-    }
-    adrt_adj_final<T><<<grid_of((size_t)N * N * nimg), 256, 0, st>>>(n, nimg, src, reinterpret_cast<T*>(x), S, active);
-    return launch_status("adrt_adj_final");
+    const size_t total = (size_t)nimg << (2 * n);
+    size_t grid = (total + 255) / 256;
+    if (grid > 65535u * 16) grid = 65535u * 16;
+    adrt_quadrant_sum<T><<<(unsigned)grid, 256, 0, st>>>(n, total, reinterpret_cast<const T*>(src),
+                                                         reinterpret_cast<T*>(x), S, active);
+    return launch_status("adrt_quadrant_sum");
 }
 
 int adrt_fwd(int dtype, int n, int nimg, const void* x, void* b, void* scratch, cudaStream_t st, const int* active) {
