@@ -18,6 +18,7 @@
 // CUDA-core kernel: the same product for any N and for FP64.
 #include "common.cuh"
 #include "launch.h"
+#include "tcgen05.cuh"
 
 namespace adrt {
 
@@ -119,46 +120,6 @@ __global__ void __launch_bounds__(DS_THREADS) dense_stream_kernel(int N, int nim
         for (int b = 0; b < NB; ++b)
             if (b0 + b < nimg) Zd[((size_t)r * nimg + b0 + b) * N + o] = acc[b];
     }
-}
-
-// ------------------------------------------------------------------ tcgen05 (sm_100 family) helpers
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor: K-major, no swizzle; LBO = byte step between core matrices along K,
-// SBO = byte step between 8-row groups along M / N; bits 46-47 = 1 (descriptor version of tcgen05)
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
-}
-
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
-}
-
-// bounded wait on an mbarrier phase; returns false if the limit ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    for (long it = 0; it < (1L << 24); ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 constexpr int TC_M = 128;   // real output rows per CTA (TMEM lanes)
@@ -397,39 +358,6 @@ __global__ void dense_split_kernel(int N, long long total, const float2* __restr
         t[2 * CX_TILE] = __uint_as_float(imh);
         t[3 * CX_TILE] = __uint_as_float(to_tf32(w.y - __uint_as_float(imh)));
     }
-}
-
-__device__ __forceinline__ void mbar_expect_bulk(uint32_t mbar, uint32_t dst, const void* src, uint32_t bytes) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}\n" ::"r"(mbar),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(mbar)
-                 : "memory");
-}
-
-// bounded wait that also gives up when another role of the CTA has set the abort flag
-__device__ __forceinline__ bool mbar_wait_or_abort(uint32_t mbar, uint32_t parity, const volatile int* abort_flag) {
-    for (long it = 0; it < (1L << 24); ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((it & 255) == 255 && *abort_flag) return false;
-    }
-    return false;
-}
-// the same, polled by lane 0 of a converged warp and broadcast, so that every lane takes the same branch
-__device__ __forceinline__ bool warp_wait(uint32_t mbar, uint32_t parity, const volatile int* abort_flag) {
-    int okv = 0;
-    if ((threadIdx.x & 31) == 0) okv = mbar_wait_or_abort(mbar, parity, abort_flag) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, okv, 0) != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" ::"r"(mbar) : "memory");
 }
 
 // Warp-specialised: warp 0 (one thread) streams the operator tiles of chunk after chunk into the ring, warps 2-3 build

@@ -94,7 +94,8 @@ class RowTables:
         # one pass G as a real operator per frequency (op_table), where the plan and the size allow it
         self.row_ops = row_operators_for(plan)
         self._g_ops = fuse_ops(_op_lists(plan)["G"])
-        self._op_dev = self._half = None
+        self._op_dev, self._half = {}, None
+        self.op_mma = None  # the row operators' form: None by batch size, or True (tensor cores) / False
         if self.high_ff:
             # the compensated rows read the roots of unity and the filter constants in FP64
             self.roots64 = torch.from_numpy(roots_of_unity(plan.L)).to(device=device, dtype=torch.complex128)
@@ -142,32 +143,43 @@ class RowTables:
         """Whether run() applies this op list as one real operator per frequency (the G list of the plan)."""
         return self.row_ops and fuse_ops(ops) == self._g_ops
 
-    def op_table(self):
-        """The plan's row operators (row_operator_table) in the row precision, shared by the plan's pipelines of that
-        precision while any of them holds it; None during a stream capture that finds it not built (the polynomial
-        rows run instead)."""
-        if self._op_dev is None:
-            shared = self.plan.__dict__.setdefault("_dense_shared", weakref.WeakValueDictionary())
-            key = (str(self.device), str(self.real), "row_ops")
-            T = shared.get(key)
-            if T is None:
-                if torch.cuda.is_current_stream_capturing():
-                    return None
-                T = row_operator_table(self, self.real)
-                torch.cuda.current_stream(self.device).synchronize()  # complete before another stream shares it
-                shared[key] = T
-            self._op_dev = T
-        if self._half is None:
+    def uses_mma(self, B):
+        """Whether the row operators of a batch of B images run on the tensor cores (op_mma, when set, decides)."""
+        fits = self.real == torch.float32 and self.plan.n in ROW_OPS_MMA_BATCH
+        return fits and (B >= ROW_OPS_MMA_BATCH[self.plan.n] if self.op_mma is None else self.op_mma)
+
+    def op_table(self, mma=False):
+        """The plan's row operators (row_operator_table) in the row precision, or (mma) the pair (split FP16 tiles, inverse
+        scales) of the tensor-core form; shared by the plan's pipelines of that precision while any of them holds them.
+        None during a stream capture that finds them not built (the polynomial rows run instead)."""
+        if self._half is None or mma not in self._op_dev:
             if torch.cuda.is_current_stream_capturing():
                 return None
-            self._half = torch.from_numpy(roots_of_unity(2 * self.plan.L)).to(device=self.device, dtype=_cdtype(self.real))
-        return self._op_dev
+            if self._half is None:
+                self._half = torch.from_numpy(roots_of_unity(2 * self.plan.L)).to(device=self.device,
+                                                                                  dtype=_cdtype(self.real))
+            shared = self.plan.__dict__.setdefault("_dense_shared", weakref.WeakValueDictionary())
+            key = (str(self.device), str(self.real), "row_ops", mma)
+            T = shared.get(key)
+            if T is None:
+                plain = shared.get(key[:3] + (False,)) if mma else None
+                T = row_operator_table(self, self.real) if plain is None else plain
+                if mma:
+                    T = _split_operators(self.plan.n, T)
+                torch.cuda.current_stream(self.device).synchronize()  # complete before another stream shares it
+                shared[key] = T
+            self._op_dev[mma] = T
+        return self._op_dev[mma]
 
     def run_operators(self, Y, T):
-        """Y[b, r] <- T_k Y[b, r] for every packed row (adrt_rows_operator), in place."""
+        """Y[b, r] <- T_k Y[b, r] for every packed row, in place (T: op_table of this batch size)."""
         B, R, N = Y.shape
-        C.call("adrt_rows_operator", self.code, self.plan.n, B, C.ptr(T), C.ptr(Y), R * N, C.ptr(self._half),
-               C.stream_handle())
+        st = C.stream_handle()
+        if self.uses_mma(B):
+            C.call("adrt_rows_operator_mma", self.plan.n, B, C.ptr(T), C.ptr(T._adrt_inv_scale), C.ptr(Y), R * N,
+                   C.ptr(self._half), C.ptr(self.err), st)
+            return
+        C.call("adrt_rows_operator", self.code, self.plan.n, B, C.ptr(T), C.ptr(Y), R * N, C.ptr(self._half), st)
 
     def main_level_rows(self, ops):
         """Level-rows processed by the polynomial-row launch of one op list (the dense rows excluded)."""
@@ -278,7 +290,7 @@ class RowTables:
         if not ops:
             return
         if not skip_main and self.row_ops and ops == self._g_ops:
-            T = self.op_table()
+            T = self.op_table(self.uses_mma(B))
             if T is not None:
                 self._timed(ops, lambda: self.run_operators(Y, T))
                 self.count += B * self.plan.level_rows(ops_unfused(ops))
@@ -356,6 +368,8 @@ def _rows_apply_f64(X, z_rows, ops, n, counter):
 # sizes whose G pass runs as row operators: above, the operators outgrow what a lane should hold (17 GB at N = 2048);
 # below, the polynomial rows are a few microseconds of latency
 ROW_OPS_MIN, ROW_OPS_MAX = 6, 9
+# batch sizes from which the FP32 row operators run on the tensor cores, by n
+ROW_OPS_MMA_BATCH = {8: 5, 9: 3}
 
 
 def row_operators_for(plan: Plan):
@@ -370,6 +384,18 @@ def row_operators_for(plan: Plan):
 def row_operator_bytes(plan: Plan, real):
     """Device bytes of a plan's row operators and of their half-shift phases in one precision."""
     return (plan.N + 1) * plan.N * plan.N // 2 * real.itemsize + 4 * plan.N * 2 * real.itemsize
+
+
+def _split_operators(n, T):
+    """The tensor-core form of FP32 row operators T: FP16 hi / lo tiles of T_k scaled by the power of two that brings its
+    largest entry to [2^13, 2^14) (adrt_rows_operator_split); the inverse scales hang on the tiles."""
+    _, e = torch.frexp(T.abs().amax(dim=(1, 2, 3)))
+    one = torch.ones_like(e, dtype=torch.float32)
+    scale = torch.ldexp(one, 14 - e)
+    Ts = torch.empty((T.numel(), 2), dtype=torch.float16, device=T.device)
+    C.call("adrt_rows_operator_split", n, C.ptr(T), C.ptr(scale), C.ptr(Ts), C.stream_handle())
+    Ts._adrt_inv_scale = torch.ldexp(one, e - 14)
+    return Ts
 
 
 def row_operator_table(tables, real):
@@ -554,6 +580,7 @@ class Pipeline:
         t = RowTables(self.plan, self.real, self.device)
         for k in ("stream_dense", "use_tc", "split_dense", "row_grid", "dense_tile", "row_ops"):
             setattr(t, k, getattr(self.tables, k))
+        t.op_mma = self.tables.uses_mma(self.B)  # the parent's operators, not a second form
         q.tables = t
         q.Y = self.Y[:b]
         q.parts = self.parts[:, :b]
@@ -699,7 +726,10 @@ class Pipeline:
         bufs += [T._adrt_split for T in t._dense_dev.values() if getattr(T, "_adrt_split", None) is not None]
         if t.high_ff:
             bufs += [t.roots64, t.coef64]
-        bufs += [x for x in (t._op_dev, t._half) if x is not None]
+        for T in t._op_dev.values():
+            bufs += [T] if getattr(T, "_adrt_inv_scale", None) is None else [T, T._adrt_inv_scale]
+        if t._half is not None:
+            bufs.append(t._half)
         if t._zd is not None:
             bufs.append(t._zd)
         for name in ("b_in", "b_in2"):
@@ -736,6 +766,8 @@ class Pipeline:
                 total += lists * nd * N * N * 16 - nd * B * N * 2 * rs
             if lists == 1:
                 total += row_operator_bytes(plan, PRECISIONS[precision])
+                if precision == "fp32" and B >= ROW_OPS_MMA_BATCH.get(plan.n, B + 1):
+                    total += (N + 1) * 4  # the inverse scales of the split form (its tiles take the FP32 operators' bytes)
         total += L * 2 * rs + 3 * L * 4 + plan.coef.size * rs  # roots; deg and the row lists; coefficients
         if captured:  # the two input buffers of the captured graphs
             total += 2 * B * 4 * (2 * N - 1) * N * 8

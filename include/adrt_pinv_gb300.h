@@ -132,6 +132,14 @@ int adrt_rows_run_multi(const adrt_row_job* jobs, const int32_t* code, const int
 int adrt_rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride,
                        const void* half_roots, void* stream);
 
+/* The same pass for FP32 rows on the tensor cores (n = 8, 9), the operators split once into FP16 pairs:
+ * adrt_rows_operator_split turns the FP32 T above, frequency k scaled by scale[k] (a power of two; largest entry below
+ * 2^14 after scaling), into Ts ((N+1) N^2 FP16 values, hi and lo tiles in the kernel's order); inv_scale[k] = 1/scale[k].
+ * err: device int, set to a positive code if a bounded wait ran out (the rows are then not all written). */
+int adrt_rows_operator_split(int n, const void* T, const float* scale, void* Ts, void* stream);
+int adrt_rows_operator_mma(int n, int nimg, const void* Ts, const float* inv_scale, void* Y, long long img_stride,
+                           const void* half_roots, int32_t* err, void* stream);
+
 /* Per-row twiddle table tab[k*(N/2+1) + t] = z_k^t (t = 0..N/2) from K complex z (FP64 in, dtype out),
  * by binary powering in FP64. */
 int adrt_twiddle_table(int dtype, int n, int K, const double* z, void* tab, void* stream);

@@ -61,6 +61,52 @@ def test_row_operators_match_rows(pkg, plans, method, p, cap, n, batches):
         rows = (y32.to(torch.complex128) - ref).norm(dim=-1).amax() / ref.norm(dim=-1).amax()
         assert float(rows) < 1e-6, B
         assert op32.count == op64.count == ref_t.count
+        if n >= 8:
+            # both forms of the FP32 operators at every batch, the tensor cores to the same bound
+            for form in (True, False):
+                op32.op_mma = form
+                y32 = Y.to(torch.complex64)
+                op32.run(y32, ops)
+                op32.raise_if_error()
+                assert float((y32.to(torch.complex128) - ref).norm() / ref.norm()) < 1e-6, (B, form)
+            op32.op_mma = None
+            op32.count = ref_t.count
+
+
+@pytest.mark.parametrize("n", [8, 9])
+def test_tensor_core_form_keeps_range_and_accuracy(pkg, plans, n):
+    """Vectors of very different magnitude (1e-30 .. 1e30) in one batch each keep their own scale, zero rows stay zero, a
+    row with a wide dynamic range keeps the accuracy of its largest values, and non-finite rows touch no other row."""
+    import torch
+    from adrt_pinv_gb300.device import _op_lists
+
+    plan = plans("hybrid", n, 32, 16)
+    ops, N, B = _op_lists(plan)["G"], 1 << n, 9
+    ref_t, t = _tables(plan, torch.float64, True), _tables(plan, torch.float32, True)
+    t.op_mma = True
+    g = torch.Generator(device="cuda").manual_seed(5)
+    Y = torch.randn((B, 4 * N, N), dtype=torch.complex128, device="cuda", generator=g)
+    mag = torch.randint(-30, 31, (B, 4 * N, 1), device="cuda", generator=g).double()
+    Y *= 10.0 ** mag
+    Y[2] = 0
+    Y[3] *= torch.exp(-20.0 * torch.rand((4 * N, N), device="cuda", generator=g, dtype=torch.float64))
+    y32 = Y.to(torch.complex64)
+    ref = y32.to(torch.complex128)
+    ref_t.run(ref, ops)
+    got = y32.clone()
+    t.run(got, ops)
+    t.raise_if_error()
+    err = (got.to(torch.complex128) - ref).norm(dim=-1)
+    assert not got[2].any()
+    assert bool((err <= 2e-6 * ref.norm(dim=-1)).all())
+    bad = y32.clone()
+    bad[4, 7, 5] = float("nan")
+    bad[5, 9, 1] = float("inf")
+    t.run(bad, ops)
+    rows = torch.isfinite(torch.view_as_real(bad)).all(dim=-1).all(dim=-1)
+    assert not rows[4, 7] and not rows[5, 9] and int(rows.sum()) == rows.numel() - 2
+    rows = rows.clone()
+    assert torch.equal(bad[rows], got[rows])
 
 
 def test_row_operators_need_symmetric_plans(pkg, plans):
