@@ -1,16 +1,22 @@
 // Offset-axis DFTs with the quadrant packing folded into the loads and stores (reference: fastops._packed,
 // fastops.py:209-220; Tq / TqT / iota, fastspec.py:142-174).
 //
-// One CTA handles a block of C strip columns of one image. The length-L (L = 2N) DFT of each column runs as an
-// in-place radix-2 decimation-in-time transform on bit-reversed input: each thread holds 8 points of its column,
-// does three stages in registers per pass and exchanges through a padded shared-memory tile between passes.
-// Twiddles come from an FP64-accurate table of L roots of unity staged in shared memory.
+// One CTA handles a block of C strip columns of one image. The length-L (L = 2N) DFT of each column runs as an in-place
+// decimation-in-time transform on bit-reversed input: each thread holds E = 8 or 16 points of its column (16 where that
+// saves a pass: L = 128, 256, 1024 and up), a pass multiplies them by their twiddles (one table value per point, none in
+// the first pass) and runs a radix-E butterfly with constant rotations, and the passes exchange through a padded
+// shared-memory tile.
 //
-// pack:   strips s_qa + i s_qb of each quadrant pair are gathered (coalesced, through the tile) from the image
-//         (Tq of the zero-padded image) or the sinogram (iota), transformed forward, and written as rows of Y.
-// unpack: both pairs of a column block are transformed back (1/L), only the first N offsets are kept, and the
-//         four quadrant strips are scattered with TqT and cropped into three image-space partial sums:
-//         colpart (quadrants II+III: out columns), rowpart0 (quadrant I: out rows), rowpart3 (quadrant IV).
+// pack:   strips s_qa + i s_qb of each quadrant pair come from the image (Tq of the zero-padded image) or the sinogram
+//         (iota), are transformed forward and written as rows of Y. Values that lie along the columns (two of the four
+//         image quadrants, the whole sinogram) go straight from global memory into the registers of the first pass;
+//         the quadrants that lie along image rows cross a small real tile. Image strips are zero from N on, so half of
+//         the first butterfly's inputs are constant zeros.
+// unpack: both pairs of a column block are transformed back (1/L), only the first N offsets are kept (half of the last
+//         butterfly is never computed), and the four quadrant strips go with TqT and cropped into three image-space
+//         partial sums: colpart (quadrants II+III: out columns), rowpart0 (quadrant I: out rows), rowpart3 (quadrant
+//         IV). Pair (0,1) runs with the threads of a column in reverse order, so that the offsets i of quadrant III and
+//         N-1-i of quadrant II meet in one thread; the row quadrants are transposed through shared memory.
 #include <type_traits>
 
 #include "common.cuh"
@@ -20,18 +26,19 @@ namespace adrt {
 
 template <int l> struct FftCfg {
     static constexpr int L = 1 << l;
-    static constexpr int e = (l >= 3) ? 3 : l;  // log2 of points per thread
+    // log2 of points per thread: 4 where that takes a pass (an exchange) less than 3
+    static constexpr int e = l < 3 ? l : ((l + 3) / 4 < (l + 2) / 3 ? 4 : 3);
     static constexpr int E = 1 << e;
     static constexpr int TPC = L / E;           // threads per column
-    static constexpr int NPASS = (l + 2) / 3;
-    __host__ __device__ static constexpr int s0(int q) { return 3 * q; }
-    __host__ __device__ static constexpr int nb(int q) { return imin(3, l - 3 * q); }
-    // physical position of register j in pass q for column-thread t
+    static constexpr int NPASS = (l + e - 1) / e;
+    __host__ __device__ static constexpr int s0(int q) { return e * q; }
+    __host__ __device__ static constexpr int nb(int q) { return imin(e, l - e * q); }
+    // physical position of register j in pass q for column-thread t: the pass's bits from the low bits of j, the rest of
+    // j (last pass) below the top of t
     __device__ static __forceinline__ int pos(int q, int t, int j) {
-        if (l < 3) return j;
         const int b = nb(q), s = s0(q);
-        if (b == 3) return (t & ((1 << s) - 1)) | (j << s) | ((t >> s) << (s + 3));
-        const int x = 3 - b;
+        if (b == e) return (t & ((1 << s) - 1)) | (j << s) | ((t >> s) << (s + e));
+        const int x = e - b;
         return (t & ((1 << (s - x)) - 1)) | ((j >> b) << (s - x)) | ((j & ((1 << b) - 1)) << s);
     }
 };
@@ -40,17 +47,45 @@ template <typename real> struct FftMax;
 template <> struct FftMax<float> { static constexpr int C = 16; };
 template <> struct FftMax<double> { static constexpr int C = 8; };
 
-// columns per CTA: the largest power of two <= Cmax, <= 1024 / threads-per-column and <= N whose unpack tiles
-// (roots L + exchange tile L x CP + pair-(0,1) result N x CP, CP = C + 1 padding for C > 1) fit in 227 KB
+// columns per CTA: the largest power of two <= Cmax, <= 1024 / (L / 8) (L / E in the wide form, fft_cols_auto) and <= N
+// whose unpack tiles (roots L + exchange tile L x CP + N x CP, CP = C + 1 padding for C > 1) fit in 227 KB
 constexpr int kSmemBudget = 227 * 1024;
 __host__ __device__ constexpr int fft_pad(int c) { return c > 1 ? c + 1 : 1; }
-template <int l> __host__ __device__ constexpr int fft_cols(int Cmax, int elem_bytes) {
-    int c = imax(1, imin(imin(Cmax, 1024 / FftCfg<l>::TPC), (1 << l) / 2));
+template <int l> __host__ __device__ constexpr int fft_fit(int c, int elem_bytes) {
     while (c > 1 && ((1 << l) + ((1 << l) + (1 << (l - 1))) * fft_pad(c)) * elem_bytes > kSmemBudget) c >>= 1;
     return c;
 }
+template <int l> __host__ __device__ constexpr int fft_cols(int Cmax, int elem_bytes) {
+    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / imax(1, (1 << l) / 8)), (1 << l) / 2)), elem_bytes);
+}
+template <int l> __host__ __device__ constexpr int fft_cols_auto(int Cmax, int elem_bytes) {
+    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / FftCfg<l>::TPC), (1 << l) / 2)), elem_bytes);
+}
 
-// all passes of the in-place DIT transform on the registers x[] of (column c, column-thread t)
+// cos and sin of 2 pi k / 16, k < 8
+template <typename real> __device__ __forceinline__ cplx<real> root16(int k) {
+    constexpr double c1 = 0.92387953251128675613, c2 = 0.70710678118654752440, c3 = 0.38268343236508977173;
+    const double re[8] = {1, c1, c2, c3, 0, -c3, -c2, -c1}, im[8] = {0, c3, c2, c1, 1, c1, c2, c3};
+    return mk<real>((real)re[k], (real)im[k]);
+}
+// x times exp(-+ 2 pi i k / 2^m) (INV: +), k < 2^(m-1), m <= 4, k and m constants: trivial rotations cost no multiply
+template <typename real, bool INV> __device__ __forceinline__ cplx<real> rotate(cplx<real> x, int k, int m) {
+    const int k16 = k << (4 - m);
+    if (k16 == 0) return x;
+    if (k16 == 4) return INV ? mk<real>(-x.y, x.x) : mk<real>(x.y, -x.x);
+    cplx<real> w = root16<real>(k16);
+    if (k16 == 2 || k16 == 6) {  // +-sqrt(1/2) (1 +- i)
+        const real h = root16<real>(2).x;
+        const real a = h * (x.x - x.y), b = h * (x.x + x.y);
+        if (k16 == 2) return INV ? mk<real>(a, b) : mk<real>(b, -a);
+        return INV ? mk<real>(-b, a) : mk<real>(-a, -b);
+    }
+    if (!INV) w.y = -w.y;
+    return cmul(w, x);
+}
+
+// all passes of the in-place DIT transform on the registers x[] of (column c, column-thread t); the caller loads x[j]
+// with input brev(pos(0, t, j)) and finds output pos(NPASS - 1, t, j) in x[j]
 template <typename real, int l, bool INV>
 __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const cplx<real>* __restrict__ roots,
                                            cplx<real>* tile, int CP, int c, int t) {
@@ -58,6 +93,7 @@ __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const 
     using C = cplx<real>;
 #pragma unroll
     for (int q = 0; q < F::NPASS; ++q) {
+        const int s = F::s0(q), b = F::nb(q);
         if (q > 0) {
             __syncthreads();
 #pragma unroll
@@ -65,19 +101,24 @@ __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const 
             __syncthreads();
 #pragma unroll
             for (int j = 0; j < F::E; ++j) x[j] = tile[F::pos(q, t, j) * CP + c];
+            // twiddles of the pass: W_(2^(s+b))^(low brev_b(j)), low = the position below the pass's bits
+#pragma unroll
+            for (int j = 0; j < F::E; ++j) {
+                const int m = brev(j & ((1 << b) - 1), b);
+                if (m == 0) continue;
+                const int low = F::pos(q, t, j) & ((1 << s) - 1);
+                C w = roots[low * m * (F::L >> (s + b))];
+                if (!INV) w.y = -w.y;
+                x[j] = cmul(w, x[j]);
+            }
         }
-        const int s = F::s0(q), b = F::nb(q);
 #pragma unroll
         for (int rb = 0; rb < b; ++rb) {
-            const int sg = s + rb;  // stage bit
 #pragma unroll
             for (int j = 0; j < F::E; ++j) {
                 if (j & (1 << rb)) continue;
-                const int p = F::pos(q, t, j);
-                C w = roots[(p & ((1 << sg) - 1)) * (F::L >> (sg + 1))];
-                if (!INV) w.y = -w.y;
                 const C u = x[j];
-                const C v = cmul(w, x[j | (1 << rb)]);
+                const C v = rotate<real, INV>(x[j | (1 << rb)], j & ((1 << rb) - 1), rb + 1);
                 x[j] = cadd(u, v);
                 x[j | (1 << rb)] = csub(u, v);
             }
@@ -85,11 +126,13 @@ __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const 
     }
 }
 
-// threads of a CTA and the CTAs per SM the register budget is sized for (the whole SM's 2048 threads in FP32)
+// threads of a CTA and the CTAs per SM the register budget is sized for
 template <typename real, int l, int CB> struct FftLaunch {
     static constexpr int threads = CB * FftCfg<l>::TPC;
-    static constexpr int pack_min = sizeof(real) == 4 ? imax(1, 2048 / threads) : imax(1, 1024 / threads);
-    static constexpr int unpack_min = imax(1, 1024 / threads);
+    // threads per SM: 64 registers each for 8 points in FP32, twice that for 16 points or FP64
+    static constexpr int resident = sizeof(real) == 4 && FftCfg<l>::e < 4 ? 1024 : 512;
+    static constexpr int pack_min = imax(1, (FftCfg<l>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads);
+    static constexpr int unpack_min = imax(1, resident / threads);
 };
 
 template <typename real, int l, int CB, typename SRC>
@@ -103,136 +146,79 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<rea
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* roots = reinterpret_cast<C*>(smem_raw);
     C* tile = roots + L;
+    real* strip = reinterpret_cast<real*>(tile);  // N x CP reals: the row quadrant's strip, before the first exchange
     const int c0 = blockIdx.x * CB;
     const int pair = blockIdx.y;
     const int img = blockIdx.z;
-    constexpr int nthr = CB * F::TPC;  // L * CB elements per gather = E per thread
+    constexpr int nthr = CB * F::TPC;
     for (int i = threadIdx.x; i < L; i += nthr) roots[i] = roots_g[i];
-
-    // ---- gather the packed strips of columns c0..c0+CB-1 into tile[i][c]; every thread issues its E loads before
-    // its shared-memory stores (E independent loads in flight)
-    if (src_kind == 0 && CB % 2 == 0) {
-        // two neighbouring elements per load: column pairs of the column reads, offset pairs of the row reads
+    const int c = threadIdx.x % CB, t = threadIdx.x / CB;
+    // input index of register j: brev(pos(0, t, j)) = brev_e(j) L/E + brev(t)
+    const int rt = F::TPC > 1 ? (int)(__brev((unsigned)t) >> (32 - (F::TPC > 1 ? l - F::e : 1))) : 0;
+    C x[F::E];
+    if (src_kind == 0) {
+        const size_t ib = (size_t)img * src_stride;
+        // column reads: pair 0 imag = x[N-1-i, c] (quadrant II), pair 1 real = x[i, c] (quadrant III)
+        real col[F::E];
+#pragma unroll
+        for (int j = 0; j < F::E; ++j) {
+            const int i = brev(j, F::e) * (L / F::E) + rt;
+            col[j] = 0;
+            if (2 * brev(j, F::e) < F::E) col[j] = (real)src[ib + (size_t)(pair == 0 ? N - 1 - i : i) * N + c0 + c];
+        }
+        // row reads: pair 0 real = x[c, N-1-i] (quadrant I), pair 1 imag = x[N-1-c, N-1-i] (quadrant IV); two
+        // neighbouring elements (offsets i + 1, i) per load where the image is aligned for it
+        const bool aligned = (reinterpret_cast<uintptr_t>(src) & (2 * sizeof(SRC) - 1)) == 0;
         using S2 = typename std::conditional<sizeof(SRC) == 8, double2, float2>::type;
-        constexpr int HC = CB / 2, HE = F::E / 2, HL = L / 2;
-        const size_t ib = (size_t)img * src_stride;
-        // column reads: pair 0 imag = x[N-1-i, c] (quadrant II), pair 1 real = x[i, c] (quadrant III)
-        real va[HE], vb[HE];
+        constexpr int HN = N / 2, PER = (HN * CB + nthr - 1) / nthr;
+        S2 v[PER];
 #pragma unroll
-        for (int k = 0; k < HE; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = 2 * (e % HC), i = e / HC;
-            va[k] = 0;
-            vb[k] = 0;
-            if (i < N) {
-                const S2 w = *reinterpret_cast<const S2*>(src + ib + (size_t)(pair == 0 ? N - 1 - i : i) * N + c0 + c);
-                va[k] = (real)w.x;
-                vb[k] = (real)w.y;
+        for (int k = 0; k < PER; ++k) {
+            const int e = threadIdx.x + k * nthr, i = 2 * (e % HN), cc = e / HN;
+            if (HN * CB % nthr == 0 || e < HN * CB) {
+                const int rowx = (pair == 0) ? (c0 + cc) : (N - 1 - c0 - cc);
+                const SRC* s2 = src + ib + (size_t)rowx * N + (N - 2 - i);
+                if (aligned) {
+                    v[k] = *reinterpret_cast<const S2*>(s2);
+                } else {
+                    v[k].x = s2[0];
+                    v[k].y = s2[1];
+                }
             }
         }
 #pragma unroll
-        for (int k = 0; k < HE; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = 2 * (e % HC), i = e / HC;
-            if (pair == 0) {
-                tile[i * CP + c].y = va[k];
-                tile[i * CP + c + 1].y = vb[k];
-            } else {
-                tile[i * CP + c].x = va[k];
-                tile[i * CP + c + 1].x = vb[k];
+        for (int k = 0; k < PER; ++k) {
+            const int e = threadIdx.x + k * nthr, i = 2 * (e % HN), cc = e / HN;
+            if (HN * CB % nthr == 0 || e < HN * CB) {
+                strip[i * CP + cc] = (real)v[k].y;
+                strip[(i + 1) * CP + cc] = (real)v[k].x;
             }
         }
-        // row reads: pair 0 real = x[c, N-1-i] (quadrant I), pair 1 imag = x[N-1-c, N-1-i] (quadrant IV); the pair
-        // (i, i+1) is the element pair (N-2-i, N-1-i) of the image row
+        __syncthreads();
 #pragma unroll
-        for (int k = 0; k < HE; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int i = 2 * (e % HL), c = e / HL;
-            va[k] = 0;
-            vb[k] = 0;
-            if (i < N) {
-                const int rowx = (pair == 0) ? (c0 + c) : (N - 1 - c0 - c);
-                const S2 w = *reinterpret_cast<const S2*>(src + ib + (size_t)rowx * N + (N - 2 - i));
-                va[k] = (real)w.y;  // offset i
-                vb[k] = (real)w.x;  // offset i + 1
+        for (int j = 0; j < F::E; ++j) {
+            const int i = brev(j, F::e) * (L / F::E) + rt;
+            x[j] = mk<real>(0, 0);
+            if (2 * brev(j, F::e) < F::E) {
+                const real row = strip[i * CP + c];
+                x[j] = pair == 0 ? mk<real>(row, col[j]) : mk<real>(col[j], row);
             }
-        }
-#pragma unroll
-        for (int k = 0; k < HE; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int i = 2 * (e % HL), c = e / HL;
-            if (pair == 0) {
-                tile[i * CP + c].x = va[k];
-                tile[(i + 1) * CP + c].x = vb[k];
-            } else {
-                tile[i * CP + c].y = va[k];
-                tile[(i + 1) * CP + c].y = vb[k];
-            }
-        }
-    } else if (src_kind == 0) {
-        const size_t ib = (size_t)img * src_stride;
-        // column reads: pair 0 imag = x[N-1-i, c] (quadrant II), pair 1 real = x[i, c] (quadrant III)
-        real v[F::E];
-#pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = e % CB, i = e / CB;
-            v[k] = 0;
-            if (i < N) v[k] = (real)src[ib + (size_t)(pair == 0 ? N - 1 - i : i) * N + c0 + c];
-        }
-#pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = e % CB, i = e / CB;
-            if (pair == 0) tile[i * CP + c].y = v[k]; else tile[i * CP + c].x = v[k];
-        }
-        // row reads: pair 0 real = x[c, N-1-i] (quadrant I), pair 1 imag = x[N-1-c, N-1-i] (quadrant IV)
-#pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int i = e % L, c = e / L;
-            v[k] = 0;
-            if (i < N) {
-                const int rowx = (pair == 0) ? (c0 + c) : (N - 1 - c0 - c);
-                v[k] = (real)src[ib + (size_t)rowx * N + (N - 1 - i)];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int i = e % L, c = e / L;
-            if (pair == 0) tile[i * CP + c].x = v[k]; else tile[i * CP + c].y = v[k];
         }
     } else {
         // iota of the sinogram quadrants qa = 2*pair, qb = 2*pair+1: S[i] = b[i+N-1] (i < N), 0 (i = N), b[i-N-1]
         const size_t H = 2 * (size_t)N - 1;
         const size_t ba = ((size_t)img * 4 + 2 * pair) * H * N, bb = ba + H * N;
-        real va[F::E], vb[F::E];
 #pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = e % CB, i = e / CB;
-            va[k] = 0;
-            vb[k] = 0;
+        for (int j = 0; j < F::E; ++j) {
+            const int i = brev(j, F::e) * (L / F::E) + rt;
+            x[j] = mk<real>(0, 0);
             if (i != N) {
                 const size_t h = (i < N) ? (size_t)(i + N - 1) : (size_t)(i - N - 1);
-                va[k] = (real)src[ba + h * N + c0 + c];
-                vb[k] = (real)src[bb + h * N + c0 + c];
+                x[j] = mk<real>((real)src[ba + h * N + c0 + c], (real)src[bb + h * N + c0 + c]);
             }
         }
-#pragma unroll
-        for (int k = 0; k < F::E; ++k) {
-            const int e = threadIdx.x + k * nthr;
-            const int c = e % CB, i = e / CB;
-            tile[i * CP + c] = mk<real>(va[k], vb[k]);
-        }
+        __syncthreads();  // roots
     }
-    __syncthreads();
-
-    const int c = threadIdx.x % CB, t = threadIdx.x / CB;
-    C x[F::E];
-#pragma unroll
-    for (int j = 0; j < F::E; ++j) x[j] = tile[(__brev((unsigned)F::pos(0, t, j)) >> (32 - l)) * CP + c];
     dit_passes<real, l, false>(x, roots, tile, CP, c, t);
     C* out = Y + ((size_t)img * 2 * L + (size_t)pair * L) * N + c0 + c;
 #pragma unroll
@@ -245,46 +231,59 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<rea
                        real* __restrict__ row3, const cplx<real>* __restrict__ roots_g) {
     using F = FftCfg<l>;
     using C = cplx<real>;
-    constexpr int L = F::L, N = L / 2;
-    constexpr int CP = fft_pad(CB);
+    constexpr int L = F::L, N = L / 2, E = F::E;
+    constexpr int CP = fft_pad(CB), RP = N + 1;  // row pitch of the transposed strips
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* roots = reinterpret_cast<C*>(smem_raw);
-    C* tile = roots + L;          // L x CP exchange tile
-    C* s01 = tile + L * CP;       // N x CP: pair (0,1) result, re = quadrant I strip, im = quadrant II strip
+    C* tile = roots + L;                              // L x CP exchange tile
+    real* rowt = reinterpret_cast<real*>(tile + L * CP);  // CB x RP: quadrant I transposed (pair (2,3) uses the tile)
     const int c0 = blockIdx.x * CB;
     const int img = blockIdx.y;
     const int nthr = CB * F::TPC;
     for (int i = threadIdx.x; i < L; i += nthr) roots[i] = roots_g[i];
-    __syncthreads();
     const int c = threadIdx.x % CB, t = threadIdx.x / CB;
     const real scale = (real)1 / (real)L;
-#pragma unroll 1
+    const size_t ib = (size_t)img * N * N;
+    real im0[E];
+#pragma unroll
     for (int pair = 0; pair < 2; ++pair) {
+        // pair (0,1) with the column's threads reversed: output p of thread t is then N-1-p of pair (2,3)'s
+        const int tt = pair == 0 ? F::TPC - 1 - t : t;
+        const int rt = F::TPC > 1 ? (int)(__brev((unsigned)tt) >> (32 - (F::TPC > 1 ? l - F::e : 1))) : 0;
         const C* in = Z + ((size_t)img * 2 * L + (size_t)pair * L) * N + c0 + c;
-        C x[F::E];
+        C x[E];
 #pragma unroll
-        for (int j = 0; j < F::E; ++j) x[j] = in[(size_t)(__brev((unsigned)F::pos(0, t, j)) >> (32 - l)) * N];
-        dit_passes<real, l, true>(x, roots, tile, CP, c, t);
-        C* dst = pair == 0 ? s01 : tile;  // pair (2,3) lands in the first N rows of the exchange tile
-        __syncthreads();
+        for (int j = 0; j < E; ++j) x[j] = in[(size_t)(brev(j, F::e) * (L / E) + rt) * N];
+        if (pair == 0) __syncthreads();  // roots
+        dit_passes<real, l, true>(x, roots, tile, CP, c, tt);
+        real* rows = rowt;
+        if (pair == 1) {
+            __syncthreads();  // the exchange tile is free
+            rows = reinterpret_cast<real*>(tile);
+        }
+        constexpr int bl = F::nb(F::NPASS - 1), top = 1 << (bl - 1);  // register bit of the offset's top bit
 #pragma unroll
-        for (int j = 0; j < F::E; ++j) {
-            const int p = F::pos(F::NPASS - 1, t, j);
-            if (p < N) dst[p * CP + c] = cscale(scale, x[j]);
+        for (int j = 0; j < E; ++j) {
+            if (j & top) continue;  // offsets >= N
+            const int p = F::pos(F::NPASS - 1, tt, j);
+            if (pair == 0) {
+                rows[c * RP + (N - 1 - p)] = scale * x[j].x;
+                im0[j] = scale * x[j].y;
+            } else {
+                rows[c * RP + (N - 1 - p)] = scale * x[j].y;
+                // colpart[i][c0+c] = S_III[i][c] + S_II[N-1-i][c]: the register of the complementary offset
+                const int jc = (E - 1 - j) & ~top;
+                colpart[ib + (size_t)p * N + c0 + c] = scale * x[j].x + im0[jc];
+            }
         }
     }
     __syncthreads();
-    // colpart[i][c0+c] = S_III[i][c] + S_II[N-1-i][c]
-    const size_t ib = (size_t)img * N * N;
-    for (int e = threadIdx.x; e < N * CB; e += nthr) {
-        const int cc = e % CB, i = e / CB;
-        colpart[ib + (size_t)i * N + c0 + cc] = tile[i * CP + cc].x + s01[(N - 1 - i) * CP + cc].y;
-    }
     // rowpart0[c0+c][N-1-r] = S_I[r][c] ; rowpart3[N-1-c0-c][N-1-r] = S_IV[r][c]
+    const real* r3 = reinterpret_cast<const real*>(tile);
     for (int e = threadIdx.x; e < N * CB; e += nthr) {
         const int r = e % N, cc = e / N;
-        row0[ib + (size_t)(c0 + cc) * N + (N - 1 - r)] = s01[r * CP + cc].x;
-        row3[ib + (size_t)(N - 1 - c0 - cc) * N + (N - 1 - r)] = tile[r * CP + cc].y;
+        row0[ib + (size_t)(c0 + cc) * N + r] = rowt[cc * RP + r];
+        row3[ib + (size_t)(N - 1 - c0 - cc) * N + r] = r3[cc * RP + r];
     }
 }
 
@@ -292,11 +291,13 @@ template <typename real, int l, int CB> static size_t pack_smem() {
     return ((size_t)(1 << l) + (size_t)(1 << l) * fft_pad(CB)) * sizeof(cplx<real>);
 }
 template <typename real, int l, int CB> static size_t unpack_smem() {
-    return ((size_t)(1 << l) + ((size_t)(1 << l) + (size_t)(1 << (l - 1))) * fft_pad(CB)) * sizeof(cplx<real>);
+    return ((size_t)(1 << l) + (size_t)(1 << l) * fft_pad(CB)) * sizeof(cplx<real>) +
+           (size_t)CB * ((1 << (l - 1)) + 1) * sizeof(real);
 }
 
-// columns per CTA: the default (as many as fit, up to 16 FP32 / 8 FP64) or a quarter of it (narrower CTAs, more of
-// them per SM, so the load, transform and store phases of different CTAs overlap); cols = 0 picks the default
+// columns per CTA: cols = 0 picks as many as fit, up to 16 FP32 / 8 FP64; the autotuner's choices are the widths of 8
+// points per thread and a quarter of them (narrower CTAs, more of them per SM)
+template <typename real, int l> constexpr int cols_auto() { return fft_cols_auto<l>(FftMax<real>::C, sizeof(cplx<real>)); }
 template <typename real, int l> constexpr int cols_wide() { return fft_cols<l>(FftMax<real>::C, sizeof(cplx<real>)); }
 template <typename real, int l> constexpr int cols_narrow() { return imax(1, cols_wide<real, l>() / 4); }
 
@@ -318,9 +319,10 @@ static int launch_pack_cb(int nimg, int src_kind, const void* src, long long src
 template <typename real, int l, typename SRC>
 static int launch_pack_src(int nimg, int src_kind, const void* src, long long src_stride, void* Y, const void* roots,
                            int cols, cudaStream_t st) {
-    constexpr int W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
-    if (cols == 0 || cols == W) return launch_pack_cb<real, l, W, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
-    if (NW != W && cols == NW) return launch_pack_cb<real, l, NW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
+    if (cols == 0 || cols == A) return launch_pack_cb<real, l, A, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    if (W != A && cols == W) return launch_pack_cb<real, l, W, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    if (NW != W && NW != A && cols == NW) return launch_pack_cb<real, l, NW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
     set_error("pack_fft: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
     return ADRT_EINVAL;
 }
@@ -350,9 +352,10 @@ static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, 
 template <typename real, int l>
 static int launch_unpack(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots, int cols,
                          cudaStream_t st) {
-    constexpr int W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
-    if (cols == 0 || cols == W) return launch_unpack_cb<real, l, W>(nimg, Z, colpart, row0, row3, roots, st);
-    if (NW != W && cols == NW) return launch_unpack_cb<real, l, NW>(nimg, Z, colpart, row0, row3, roots, st);
+    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
+    if (cols == 0 || cols == A) return launch_unpack_cb<real, l, A>(nimg, Z, colpart, row0, row3, roots, st);
+    if (W != A && cols == W) return launch_unpack_cb<real, l, W>(nimg, Z, colpart, row0, row3, roots, st);
+    if (NW != W && NW != A && cols == NW) return launch_unpack_cb<real, l, NW>(nimg, Z, colpart, row0, row3, roots, st);
     set_error("ifft_unpack: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
     return ADRT_EINVAL;
 }
