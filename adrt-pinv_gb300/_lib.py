@@ -80,9 +80,9 @@ PROTOTYPES = {
     "adrt_rows_multi_code": [ctypes.POINTER(RowJob)],
     "adrt_rows_lanes_per_row": [_I],
     "adrt_rows_run_multi": [_P, _P, _P, _I, _P, _I, _P],
-    "adrt_rows_operator": [_I, _I, _I, _P, _P, _L, _P, _P],
+    "adrt_rows_operator": [_I, _I, _I, _I, _P, _P, _L, _P, _P],
     "adrt_rows_operator_split": [_I, _P, _P, _P, _P],
-    "adrt_rows_operator_mma": [_I, _I, _P, _P, _P, _L, _P, _P, _P],
+    "adrt_rows_operator_mma": [_I, _I, _I, _P, _P, _P, _L, _P, _P, _P],
     "adrt_twiddle_table": [_I, _I, _I, _P, _P, _P],
     "adrt_power_rows": [_I, _I, _I, _P, _P, _I, _I, _D, _P, _P, _P],
     "adrt_cert_rowsum_dev": [_I, _I, _P, _I, _P, _P],

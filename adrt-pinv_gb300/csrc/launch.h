@@ -39,7 +39,7 @@ int ff_to_f64(int n, int nimg, const float* x, double* out, cudaStream_t st);
 int dense_rows(int dtype, int n, int nimg, int nrows, const int* rows, const void* W, void* Y, long long img_stride,
                void* Zd, int* err, int use_tc, int tile, cudaStream_t st);
 int dense_split(int n, int nrows, const void* W, void* Ws, cudaStream_t st);
-int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride, const void* half,
+int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp,
                   cudaStream_t st);
 int cert_rowsum_dev(int n, int K, const double* omega, int m_lo, double* out, cudaStream_t st);
 }  // namespace adrt

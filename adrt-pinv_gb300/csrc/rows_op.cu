@@ -1,19 +1,20 @@
-// Row operators: one pass G (the op lists [B_1] P M [B_1^*] of the hybrid's G_h and of the L_p frame operator,
-// fastops.py:277-281, 325-331) on the packed rows as one small real matrix per frequency instead of d_k fused Gram
-// passes.
+// Row operators: one packed pass (op list) as one small real matrix pair per frequency instead of d_k fused Gram passes.
 //
-// The operator of frequency k is T_k = B_1^* M p_k(M) B_1 (or M p_k(M)), M = A^* A with A_{s,c} = z_k^{off(s,c)} over
-// the digital lines. A line of slope s and its complement N-1-s have offsets that add up to c, so conjugating T_k with
-// the half-shift phases D = diag(z_k^{c/2}) makes it REAL: T_k = D^* R_k D. Reversing a line, off(s, N-1-c) =
-// s - off(s, c), makes R_k centro-symmetric: R_k(N-1-c, N-1-j) = R_k(c, j). So with H = N/2, a = D y,
+// G, the op lists [B_1] P M [B_1^*] of the hybrid's G_h and of the L_p frame operator (fastops.py:277-281, 325-331): the
+// operator of frequency k is T_k = B_1^* M p_k(M) B_1 (or M p_k(M)), M = A^* A with A_{s,c} = z_k^{off(s,c)} over the
+// digital lines. A line of slope s and its complement N-1-s have offsets that add up to c, so conjugating T_k with the
+// half-shift phases D = diag(z_k^{c/2}) makes it REAL: T_k = D^* R_k D. Reversing a line, off(s, N-1-c) = s - off(s, c),
+// makes R_k centro-symmetric: R_k(N-1-c, N-1-j) = R_k(c, j). So with H = N/2, a = D y,
 //     E_j = a_j + a_{N-1-j},  O_j = a_j - a_{N-1-j},   e = T_e E,  o = T_o O   (two real H x H matrices)
-//     z_c = conj(D_c) (e_c + o_c),   z_{N-1-c} = conj(D_{N-1-c}) (e_c - o_c)        (c, j < H)
-// and R_{-k} = R_k with D conjugated, so the rows k and L-k of both quadrant pairs of every image share one pair of
-// matrices: 4 B complex vectors per frequency 0 < k < N (2 B at k = 0 and N, which are their own negatives). A row
-// costs N^2/2 complex-by-real multiply-adds (N^2 real FMAs) whatever its degree; the polynomial needs
-// 4 N (n - 1) FMAs per Gram and d_k of them (mean degree 7 at N = 256: 100 k against 66 k), and the filter's
-// ill-conditioned rows lose nothing to the recurrence, because the matrices are evaluated in FP64 when the plan's
-// tables are built.
+//     z_c = conj(D_c) (e_c + o_c),   z_{N-1-c} = conj(D_{N-1-c}) (e_c - o_c)        (c, j < H).
+// BP, the back-projections' [A^*] P [B_1^*] (fastops.py:283-285, 333-335), takes rows in slope order: rotating slope s by
+// beta_s = z_k^{(2s-N+1)/4} makes the complementary slopes' rows of A D^* conjugates of one another and each of them
+// conjugate-symmetric in c, so the same form holds with a = conj(beta) y and O_s = -i (a_s - a_{N-1-s}).
+// The operators of -k are the conjugates, so the rows k and L-k of both quadrant pairs of every image (the latter
+// conjugated on the way in and out) share one pair of matrices: 4 B complex vectors per frequency 0 < k < N (2 B at k = 0
+// and N, which are their own negatives). A row costs N^2 real FMAs whatever its degree; the polynomial needs 4 N (n - 1)
+// FMAs per Gram and d_k of them (mean degree 7 at N = 256: 100 k against 66 k), and the filter's ill-conditioned rows lose
+// nothing to the recurrence, because the matrices are evaluated in FP64 when the plan's tables are built.
 //
 // Two kernels, both in place (a CTA reads whole rows before it writes them):
 //  rows_op_small  few vectors (and FP64): bounded by reading the matrices (N^2/2 values per frequency, 34 MB in FP32
@@ -25,14 +26,15 @@
 //                 products (128 FMAs per eight 16-byte shared loads), so e_c and o_c meet in registers.
 #include "common.cuh"
 #include "launch.h"
+#include "rows_op.cuh"
 
 namespace adrt {
 
 template <int n> struct OpCfg {
-    static constexpr int N = 1 << n, H = N / 2, L = 2 * N;
+    static constexpr int N = 1 << n, H = N / 2;
 };
 
-// vector v of frequency k: image, packed row and whether the row is that of -k (its phases are conjugated)
+// vector v of frequency k: image, packed row and whether the row is that of -k (it enters and leaves conjugated)
 struct OpVec {
     int img, row;
     bool neg;
@@ -55,10 +57,10 @@ template <typename C> __device__ __forceinline__ C conj_if(C a, bool c) {
 // E and O of VT vectors (zero beyond nv) into shared memory as [j][vector] complex, row stride RS complex
 template <typename real, int n, int VT, int THREADS, int RS>
 __device__ __forceinline__ void op_load(const cplx<real>* __restrict__ Y, long long img_stride,
-                                        const cplx<real>* __restrict__ half, int k, int v0, int nv, cplx<real>* E,
-                                        cplx<real>* O) {
+                                        const cplx<real>* __restrict__ roots, bool bp, int k, int v0, int nv,
+                                        cplx<real>* E, cplx<real>* O) {
     using C = cplx<real>;
-    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H, MASK = 2 * OpCfg<n>::L - 1;
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H;
 #pragma unroll 4
     for (int e = threadIdx.x; e < VT * H; e += THREADS) {
         const int v = e / H, c = e % H;
@@ -66,20 +68,21 @@ __device__ __forceinline__ void op_load(const cplx<real>* __restrict__ Y, long l
         if (v0 + v < nv) {
             const OpVec w = op_vec<n>(k, v0 + v);
             const C* y = Y + (long long)w.img * img_stride + (long long)w.row * N;
-            a = cmul(conj_if(half[(k * c) & MASK], w.neg), y[c]);
-            b = cmul(conj_if(half[(k * (N - 1 - c)) & MASK], w.neg), y[N - 1 - c]);
+            a = cmul(roots[op_phase_in<n>(k, c, bp)], conj_if(y[c], w.neg));
+            b = cmul(roots[op_phase_in<n>(k, N - 1 - c, bp)], conj_if(y[N - 1 - c], w.neg));
         }
+        const C d = csub(a, b);
         E[c * RS + v] = cadd(a, b);
-        O[c * RS + v] = csub(a, b);
+        O[c * RS + v] = bp ? mk<real>(d.y, -d.x) : d;
     }
 }
 
 // ------------------------------------------------------------------ few vectors, or FP64
 template <typename real, int n, int VT>
 __global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __restrict__ T, cplx<real>* Y,
-                                                     long long img_stride, const cplx<real>* __restrict__ half) {
+                                                     long long img_stride, const cplx<real>* __restrict__ roots, bool bp) {
     using C = cplx<real>;
-    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H, MASK = 2 * OpCfg<n>::L - 1;
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H;
     constexpr int CG = H / 4;              // groups of four outputs c
     constexpr int KS = CG >= 256 ? 1 : 256 / CG;  // slices of the sum over j
     constexpr int VB = VT < 4 ? VT : 4;    // vectors per reduction round
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __res
     const int k = blockIdx.y, v0 = blockIdx.x * VT;
     const int nv = nimg * ((k == 0 || k == N) ? 2 : 4);
     if (v0 >= nv) return;
-    op_load<real, n, VT, 256, VT>(Y, img_stride, half, k, v0, nv, E, O);
+    op_load<real, n, VT, 256, VT>(Y, img_stride, roots, bp, k, v0, nv, E, O);
     __syncthreads();
 
     const int cg = threadIdx.x % CG, ks = threadIdx.x / CG;
@@ -140,8 +143,8 @@ __global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __res
             }
             const OpVec w = op_vec<n>(k, v0 + vb + v);
             C* y = Y + (long long)w.img * img_stride + (long long)w.row * N;
-            y[c] = cmul(conj_if(half[(k * c) & MASK], !w.neg), cadd(se, so));
-            y[N - 1 - c] = cmul(conj_if(half[(k * (N - 1 - c)) & MASK], !w.neg), csub(se, so));
+            y[c] = conj_if(cmulc(roots[op_phase_out<n>(k, c)], cadd(se, so)), w.neg);
+            y[N - 1 - c] = conj_if(cmulc(roots[op_phase_out<n>(k, N - 1 - c)], csub(se, so)), w.neg);
         }
     }
 }
@@ -167,10 +170,11 @@ template <int n> struct OpTile {
 
 template <int n>
 __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
-    rows_op_tile(int nimg, const float* __restrict__ T, float2* Y, long long img_stride, const float2* __restrict__ half) {
+    rows_op_tile(int nimg, const float* __restrict__ T, float2* Y, long long img_stride, const float2* __restrict__ roots,
+                 bool bp) {
     using W = OpTile<n>;
     constexpr int N = OpCfg<n>::N, H = W::H, VT = W::VT, RS = W::RS, KC = W::KC, S = W::STAGES;
-    constexpr int MASK = 2 * OpCfg<n>::L - 1, NCH = H / KC;
+    constexpr int NCH = H / KC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* ring = reinterpret_cast<float*>(smem_raw);
     float2* E = reinterpret_cast<float2*>(ring + S * W::STAGE);
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
     };
 #pragma unroll
     for (int ch = 0; ch < S - 1; ++ch) fetch(ch);
-    op_load<float, n, VT, W::THREADS, RS>(Y, img_stride, half, k, v0, nv, E, O);
+    op_load<float, n, VT, W::THREADS, RS>(Y, img_stride, roots, bp, k, v0, nv, E, O);
 
     const int cg = threadIdx.x % W::CGS, vg = threadIdx.x / W::CGS;
     const int c0 = 4 * cg, u0 = 2 * vg;
@@ -236,8 +240,8 @@ __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
         float2 pa[4], pb[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            pa[q] = half[(k * (cr + q)) & MASK];
-            pb[q] = half[(k * (N - 1 - cr - q)) & MASK];
+            pa[q] = roots[op_phase_out<n>(k, cr + q)];
+            pb[q] = roots[op_phase_out<n>(k, N - 1 - cr - q)];
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -248,8 +252,8 @@ __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
             float2 za[4], zb[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                za[q] = cmul(conj_if(pa[q], !w.neg), cadd(ae[run * 4 + q][v], ao[run * 4 + q][v]));
-                zb[q] = cmul(conj_if(pb[q], !w.neg), csub(ae[run * 4 + q][v], ao[run * 4 + q][v]));
+                za[q] = conj_if(cmulc(pa[q], cadd(ae[run * 4 + q][v], ao[run * 4 + q][v])), w.neg);
+                zb[q] = conj_if(cmulc(pb[q], csub(ae[run * 4 + q][v], ao[run * 4 + q][v])), w.neg);
             }
             float4* lo = reinterpret_cast<float4*>(y + cr);
             lo[0] = make_float4(za[0].x, za[0].y, za[1].x, za[1].y);
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
 
 // ------------------------------------------------------------------ dispatch
 template <typename real, int n, int VT>
-static int launch_small(int nimg, const void* T, void* Y, long long img_stride, const void* half, cudaStream_t st) {
+static int launch_small(int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp, cudaStream_t st) {
     constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H;
     constexpr int KS = 1024 / H, VB = VT < 4 ? VT : 4;
     const size_t smem = (size_t)(2 * H * VT + KS * 2 * VB * H) * sizeof(cplx<real>);
@@ -271,37 +275,37 @@ static int launch_small(int nimg, const void* T, void* Y, long long img_stride, 
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     kern<<<dim3((4 * nimg + VT - 1) / VT, N + 1), 256, smem, st>>>(nimg, reinterpret_cast<const real*>(T),
                                                                    reinterpret_cast<cplx<real>*>(Y), img_stride,
-                                                                   reinterpret_cast<const cplx<real>*>(half));
+                                                                   reinterpret_cast<const cplx<real>*>(roots), bp);
     return launch_status("rows_op_small");
 }
 
 template <int n>
-static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, const void* half, cudaStream_t st) {
+static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp, cudaStream_t st) {
     using W = OpTile<n>;
     auto kern = rows_op_tile<n>;
     if (int rc = ensure_smem((const void*)kern, W::smem)) return rc;
     kern<<<dim3((4 * nimg + W::VT - 1) / W::VT, W::H * 2 + 1), W::THREADS, W::smem, st>>>(
         nimg, reinterpret_cast<const float*>(T), reinterpret_cast<float2*>(Y), img_stride,
-        reinterpret_cast<const float2*>(half));
+        reinterpret_cast<const float2*>(roots), bp);
     return launch_status("rows_op_tile");
 }
 
 template <int n>
-static int rows_operator_n(int dtype, int nimg, const void* T, void* Y, long long img_stride, const void* half,
+static int rows_operator_n(int dtype, int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp,
                            cudaStream_t st) {
     if (dtype == ADRT_F64) {
-        if (nimg == 1) return launch_small<double, n, 2>(nimg, T, Y, img_stride, half, st);
-        return launch_small<double, n, 4>(nimg, T, Y, img_stride, half, st);
+        if (nimg == 1) return launch_small<double, n, 2>(nimg, T, Y, img_stride, roots, bp, st);
+        return launch_small<double, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
     }
-    if (nimg == 1) return launch_small<float, n, 4>(nimg, T, Y, img_stride, half, st);
-    if (4 * nimg <= OpTile<n>::VT / 2) return launch_small<float, n, 8>(nimg, T, Y, img_stride, half, st);
-    return launch_tile<n>(nimg, T, Y, img_stride, half, st);
+    if (nimg == 1) return launch_small<float, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
+    if (4 * nimg <= OpTile<n>::VT / 2) return launch_small<float, n, 8>(nimg, T, Y, img_stride, roots, bp, st);
+    return launch_tile<n>(nimg, T, Y, img_stride, roots, bp, st);
 }
 
-int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride, const void* half,
+int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp,
                   cudaStream_t st) {
     if ((dtype != ADRT_F32 && dtype != ADRT_F64) || n < 6 || n > 9 || nimg < 0 || nimg > 65535 ||
-        (nimg && (!T || !Y || !half))) {
+        (nimg && (!T || !Y || !roots))) {
         set_error("rows_operator: bad arguments (dtype=%d n=%d nimg=%d; n must be 6..9)", dtype, n, nimg);
         return ADRT_EINVAL;
     }
@@ -311,16 +315,20 @@ int rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long 
     }
     if (!nimg) return ADRT_OK;
     switch (n) {
-        case 6: return rows_operator_n<6>(dtype, nimg, T, Y, img_stride, half, st);
-        case 7: return rows_operator_n<7>(dtype, nimg, T, Y, img_stride, half, st);
-        case 8: return rows_operator_n<8>(dtype, nimg, T, Y, img_stride, half, st);
-        default: return rows_operator_n<9>(dtype, nimg, T, Y, img_stride, half, st);
+        case 6: return rows_operator_n<6>(dtype, nimg, T, Y, img_stride, roots, bp, st);
+        case 7: return rows_operator_n<7>(dtype, nimg, T, Y, img_stride, roots, bp, st);
+        case 8: return rows_operator_n<8>(dtype, nimg, T, Y, img_stride, roots, bp, st);
+        default: return rows_operator_n<9>(dtype, nimg, T, Y, img_stride, roots, bp, st);
     }
 }
 
 }  // namespace adrt
 
-extern "C" int adrt_rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride,
-                                  const void* half_roots, void* stream) {
-    return adrt::rows_operator(dtype, n, nimg, T, Y, img_stride, half_roots, adrt::as_stream(stream));
+extern "C" int adrt_rows_operator(int dtype, int n, int nimg, int kind, const void* T, void* Y, long long img_stride,
+                                  const void* roots8, void* stream) {
+    if (kind != 0 && kind != 1) {
+        adrt::set_error("rows_operator: kind must be 0 (G) or 1 (BP)");
+        return ADRT_EINVAL;
+    }
+    return adrt::rows_operator(dtype, n, nimg, T, Y, img_stride, roots8, kind == 1, adrt::as_stream(stream));
 }

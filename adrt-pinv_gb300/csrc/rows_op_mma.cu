@@ -9,7 +9,7 @@
 //
 // Persistent CTAs, one per SM, warp-specialised, over units of (frequency, 32 vectors); the units of a frequency run on
 // neighbouring CTAs, which share its matrices through L2:
-//   warps 8-15  load a unit's rows (coalesced, LPV = H/8 lanes per vector), apply the half-shift phases, fold E and O,
+//   warps 8-15  load a unit's rows (coalesced, LPV = H/8 lanes per vector), apply the phases, fold E and O,
 //               scale, split and store both as K-major core matrices. K runs in the order the lanes hold the values
 //               (slot 8 l + 2 q + r is column 2 l + 2 LPV q + r; the matrices are stored in the same order), so each
 //               lane writes 16-byte pieces; core matrices lie 144 bytes apart, which makes those stores conflict-free.
@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "launch.h"
+#include "rows_op.cuh"
 #include "tcgen05.cuh"
 
 namespace adrt {
@@ -100,9 +101,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
 template <int n>
 __global__ void __launch_bounds__(OM_THREADS, 1)
     rows_op_mma_kernel(int nimg, int tiles, const __half* __restrict__ Ts, const float* __restrict__ tinv, float2* Y,
-                       long long img_stride, const float2* __restrict__ half, int* __restrict__ err) {
+                       long long img_stride, const float2* __restrict__ roots, bool bp, int* __restrict__ err) {
     using W = OmCfg<n>;
-    constexpr int N = W::N, L = W::L, VT = W::VT, LPV = W::LPV, MASK = 2 * L - 1;
+    constexpr int N = W::N, L = W::L, VT = W::VT, LPV = W::LPV;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* ring = smem_raw;
     unsigned char* bbuf = smem_raw + (size_t)W::RING * W::CHUNK * 2;
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(OM_THREADS, 1)
             const float* iv = inv + (un & 3) * VT;
             for (int mt = 0; mt < W::MT; ++mt, ++ac) {
                 const int ai = ac & 1, c = mt * 128 + (warp & 3) * 32 + lane;
-                const float2 pa = half[(k * c) & MASK], pb = half[(k * (N - 1 - c)) & MASK];
+                const float2 pa = roots[op_phase_out<n>(k, c)], pb = roots[op_phase_out<n>(k, N - 1 - c)];
                 if (!warp_wait(smem_addr(&acc_full[ai]), (uint32_t)((ac >> 1) & 1), abort_flag)) {
                     if (lane == 0) *abort_flag = 1;
                     ok = false;
@@ -298,14 +299,14 @@ __global__ void __launch_bounds__(OM_THREADS, 1)
             const int bi = un % W::NB, br = un / W::NB;
             unsigned char* B0 = bbuf + (size_t)bi * 4 * W::BT;
             float* iv = inv + (un & 3) * VT;
-            float2 pa[8], pb[8];  // phases of columns c = 2 l + 2 LPV q + r and N - 1 - c
+            float2 pa[8], pb[8];  // phases of entries c = 2 l + 2 LPV q + r and N - 1 - c
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const int c = 2 * l + 2 * LPV * q + r;
-                    pa[2 * q + r] = half[(k * c) & MASK];
-                    pb[2 * q + r] = half[(k * (N - 1 - c)) & MASK];
+                    pa[2 * q + r] = roots[op_phase_in<n>(k, c, bp)];
+                    pb[2 * q + r] = roots[op_phase_in<n>(k, N - 1 - c, bp)];
                 }
             bool waited = br == 0;
             for (int vb = (warp - 8) * VPW; vb < VT; vb += 8 * VPW) {
@@ -332,8 +333,8 @@ __global__ void __launch_bounds__(OM_THREADS, 1)
                             const float2 b = cmul(pb[i], r ? make_float2(yb[q].x, sg * yb[q].y) : make_float2(yb[q].z, sg * yb[q].w));
                             er[i] = a.x + b.x;
                             ei[i] = a.y + b.y;
-                            orr[i] = a.x - b.x;
-                            oi[i] = a.y - b.y;
+                            orr[i] = bp ? a.y - b.y : a.x - b.x;
+                            oi[i] = bp ? b.x - a.x : a.y - b.y;
                             m = fmaxf(m, fmaxf(fmaxf(fabsf(er[i]), fabsf(ei[i])), fmaxf(fabsf(orr[i]), fabsf(oi[i]))));
                         }
                 }
@@ -394,8 +395,8 @@ __global__ void __launch_bounds__(OM_THREADS, 1)
 }
 
 template <int n>
-static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long long img_stride, const void* half, int* err,
-                      cudaStream_t st) {
+static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long long img_stride, const void* roots, bool bp,
+                      int* err, cudaStream_t st) {
     using W = OmCfg<n>;
     static_assert(W::smem <= 227 * 1024, "shared memory");
     auto kern = rows_op_mma_kernel<n>;
@@ -404,7 +405,7 @@ static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long
     const int total = (W::N + 1) * tiles, sms = device_sm_count();
     kern<<<total < sms ? total : sms, OM_THREADS, W::smem, st>>>(
         nimg, tiles, reinterpret_cast<const __half*>(Ts), tinv, reinterpret_cast<float2*>(Y), img_stride,
-        reinterpret_cast<const float2*>(half), err);
+        reinterpret_cast<const float2*>(roots), bp, err);
     return launch_status("rows_op_mma_kernel");
 }
 
@@ -426,10 +427,11 @@ extern "C" int adrt_rows_operator_split(int n, const void* T, const float* scale
     return launch_status("rows_op_split_kernel");
 }
 
-extern "C" int adrt_rows_operator_mma(int n, int nimg, const void* Ts, const float* inv_scale, void* Y,
-                                      long long img_stride, const void* half_roots, int32_t* err, void* stream) {
-    if (n < 8 || n > 9 || nimg < 0 || nimg > 65535 || (nimg && (!Ts || !inv_scale || !Y || !half_roots || !err))) {
-        set_error("rows_operator_mma: bad arguments (n=%d nimg=%d; n must be 8 or 9)", n, nimg);
+extern "C" int adrt_rows_operator_mma(int n, int nimg, int kind, const void* Ts, const float* inv_scale, void* Y,
+                                      long long img_stride, const void* roots8, int32_t* err, void* stream) {
+    if (n < 8 || n > 9 || nimg < 0 || nimg > 65535 || (kind != 0 && kind != 1) ||
+        (nimg && (!Ts || !inv_scale || !Y || !roots8 || !err))) {
+        set_error("rows_operator_mma: bad arguments (n=%d nimg=%d kind=%d; n must be 8 or 9)", n, nimg, kind);
         return ADRT_EINVAL;
     }
     if ((reinterpret_cast<uintptr_t>(Y) & 15) || (reinterpret_cast<uintptr_t>(Ts) & 15) || (img_stride & 1)) {
@@ -438,6 +440,6 @@ extern "C" int adrt_rows_operator_mma(int n, int nimg, const void* Ts, const flo
     }
     if (!nimg) return ADRT_OK;
     cudaStream_t st = as_stream(stream);
-    if (n == 8) return launch_mma<8>(nimg, Ts, inv_scale, Y, img_stride, half_roots, err, st);
-    return launch_mma<9>(nimg, Ts, inv_scale, Y, img_stride, half_roots, err, st);
+    if (n == 8) return launch_mma<8>(nimg, Ts, inv_scale, Y, img_stride, roots8, kind == 1, err, st);
+    return launch_mma<9>(nimg, Ts, inv_scale, Y, img_stride, roots8, kind == 1, err, st);
 }

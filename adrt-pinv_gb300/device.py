@@ -91,10 +91,10 @@ class RowTables:
         # polynomial rows (FP64 is accurate enough there)
         self.high_poly = getattr(plan, "high_rows", "dense") == "ff" and len(plan.dense_freqs) > 0
         self.high_ff = self.high_poly and real == torch.float32
-        # one pass G as a real operator per frequency (op_table), where the plan and the size allow it
+        # the packed passes as a real operator pair per frequency (op_table), where the plan and the size allow it
         self.row_ops = row_operators_for(plan)
-        self._g_ops = fuse_ops(_op_lists(plan)["G"])
-        self._op_dev, self._half = {}, None
+        self._op_lists = {kind: fuse_ops(ops) for kind, ops in _op_lists(plan).items()}
+        self._op_dev, self._roots8 = {}, None
         self.op_mma = None  # the row operators' form: None by batch size, or True (tensor cores) / False
         if self.high_ff:
             # the compensated rows read the roots of unity and the filter constants in FP64
@@ -139,47 +139,52 @@ class RowTables:
     def _timed_main(self, Y, ops, st):
         self._timed(ops, lambda: C.call("adrt_rows_run", ctypes.byref(self.job(Y, ops, self.rows_main)), st))
 
-    def runs_operators(self, ops):
-        """Whether run() applies this op list as one real operator per frequency (the G list of the plan)."""
-        return self.row_ops and fuse_ops(ops) == self._g_ops
+    def operator_kind(self, ops):
+        """"G" or "BP" if run() applies this op list as one real operator pair per frequency (the plan's own packed
+        passes), else None."""
+        if not self.row_ops:
+            return None
+        ops = fuse_ops(ops)
+        return next((kind for kind, own in self._op_lists.items() if own == ops), None)
 
     def uses_mma(self, B):
         """Whether the row operators of a batch of B images run on the tensor cores (op_mma, when set, decides)."""
         fits = self.real == torch.float32 and self.plan.n in ROW_OPS_MMA_BATCH
         return fits and (B >= ROW_OPS_MMA_BATCH[self.plan.n] if self.op_mma is None else self.op_mma)
 
-    def op_table(self, mma=False):
-        """The plan's row operators (row_operator_table) in the row precision, or (mma) the pair (split FP16 tiles, inverse
-        scales) of the tensor-core form; shared by the plan's pipelines of that precision while any of them holds them.
-        None during a stream capture that finds them not built (the polynomial rows run instead)."""
-        if self._half is None or mma not in self._op_dev:
+    def op_table(self, kind, mma=False):
+        """The plan's row operators of a packed pass ("G" or "BP", row_operator_table) in the row precision, or (mma) the
+        split FP16 tiles of the tensor-core form with their inverse scales; shared by the plan's pipelines of that
+        precision while any of them holds them. None during a stream capture that finds them not built (the polynomial
+        rows run instead)."""
+        if self._roots8 is None or (kind, mma) not in self._op_dev:
             if torch.cuda.is_current_stream_capturing():
                 return None
-            if self._half is None:
-                self._half = torch.from_numpy(roots_of_unity(2 * self.plan.L)).to(device=self.device,
-                                                                                  dtype=_cdtype(self.real))
+            if self._roots8 is None:
+                self._roots8 = torch.from_numpy(roots_of_unity(8 * self.plan.N)).to(device=self.device,
+                                                                                    dtype=_cdtype(self.real))
             shared = self.plan.__dict__.setdefault("_dense_shared", weakref.WeakValueDictionary())
-            key = (str(self.device), str(self.real), "row_ops", mma)
+            key = (str(self.device), str(self.real), "row_ops", kind, mma)
             T = shared.get(key)
             if T is None:
-                plain = shared.get(key[:3] + (False,)) if mma else None
-                T = row_operator_table(self, self.real) if plain is None else plain
+                plain = shared.get(key[:4] + (False,)) if mma else None
+                T = row_operator_table(self, kind) if plain is None else plain
                 if mma:
                     T = _split_operators(self.plan.n, T)
                 torch.cuda.current_stream(self.device).synchronize()  # complete before another stream shares it
                 shared[key] = T
-            self._op_dev[mma] = T
-        return self._op_dev[mma]
+            self._op_dev[kind, mma] = T
+        return self._op_dev[kind, mma]
 
-    def run_operators(self, Y, T):
-        """Y[b, r] <- T_k Y[b, r] for every packed row, in place (T: op_table of this batch size)."""
+    def run_operators(self, Y, kind, T):
+        """Y[b, r] <- T_k Y[b, r] for every packed row, in place (T: op_table of this pass and batch size)."""
         B, R, N = Y.shape
-        st = C.stream_handle()
+        st, code = C.stream_handle(), 0 if kind == "G" else 1
         if self.uses_mma(B):
-            C.call("adrt_rows_operator_mma", self.plan.n, B, C.ptr(T), C.ptr(T._adrt_inv_scale), C.ptr(Y), R * N,
-                   C.ptr(self._half), C.ptr(self.err), st)
+            C.call("adrt_rows_operator_mma", self.plan.n, B, code, C.ptr(T), C.ptr(T._adrt_inv_scale), C.ptr(Y), R * N,
+                   C.ptr(self._roots8), C.ptr(self.err), st)
             return
-        C.call("adrt_rows_operator", self.code, self.plan.n, B, C.ptr(T), C.ptr(Y), R * N, C.ptr(self._half), st)
+        C.call("adrt_rows_operator", self.code, self.plan.n, B, code, C.ptr(T), C.ptr(Y), R * N, C.ptr(self._roots8), st)
 
     def main_level_rows(self, ops):
         """Level-rows processed by the polynomial-row launch of one op list (the dense rows excluded)."""
@@ -284,17 +289,18 @@ class RowTables:
         the level-1 butterflies of the hybrid around it) into one precomputed operator per row; with compensated
         high rows (plan.high_rows == "ff") they keep the polynomial filter in float-float arithmetic instead.
         skip_main: the polynomial rows (main_job) were run by the caller; only the rest is done here.
-        The plan's own G list runs as one real operator per frequency, dense rows included, where row_ops is set."""
+        The plan's own packed passes run as one real operator pair per frequency, dense rows included, where row_ops is
+        set."""
         ops = fuse_ops(ops)
         B = Y.shape[0]
         if not ops:
             return
-        if not skip_main and self.row_ops and ops == self._g_ops:
-            T = self.op_table(self.uses_mma(B))
-            if T is not None:
-                self._timed(ops, lambda: self.run_operators(Y, T))
-                self.count += B * self.plan.level_rows(ops_unfused(ops))
-                return
+        kind = None if skip_main else self.operator_kind(ops)
+        T = None if kind is None else self.op_table(kind, self.uses_mma(B))
+        if T is not None:
+            self._timed(ops, lambda: self.run_operators(Y, kind, T))
+            self.count += B * self.plan.level_rows(ops_unfused(ops))
+            return
         st = C.stream_handle()
         pidx = [i for i, o in enumerate(ops) if o[0] == "P"]
         if len(pidx) > 1:
@@ -365,7 +371,7 @@ def _rows_apply_f64(X, z_rows, ops, n, counter):
     C.call("adrt_rows_run", ctypes.byref(j), st)
 
 
-# sizes whose G pass runs as row operators: above, the operators outgrow what a lane should hold (17 GB at N = 2048);
+# sizes whose packed passes run as row operators: above, the operators outgrow what a lane should hold (17 GB at N = 2048);
 # below, the polynomial rows are a few microseconds of latency
 ROW_OPS_MIN, ROW_OPS_MAX = 6, 9
 # batch sizes from which the FP32 row operators run on the tensor cores, by n
@@ -373,17 +379,21 @@ ROW_OPS_MMA_BATCH = {8: 5, 9: 3}
 
 
 def row_operators_for(plan: Plan):
-    """Whether a pass G of this plan runs as one real operator per frequency: the operators of k and -k are conjugates
-    only if the bounds and degrees are symmetric, and plans that asked for no operator memory (compensated high rows)
-    keep the polynomial."""
+    """Whether the packed passes of this plan run as one real operator pair per frequency: the operators of k and -k are
+    conjugates only if the bounds and degrees are symmetric, and plans that asked for no operator memory (compensated
+    high rows) keep the polynomial."""
     idx = (-np.arange(plan.L)) % plan.L
     return (ROW_OPS_MIN <= plan.n <= ROW_OPS_MAX and getattr(plan, "high_rows", "dense") == "dense"
             and np.array_equal(plan.deg, plan.deg[idx]) and np.array_equal(plan.lam_max, plan.lam_max[idx]))
 
 
-def row_operator_bytes(plan: Plan, real):
-    """Device bytes of a plan's row operators and of their half-shift phases in one precision."""
-    return (plan.N + 1) * plan.N * plan.N // 2 * real.itemsize + 4 * plan.N * 2 * real.itemsize
+def row_operator_bytes(plan: Plan, real, batch):
+    """Device bytes of a plan's row operators (G and BP) and of their phases, for a pipeline of that batch and precision."""
+    N = plan.N
+    total = 2 * (N + 1) * N * N // 2 * real.itemsize + 8 * N * 2 * real.itemsize
+    if real == torch.float32 and batch >= ROW_OPS_MMA_BATCH.get(plan.n, batch + 1):
+        total += 2 * (N + 1) * 4  # the inverse scales of the split form (its tiles take the FP32 operators' bytes)
+    return total
 
 
 def _split_operators(n, T):
@@ -398,25 +408,29 @@ def _split_operators(n, T):
     return Ts
 
 
-def row_operator_table(tables, real):
-    """The operators of one pass G, (N + 1, 2, H, H) real, H = N/2, frequencies k = 0..N: with D = diag(z_k^(c/2)) the
-    operator T_k of an op list is D^* R_k D with R_k real and centro-symmetric (csrc/rows_op.cu), and the two blocks are
-    (P + Q)/2 and (P - Q)/2, P(c, j) = R_k(c, j), Q(c, j) = R_k(N-1-c, j), stored [j][c]. Evaluated in FP64: the columns
-    T_k e_j, j < H, by the FP64 row kernels on unit vectors (polynomial rows), or from the exact dense operators."""
-    plan, dev = tables.plan, tables.device
+def row_operator_table(tables, kind):
+    """The operators of a packed pass in the tables' precision, (N + 1, 2, H, H) real, H = N/2, frequencies k = 0..N, blocks
+    stored [j][c] (csrc/rows_op.cu): with D = diag(z_k^(c/2)), P(c, j) = R_k(c, j) and Q(c, j) = R_k(N-1-c, j), c, j < H,
+      G:  R_k = D T_k D^*, real and centro-symmetric, blocks (P + Q)/2 and (P - Q)/2
+      BP: R_k = D T_k diag(z_k^((2s-N+1)/4)), real part even and imaginary part odd in c, blocks (Re P + Re Q)/2 and
+          -(Im P - Im Q)/2.
+    Evaluated in FP64: the columns T_k e_j, j < H, by the FP64 row kernels on unit vectors (polynomial rows), or from the
+    exact dense operators."""
+    plan, dev, real = tables.plan, tables.device, tables.real
     n, N, L, H = plan.n, plan.N, plan.L, plan.N // 2
     out = torch.empty((N + 1, 2, H, H), dtype=real, device=dev)
-    half = torch.from_numpy(roots_of_unity(2 * L)).to(dev)
-
-    def phases(k):  # z_k^(c/2) for frequencies k (K,) and every c
-        return half[(k[:, None] * torch.arange(N, device=dev)[None, :]) % (2 * L)]
+    roots8 = torch.from_numpy(roots_of_unity(8 * N)).to(dev)
+    c = torch.arange(N, device=dev)[None, :]
 
     def store(k, j0, cols):  # cols (J, K, N): T_k e_j for j = j0.. and frequencies k
-        D = phases(k)
-        R = (cols * D[None] * D[:, j0:j0 + cols.shape[0]].T.conj()[:, :, None]).real
+        J = cols.shape[0]
+        D = roots8[2 * k[:, None] * c % (8 * N)]
+        right = D.conj() if kind == "G" else roots8[k[:, None] * (2 * c - N + 1) % (8 * N)]
+        R = cols * D[None] * right[:, j0:j0 + J].T[:, :, None]
         P, Q = R[..., :H], R[..., H:].flip(-1)
-        out[k, 0, j0:j0 + cols.shape[0]] = (0.5 * (P + Q)).transpose(0, 1).to(real)
-        out[k, 1, j0:j0 + cols.shape[0]] = (0.5 * (P - Q)).transpose(0, 1).to(real)
+        even, odd = (P + Q).real, (P - Q).real if kind == "G" else -(P - Q).imag
+        out[k, 0, j0:j0 + J] = (0.5 * even).transpose(0, 1).to(real)
+        out[k, 1, j0:j0 + J] = (0.5 * odd).transpose(0, 1).to(real)
 
     dense = plan.dense_freqs[plan.dense_freqs <= N]
     poly = np.setdiff1d(np.arange(N + 1), dense)
@@ -435,19 +449,20 @@ def row_operator_table(tables, real):
             J = min(step, H - j0)
             X = torch.zeros((J, len(poly), N), dtype=torch.complex128, device=dev)
             X[torch.arange(J, device=dev), :, torch.arange(j0, j0 + J, device=dev)] = 1
-            job = t64.job(X, tables._g_ops, rows)
+            job = t64.job(X, tables._op_lists[kind], rows)
             job.freq_mod, job.roots, job.twtab = len(poly), None, tab.data_ptr()
             job.deg, job.coef = deg.data_ptr(), coef.data_ptr()
             C.call("adrt_rows_run", ctypes.byref(job), C.stream_handle())
             store(kp, j0, X)
     if len(dense):
-        b1 = plan.method == "hybrid"
+        b1, bp = plan.method == "hybrid", kind == "BP"
+        folds = (bp, not bp, b1 and not bp, b1)
         sel = torch.from_numpy(np.nonzero(plan.dense_freqs <= N)[0]).to(dev)
         freqs = torch.from_numpy(plan.dense_freqs).to(dev)
         if n >= 9 and dev.type == "cuda":
-            chunks = dense_row_operator_device(plan, False, True, b1, b1, dev)
+            chunks = dense_row_operator_device(plan, *folds, dev)
         else:
-            chunks = [(0, torch.from_numpy(np.ascontiguousarray(plan.dense_row_operator(False, True, b1, b1))).to(dev))]
+            chunks = [(0, torch.from_numpy(np.ascontiguousarray(plan.dense_row_operator(*folds))).to(dev))]
         for c0, T in chunks:
             hit = sel[(sel >= c0) & (sel < c0 + T.shape[0])]
             if len(hit):
@@ -728,8 +743,8 @@ class Pipeline:
             bufs += [t.roots64, t.coef64]
         for T in t._op_dev.values():
             bufs += [T] if getattr(T, "_adrt_inv_scale", None) is None else [T, T._adrt_inv_scale]
-        if t._half is not None:
-            bufs.append(t._half)
+        if t._roots8 is not None:
+            bufs.append(t._roots8)
         if t._zd is not None:
             bufs.append(t._zd)
         for name in ("b_in", "b_in2"):
@@ -746,8 +761,8 @@ class Pipeline:
     @staticmethod
     def estimate_bytes(plan: Plan, batch, precision="fp32", stencil_precision=None, captured=True):
         """Device bytes a pipeline for (plan, batch, precision) holds once it has run apply (and capture, which adds
-        the two input buffers): the buffers of __init__, the row operators of G (or its folded dense-row table), the
-        back-projection's folded dense-row table and the dense-row staging, computed without allocating anything."""
+        the two input buffers): the buffers of __init__, the row operators of both passes or, without
+        them, the two folded dense-row tables and the dense-row staging, computed without allocating anything."""
         N, L, B = plan.N, plan.L, int(batch)
         rs = PRECISIONS[precision].itemsize
         ss = STENCIL_PRECISIONS[stencil_precision or precision].itemsize
@@ -760,14 +775,12 @@ class Pipeline:
         if ff:  # FP64 roots and coefficients of the compensated rows instead of dense operators
             total += L * 16 + plan.coef.size * 8
         else:
-            lists = 1 if row_operators_for(plan) else 2  # op lists with dense tables: G has its row operators instead
-            total += lists * nd * N * N * 2 * rs + nd * B * N * 2 * rs
-            if precision == "fp32" and B > 16 and 7 <= plan.n <= 10:  # their pre-split tensor-core form (in place)
-                total += lists * nd * N * N * 16 - nd * B * N * 2 * rs
-            if lists == 1:
-                total += row_operator_bytes(plan, PRECISIONS[precision])
-                if precision == "fp32" and B >= ROW_OPS_MMA_BATCH.get(plan.n, B + 1):
-                    total += (N + 1) * 4  # the inverse scales of the split form (its tiles take the FP32 operators' bytes)
+            if row_operators_for(plan):
+                total += row_operator_bytes(plan, PRECISIONS[precision], B)
+            else:
+                total += 2 * nd * N * N * 2 * rs + nd * B * N * 2 * rs
+                if precision == "fp32" and B > 16 and 7 <= plan.n <= 10:  # their pre-split tensor-core form (in place)
+                    total += 2 * nd * N * N * 16 - nd * B * N * 2 * rs
         total += L * 2 * rs + 3 * L * 4 + plan.coef.size * rs  # roots; deg and the row lists; coefficients
         if captured:  # the two input buffers of the captured graphs
             total += 2 * B * 4 * (2 * N - 1) * N * 8

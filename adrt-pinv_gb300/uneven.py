@@ -68,8 +68,8 @@ class UnevenBatch:
 
 
 class PersistentUnevenBatch:
-    """Uneven batch whose polynomial rows run in ONE persistent launch per outer step (the back-projection of every class,
-    and the G passes of the classes that do not run them as row operators).
+    """Uneven batch whose polynomial rows run in ONE persistent launch per outer step. (Classes whose passes run as row
+    operators have no polynomial rows: their operators run beside that launch, on the class's own stream.)
 
     All classes step through the outer iteration together (class c takes D_c steps; it drops out once they are
     done): at every step each class packs its images (or, at step 0, its sinograms) on its own stream, then one
@@ -124,10 +124,11 @@ class PersistentUnevenBatch:
             return (raw, torch.tensor(codes, dtype=torch.int32, device=self.device),
                     torch.tensor(starts, dtype=torch.int32, device=self.device), len(jobs))
 
-        # classes whose G pass runs as row operators launch it themselves; the others share the persistent launch
-        self.own_rows = [p.tables.runs_operators(p.ops["G"]) for p in self.pipes]
+        # classes whose packed passes run as row operators launch them themselves; the others share the persistent launch
+        self.own_rows = [p.tables.operator_kind(p.ops["G"]) is not None for p in self.pipes]
         self.counter = torch.zeros(4, dtype=torch.int32, device=self.device)
-        self.job_sets = {("BP", None): job_set("BP", self.order)}
+        shared = [i for i in self.order if not self.own_rows[i]]
+        self.job_sets = {("BP", None): job_set("BP", shared)} if shared else {}
         for s in range(1, max(self.D)):
             act = tuple(i for i in self.order if self.D[i] > s and not self.own_rows[i])
             if act and ("G", act) not in self.job_sets:
@@ -172,14 +173,15 @@ class PersistentUnevenBatch:
 
         def finish_bp(i):
             p = self.pipes[i]
-            p.finish_pass(p.ops["BP"])
+            p.finish_pass(p.ops["BP"], skip_main=not self.own_rows[i])
             p.sum_parts(p.y)
             a = self.coeffs[i][0]
             p.first_step(p.y, p.xs[0], a)
             state[i] = [p.xs[0], None, [p.xs[1], p.xs[2]]]
 
         self._fork(cap, allc, pack_bp)
-        self._rows(("BP", None), cap)
+        if ("BP", None) in self.job_sets:
+            self._rows(("BP", None), cap)
         self._fork(cap, allc, finish_bp)
         for s in range(1, max(self.D)):
             act = tuple(i for i in self.order if self.D[i] > s)

@@ -373,7 +373,7 @@ def run_ours(args):
     g_ms = [a.elapsed_time(b) for a, b, ops in timer if ops == fuse_ops(pipe.ops["G"])]
     rows_launch_ms = float(np.mean(g_ms)) if g_ms else None
     # row operators: N^2 real FMAs per packed row (two half-size real matrices on complex rows); polynomial rows: 8N per level-row
-    operators = pipe.tables.runs_operators(pipe.ops["G"])
+    operators = pipe.tables.operator_kind(pipe.ops["G"]) is not None
     flops_per_launch = B * 4 * N * 2 * N * N if operators else pipe.tables.main_level_rows(pipe.ops["G"]) * B * 8 * N
 
     # ---- end to end through the public API with pinned host buffers

@@ -124,21 +124,22 @@ int adrt_rows_lanes_per_row(int n);
 int adrt_rows_run_multi(const adrt_row_job* jobs, const int32_t* code, const int32_t* wstart, int njobs,
                         int32_t* counter, int grid, void* stream);
 
-/* One pass G on every packed row (2L rows per image, copies of the L frequencies stacked) as one real operator per
- * frequency: T (N+1 x 2 x N/2 x N/2, dtype) holds for k = 0..N the blocks (P + Q)/2 and (P - Q)/2, [j][c], of the
- * centro-symmetric R_k = D T_k D^*, D = diag(z_k^(c/2)), P(c,j) = R_k(c,j), Q(c,j) = R_k(N-1-c,j), c, j < N/2;
- * half_roots: 4N roots exp(2 pi i j / 4N) (dtype). Rows k and L-k share T_k. In place on Y (16-byte aligned, img_stride
- * even, complex elements). 6 <= n <= 9. */
-int adrt_rows_operator(int dtype, int n, int nimg, const void* T, void* Y, long long img_stride,
-                       const void* half_roots, void* stream);
-
+/* One packed pass on every packed row (2L rows per image, copies of the L frequencies stacked) as one real operator
+ * pair per frequency. kind 0, G: rows in natural order in and out; T (N+1 x 2 x N/2 x N/2, dtype) holds for k = 0..N the
+ * blocks (P + Q)/2 and (P - Q)/2, [j][c], of the centro-symmetric R_k = D T_k D^*, D = diag(z_k^(c/2)), P(c,j) = R_k(c,j),
+ * Q(c,j) = R_k(N-1-c,j), c, j < N/2. kind 1, BP: rows in slope order in; the blocks are (Re P + Re Q)/2 and
+ * -(Im P - Im Q)/2 of R_k = D T_k diag(z_k^((2s-N+1)/4)), columns s < N/2. Rows k and L-k share T_k (conjugated).
+ * roots8: the 8N roots exp(2 pi i j / 8N) (dtype). In place on Y (16-byte aligned, img_stride even, complex elements).
+ * 6 <= n <= 9. */
+int adrt_rows_operator(int dtype, int n, int nimg, int kind, const void* T, void* Y, long long img_stride,
+                       const void* roots8, void* stream);
 /* The same pass for FP32 rows on the tensor cores (n = 8, 9), the operators split once into FP16 pairs:
  * adrt_rows_operator_split turns the FP32 T above, frequency k scaled by scale[k] (a power of two; largest entry below
  * 2^14 after scaling), into Ts ((N+1) N^2 FP16 values, hi and lo tiles in the kernel's order); inv_scale[k] = 1/scale[k].
  * err: device int, set to a positive code if a bounded wait ran out (the rows are then not all written). */
 int adrt_rows_operator_split(int n, const void* T, const float* scale, void* Ts, void* stream);
-int adrt_rows_operator_mma(int n, int nimg, const void* Ts, const float* inv_scale, void* Y, long long img_stride,
-                           const void* half_roots, int32_t* err, void* stream);
+int adrt_rows_operator_mma(int n, int nimg, int kind, const void* Ts, const float* inv_scale, void* Y,
+                           long long img_stride, const void* roots8, int32_t* err, void* stream);
 
 /* Per-row twiddle table tab[k*(N/2+1) + t] = z_k^t (t = 0..N/2) from K complex z (FP64 in, dtype out),
  * by binary powering in FP64. */

@@ -1,5 +1,5 @@
-"""Row operators (adrt_rows_operator: a pass G as one real centro-symmetric matrix per frequency) against the FP64
-polynomial and dense rows of the row engine on random packed rows.
+"""Row operators (adrt_rows_operator: a packed pass as one real matrix pair per frequency) against the FP64 polynomial and
+dense rows of the row engine on random packed rows.
 
 Tolerances, norm-wise over all rows: FP64 1e-12, as the row kernels are held to; FP32 1e-6: two half-shift phases, the
 sums over N/2 <= 256 terms of rounded products (about sqrt(256) eps = 1e-6 at worst, norm-wise less) and FP32 matrices."""
@@ -37,12 +37,13 @@ def _tables(plan, real, ops):
 # batches around the kernels' tiles: one image, the few-vector kernel, its limit (2 VT / 4 vectors), ragged tiles
 @pytest.mark.parametrize("n,batches", [(6, (1, 3, 16, 17, 37)), (7, (1, 8, 9, 33)), (8, (1, 2, 4, 5, 13)), (9, (1, 2, 3, 7))])
 @pytest.mark.parametrize("method,p,cap", [("lp", 16, 12), ("hybrid", 32, 16), ("hybrid", 8, None)])
-def test_row_operators_match_rows(pkg, plans, method, p, cap, n, batches):
+@pytest.mark.parametrize("kind", ["G", "BP"])
+def test_row_operators_match_rows(pkg, plans, kind, method, p, cap, n, batches):
     import torch
     from adrt_pinv_gb300.device import _op_lists
 
     plan = plans(method, n, p, cap)
-    ops = _op_lists(plan)["G"]
+    ops = _op_lists(plan)[kind]
     N = 1 << n
     g = torch.Generator(device="cuda").manual_seed(n)
     ref_t, op64, op32 = (_tables(plan, torch.float64, False), _tables(plan, torch.float64, True),
@@ -133,15 +134,15 @@ def test_row_operators_row_stride_and_errors(pkg, plans):
     plan = plans("lp", 6, 16, 12)
     C = pkg._lib
     t = _tables(plan, torch.float32, True)
-    T, N = t.op_table(), 64
+    T, N = t.op_table("G"), 64
     Y = torch.randn((3, 4 * N + 2, N), dtype=torch.complex64, device="cuda")
     want = Y[:, :4 * N].clone()
-    t.run_operators(want, T)
+    t.run_operators(want, "G", T)
     got = Y.clone()
     st = C.stream_handle()
-    C.call("adrt_rows_operator", C.F32, 6, 3, C.ptr(T), C.ptr(got), (4 * N + 2) * N, C.ptr(t._half), st)
+    C.call("adrt_rows_operator", C.F32, 6, 3, 0, C.ptr(T), C.ptr(got), (4 * N + 2) * N, C.ptr(t._roots8), st)
     assert torch.equal(got[:, :4 * N], want) and torch.equal(got[:, 4 * N:], Y[:, 4 * N:])
-    for args in ((C.I32, 6, 3, C.ptr(T)), (C.F32, 5, 3, C.ptr(T)), (C.F32, 10, 3, C.ptr(T)), (C.F32, 6, -1, C.ptr(T)),
-                 (C.F32, 6, 3, None)):
+    for args in ((C.I32, 6, 3, 0, C.ptr(T)), (C.F32, 5, 3, 0, C.ptr(T)), (C.F32, 10, 3, 0, C.ptr(T)),
+                 (C.F32, 6, -1, 0, C.ptr(T)), (C.F32, 6, 3, 2, C.ptr(T)), (C.F32, 6, 3, 0, None)):
         with pytest.raises(RuntimeError):
-            C.call("adrt_rows_operator", *args, C.ptr(got), 4 * N * N, C.ptr(t._half), st)
+            C.call("adrt_rows_operator", *args, C.ptr(got), 4 * N * N, C.ptr(t._roots8), st)
