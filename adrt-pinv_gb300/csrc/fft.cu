@@ -24,10 +24,11 @@
 
 namespace adrt {
 
-template <int l> struct FftCfg {
+template <typename real, int l> struct FftCfg {
     static constexpr int L = 1 << l;
-    // log2 of points per thread: 4 where that takes a pass (an exchange) less than 3
-    static constexpr int e = l < 3 ? l : ((l + 3) / 4 < (l + 2) / 3 ? 4 : 3);
+    // log2 of points per thread: in FP32 4 where that takes a pass (an exchange) less than 3; FP64 is bound by its pipe
+    // (a warp's instruction takes 16 cycles), so there more threads with fewer points each
+    static constexpr int e = l < 3 ? l : (sizeof(real) == 4 && (l + 3) / 4 < (l + 2) / 3 ? 4 : 3);
     static constexpr int E = 1 << e;
     static constexpr int TPC = L / E;           // threads per column
     static constexpr int NPASS = (l + e - 1) / e;
@@ -58,8 +59,8 @@ template <int l> __host__ __device__ constexpr int fft_fit(int c, int elem_bytes
 template <int l> __host__ __device__ constexpr int fft_cols(int Cmax, int elem_bytes) {
     return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / imax(1, (1 << l) / 8)), (1 << l) / 2)), elem_bytes);
 }
-template <int l> __host__ __device__ constexpr int fft_cols_auto(int Cmax, int elem_bytes) {
-    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / FftCfg<l>::TPC), (1 << l) / 2)), elem_bytes);
+template <typename real, int l> __host__ __device__ constexpr int fft_cols_auto(int Cmax, int elem_bytes) {
+    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / FftCfg<real, l>::TPC), (1 << l) / 2)), elem_bytes);
 }
 
 // cos and sin of 2 pi k / 16, k < 8
@@ -87,9 +88,9 @@ template <typename real, bool INV> __device__ __forceinline__ cplx<real> rotate(
 // all passes of the in-place DIT transform on the registers x[] of (column c, column-thread t); the caller loads x[j]
 // with input brev(pos(0, t, j)) and finds output pos(NPASS - 1, t, j) in x[j]
 template <typename real, int l, bool INV>
-__device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const cplx<real>* __restrict__ roots,
+__device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<real, l>::E], const cplx<real>* __restrict__ roots,
                                            cplx<real>* tile, int CP, int c, int t) {
-    using F = FftCfg<l>;
+    using F = FftCfg<real, l>;
     using C = cplx<real>;
 #pragma unroll
     for (int q = 0; q < F::NPASS; ++q) {
@@ -128,18 +129,18 @@ __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<l>::E], const 
 
 // threads of a CTA and the CTAs per SM the register budget is sized for
 template <typename real, int l, int CB> struct FftLaunch {
-    static constexpr int threads = CB * FftCfg<l>::TPC;
+    static constexpr int threads = CB * FftCfg<real, l>::TPC;
     // threads per SM: 64 registers each for 8 points in FP32, twice that for 16 points or FP64
-    static constexpr int resident = sizeof(real) == 4 && FftCfg<l>::e < 4 ? 1024 : 512;
-    static constexpr int pack_min = imax(1, (FftCfg<l>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads);
-    static constexpr int unpack_min = imax(1, resident / threads);
+    static constexpr int resident = sizeof(real) == 4 && FftCfg<real, l>::e < 4 ? 1024 : 512;
+    static constexpr int pack_min = imin(16, imax(1, (FftCfg<real, l>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads));
+    static constexpr int unpack_min = imin(16, imax(1, resident / threads));
 };
 
 template <typename real, int l, int CB, typename SRC>
 __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<real, l, CB>::pack_min)
     pack_fft_kernel(int nimg, int src_kind, const SRC* __restrict__ src, long long src_stride, cplx<real>* __restrict__ Y,
                     const cplx<real>* __restrict__ roots_g) {
-    using F = FftCfg<l>;
+    using F = FftCfg<real, l>;
     using C = cplx<real>;
     constexpr int L = F::L, N = L / 2;
     constexpr int CP = fft_pad(CB);
@@ -229,7 +230,7 @@ template <typename real, int l, int CB>
 __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<real, l, CB>::unpack_min)
     ifft_unpack_kernel(int nimg, const cplx<real>* __restrict__ Z, real* __restrict__ colpart, real* __restrict__ row0,
                        real* __restrict__ row3, const cplx<real>* __restrict__ roots_g) {
-    using F = FftCfg<l>;
+    using F = FftCfg<real, l>;
     using C = cplx<real>;
     constexpr int L = F::L, N = L / 2, E = F::E;
     constexpr int CP = fft_pad(CB), RP = N + 1;  // row pitch of the transposed strips
@@ -297,7 +298,11 @@ template <typename real, int l, int CB> static size_t unpack_smem() {
 
 // columns per CTA: cols = 0 picks as many as fit, up to 16 FP32 / 8 FP64; the autotuner's choices are the widths of 8
 // points per thread and a quarter of them (narrower CTAs, more of them per SM)
-template <typename real, int l> constexpr int cols_auto() { return fft_cols_auto<l>(FftMax<real>::C, sizeof(cplx<real>)); }
+template <typename real, int l> constexpr int cols_auto() { return fft_cols_auto<real, l>(FftMax<real>::C, sizeof(cplx<real>)); }
+// the width of launches that would leave SMs idle at the others (small batches): an eighth of the widest, whole warps
+template <typename real, int l> constexpr int cols_small() {
+    return imin(cols_auto<real, l>(), imax(imax(1, cols_auto<real, l>() / 8), 32 / FftCfg<real, l>::TPC));
+}
 template <typename real, int l> constexpr int cols_wide() { return fft_cols<l>(FftMax<real>::C, sizeof(cplx<real>)); }
 template <typename real, int l> constexpr int cols_narrow() { return imax(1, cols_wide<real, l>() / 4); }
 
@@ -309,7 +314,7 @@ static int launch_pack_cb(int nimg, int src_kind, const void* src, long long src
     auto kern = pack_fft_kernel<real, l, CB, SRC>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, 2, nimg);
-    kern<<<grid, CB * FftCfg<l>::TPC, smem, st>>>(nimg, src_kind, reinterpret_cast<const SRC*>(src),
+    kern<<<grid, CB * FftCfg<real, l>::TPC, smem, st>>>(nimg, src_kind, reinterpret_cast<const SRC*>(src),
                                                    src_stride ? src_stride : (long long)N * N,
                                                    reinterpret_cast<cplx<real>*>(Y),
                                                    reinterpret_cast<const cplx<real>*>(roots));
@@ -319,8 +324,16 @@ static int launch_pack_cb(int nimg, int src_kind, const void* src, long long src
 template <typename real, int l, typename SRC>
 static int launch_pack_src(int nimg, int src_kind, const void* src, long long src_stride, void* Y, const void* roots,
                            int cols, cudaStream_t st) {
-    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
-    if (cols == 0 || cols == A) return launch_pack_cb<real, l, A, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>(), SW = cols_small<real, l>();
+    constexpr int N = 1 << (l - 1);
+    if (cols == 0) {  // the widest that still gives every SM a CTA
+        const long long cta1 = 2ll * nimg * N;  // CTAs at one column each
+        const int sms = device_sm_count();
+        cols = cta1 / A >= sms ? A : (cta1 / NW >= sms ? NW : SW);
+        if (SW != A && SW != NW && cols == SW)
+            return launch_pack_cb<real, l, SW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    }
+    if (cols == A) return launch_pack_cb<real, l, A, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
     if (W != A && cols == W) return launch_pack_cb<real, l, W, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
     if (NW != W && NW != A && cols == NW) return launch_pack_cb<real, l, NW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
     set_error("pack_fft: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
@@ -343,7 +356,7 @@ static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, 
     auto kern = ifft_unpack_kernel<real, l, CB>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, nimg);
-    kern<<<grid, CB * FftCfg<l>::TPC, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z), reinterpret_cast<real*>(colpart),
+    kern<<<grid, CB * FftCfg<real, l>::TPC, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z), reinterpret_cast<real*>(colpart),
                                                    reinterpret_cast<real*>(row0), reinterpret_cast<real*>(row3),
                                                    reinterpret_cast<const cplx<real>*>(roots));
     return launch_status("ifft_unpack_kernel");
@@ -352,8 +365,15 @@ static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, 
 template <typename real, int l>
 static int launch_unpack(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots, int cols,
                          cudaStream_t st) {
-    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
-    if (cols == 0 || cols == A) return launch_unpack_cb<real, l, A>(nimg, Z, colpart, row0, row3, roots, st);
+    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>(), SW = cols_small<real, l>();
+    constexpr int N = 1 << (l - 1);
+    if (cols == 0) {
+        const long long cta1 = (long long)nimg * N;
+        const int sms = device_sm_count();
+        cols = cta1 / A >= sms ? A : (cta1 / NW >= sms ? NW : SW);
+        if (SW != A && SW != NW && cols == SW) return launch_unpack_cb<real, l, SW>(nimg, Z, colpart, row0, row3, roots, st);
+    }
+    if (cols == A) return launch_unpack_cb<real, l, A>(nimg, Z, colpart, row0, row3, roots, st);
     if (W != A && cols == W) return launch_unpack_cb<real, l, W>(nimg, Z, colpart, row0, row3, roots, st);
     if (NW != W && NW != A && cols == NW) return launch_unpack_cb<real, l, NW>(nimg, Z, colpart, row0, row3, roots, st);
     set_error("ifft_unpack: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
