@@ -201,6 +201,66 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 }
 
+// One Gram M = B^* B over levels 1..n (the normal operator's rows): compile-time levels, register-resident rows as in the
+// row programs. Bounded by memory and by the twiddles (about as many loads and registers as a row itself), so a group
+// keeps them for up to `per` consecutive images of its row, and two CTAs share an SM.
+template <typename real, int n>
+__global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
+    rows_gram_kernel(const adrt_row_job J, const TwSrc<real> tw, const int per, const int total) {
+    using C = cplx<real>;
+    using F = FastCfg<n>;
+    using Ln = Lanes<C, n>;
+    using Ct = CtLanes<C, n>;
+    constexpr int N = F::N, R = F::R, T = F::T, tb = F::tb, NB = F::NB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    const int giw = T >= 32 ? 0 : lane / T;
+    const int u = threadIdx.x & (T - 1);
+    C* buf = reinterpret_cast<C*>(smem_raw) + (threadIdx.x / T) * F::GS;
+    C* zt = buf + F::BUF + F::N;
+    const unsigned gm = (T >= 32) ? 0xffffffffu : (((1u << T) - 1u) << (giw * T));
+    constexpr int GROUPS = FAST_THREADS / T;
+    const int chunks = (J.nimg + per - 1) / per;
+    for (int item = blockIdx.x * GROUPS + threadIdx.x / T; item < total; item += gridDim.x * GROUPS) {
+        const int sel = item / chunks, img0 = (item - sel * chunks) * per;
+        const int row = J.rows ? J.rows[sel] : sel;
+        const int key = tw.roots ? row % J.freq_mod : row;
+        C tA[R / 2 + 1];
+#pragma unroll
+        for (int t = 0; t <= R / 2; ++t) tA[t] = tw.get(key, t);
+        C t0[NB ? NB : 1], t1[NB ? NB : 1];
+        if (NB) {
+            const int U = tb ? (int)(__brev((unsigned)u) >> (32 - tb)) : 0;
+#pragma unroll
+            for (int b = F::BLO; b < n; ++b) {
+                const int jb = b - tb;
+#pragma unroll
+                for (int vv = 0; vv < (1 << jb); ++vv) {
+                    const int t = (U << jb) + brev(vv, jb);
+                    t0[F::offB(b) + vv] = tw.get(key, t);
+                    t1[F::offB(b) + vv] = tw.get(key, t + 1);
+                }
+            }
+        }
+        if (F::ZT) {
+            Ln::gsync(gm);  // the previous item's table is no longer read
+#pragma unroll 1
+            for (int t = u; t < F::ZT; t += T) zt[t] = tw.get(key, t);
+            Ln::gsync(gm);
+        }
+        const int img1 = img0 + per < J.nimg ? img0 + per : J.nimg;
+        for (int img = img0; img < img1; ++img) {
+            C* ptr = reinterpret_cast<C*>(J.X) + (size_t)img * J.img_stride + (size_t)row * N;
+            C v[R], w[R];
+#pragma unroll
+            for (int j = 0; j < R; j += 2) ld2(ptr + j + R * u, v[j], v[j + 1]);
+            Ct::template gram_oop<1, n>(v, w, tA, t0, t1, buf, u, gm, zt);
+#pragma unroll
+            for (int j = 0; j < R; j += 2) st2(ptr + j + R * u, w[j], w[j + 1]);
+        }
+    }
+}
+
 // ------------------------------------------------------------------ simple kernel (natural order, shared memory)
 template <typename real>
 __device__ void simple_fwd(cplx<real>*& a, cplx<real>*& b, int N, int lo, int hi, const TwSrc<real>& tw, int key) {
@@ -440,6 +500,22 @@ static int launch_prog(const adrt_row_job& J, const TwSrc<real>& tw, int total, 
 }
 
 
+template <typename real, int n>
+static int launch_gram(const adrt_row_job& J, const TwSrc<real>& tw, cudaStream_t st) {
+    using F = FastCfg<n>;
+    const size_t smem = (size_t)(FAST_THREADS / F::T) * F::GS * sizeof(cplx<real>);
+    auto kern = rows_gram_kernel<real, n>;
+    if (int rc = ensure_smem((const void*)kern, smem)) return rc;
+    const int groups = FAST_THREADS / F::T, slots = (J.grid > 0 ? J.grid : num_sms()) * (sizeof(real) == 4 ? 2 : 1);
+    // images per item: as many as keep two items per resident group, up to 4
+    int per = 1;
+    while (per < 4 && (long long)J.nsel * ((J.nimg + 2 * per - 1) / (2 * per)) >= 2ll * slots * groups) per *= 2;
+    const long long total = (long long)J.nsel * ((J.nimg + per - 1) / per);
+    const long long ctas = (total + groups - 1) / groups;
+    kern<<<(unsigned)(ctas < slots ? ctas : slots), FAST_THREADS, smem, st>>>(J, tw, per, (int)total);
+    return launch_status("rows_gram_kernel");
+}
+
 template <typename real>
 static int rows_dispatch(const adrt_row_job& J, int iters, double safety, double* pout, cudaStream_t st) {
     TwSrc<real> tw;
@@ -475,6 +551,27 @@ static int rows_dispatch(const adrt_row_job& J, int iters, double safety, double
                 break;
             case 11:
                 if constexpr (std::is_same<real, float>::value) return launch_prog<real, 11>(J, tw, total, prog, st);
+                break;
+        }
+    }
+    if (!pout && prog_n && J.nops == 1 && J.op[0] == ADRT_OP_M && J.lo[0] == 1 && J.hi[0] == J.n) {
+        switch (J.n) {
+            case 1: return launch_gram<real, 1>(J, tw, st);
+            case 2: return launch_gram<real, 2>(J, tw, st);
+            case 3: return launch_gram<real, 3>(J, tw, st);
+            case 4: return launch_gram<real, 4>(J, tw, st);
+            case 5: return launch_gram<real, 5>(J, tw, st);
+            case 6: return launch_gram<real, 6>(J, tw, st);
+            case 7: return launch_gram<real, 7>(J, tw, st);
+            case 8: return launch_gram<real, 8>(J, tw, st);
+            case 9:
+                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 9>(J, tw, st);
+                break;
+            case 10:
+                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 10>(J, tw, st);
+                break;
+            case 11:
+                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 11>(J, tw, st);
                 break;
         }
     }
