@@ -12,7 +12,7 @@ or torch; a batch is solved at once, each sinogram with its own scalars and its 
 with the iterate the reference's loop would return for it alone. NumPy in -> NumPy out; torch in -> torch (CUDA)
 out. Histories: one array per sinogram (the reference's `hist`), a list of them for a batch.
 
-Without a callback the iterations run in blocks recorded once as a CUDA graph and replayed; the host reads the
+Without a callback the iterations run in blocks (long runs replay a block recorded as a CUDA graph); the host reads the
 per-image active flags between blocks only. With a callback (single sinogram only, as in the reference) each
 iteration is followed by callback(it, x, norm) with x on the host.
 
@@ -41,6 +41,11 @@ def _as_batch(b, N, what):
     shape = (4, 2 * N - 1, N) if what == "sino" else (N, N)
     bt = bt.reshape((-1,) + shape)
     return is_torch, single, bt
+
+
+# blocks of iterations launched directly before one is recorded as a CUDA graph: recording costs about 20 ms (torch
+# collects garbage and empties its allocator cache), a replayed block of 16 iterations saves at most about 0.2 ms of launches
+GRAPH_AFTER = 64
 
 
 class _Solver:
@@ -78,15 +83,22 @@ class _Solver:
         return [hist[i, : its[i] + 1].copy() for i in range(self.nimg)]
 
     def _run_blocks(self, step_block):
-        """Replay blocks of iterations until no image is active (graph recorded on the first block)."""
+        """Blocks of iterations until no image is active, launched directly; a run longer than GRAPH_AFTER blocks (small
+        images, many iterations: bound by launches) continues as replays of a recorded block."""
+        done = 0
         while bool(self.active.any()):
+            if done < GRAPH_AFTER * self.block:
+                k = min(self.block, max(1, self.maxit - done))
+                step_block(k)
+                done += k
+                continue
             if self.graph is None:
                 side = torch.cuda.Stream(device=self.device)
                 side.wait_stream(torch.cuda.current_stream(self.device))
                 with torch.cuda.stream(side):
                     g = torch.cuda.CUDAGraph()
                     with graph_capture(g, side):
-                        step_block()
+                        step_block(self.block)
                 torch.cuda.current_stream(self.device).wait_stream(side)
                 self.graph = g
             self.graph.replay()
@@ -117,7 +129,7 @@ class CglsSolver(_Solver):
         """Run to convergence (or maxit) for every sinogram; returns (x (nimg, N, N) device tensor, histories)."""
         self.start(b, x0)
         if callback is None:
-            self._run_blocks(lambda: self.iterate(self.block))
+            self._run_blocks(self.iterate)
         else:
             while bool(self.active.any()):
                 self.iterate(1)
@@ -128,7 +140,7 @@ class CglsSolver(_Solver):
 
 class PcgSolver(_Solver):
     """Device state of PCG on R^T R x = R^T b for `nimg` images (pinv.py:51-82). M: None (identity, the whole
-    iteration on the device, replayed from a CUDA graph) or a callable taking the residuals as a device tensor
+    iteration on the device) or a callable taking the residuals as a device tensor
     (nimg, N, N) FP64 and returning M r of the same shape (called once per iteration, for all images)."""
 
     def __init__(self, n, nimg=1, M=None, maxit=10000, tol=1e-12, device="cuda", block=16):
@@ -161,7 +173,7 @@ class PcgSolver(_Solver):
         self._precondition()
         C.call("adrt_pcg_rho", ctypes.byref(self.state), st)
         if callback is None and self.M is None:
-            self._run_blocks(lambda: [self._one() for _ in range(self.block)])
+            self._run_blocks(lambda k: [self._one() for _ in range(k)])
         else:
             while bool(self.active.any()):
                 self._one()
