@@ -33,14 +33,15 @@ constexpr int AW_PAD = 17;       // rows past the band that a step may touch (at
 __host__ __device__ constexpr int aw_pitch(int R) { return 32 * R + AW_PAD; }
 template <int G> __host__ __device__ constexpr int aw_rows(int R) { return 32 * R - ((1 << G) - 1); }  // rows kept
 
-// (T_q x)(i, j) (adrtcore.py:29-39)
-template <typename T> __device__ __forceinline__ T tq_read(const T* x, int N, int q, int i, int j) {
-    switch (q) {
-        case 0: return x[(size_t)j * N + (N - 1 - i)];
-        case 1: return x[(size_t)(N - 1 - i) * N + j];
-        case 2: return x[(size_t)i * N + j];
-        default: return x[(size_t)(N - 1 - j) * N + (N - 1 - i)];
-    }
+// one element to shared memory, asynchronously (all of a tile's loads in flight at once); zero where !ok
+template <typename T> __device__ __forceinline__ void aw_copy(T* dst, const T* src, const T* valid, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(ok ? src : valid), "n"((int)sizeof(T)), "r"(ok ? (int)sizeof(T) : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void aw_copy_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
 }
 
 // what one CTA of a pass works on: levels m0+1..m0+G of image quadrant `slot`, groups slice0..slice0+nt-1 (group =
@@ -208,21 +209,25 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_fwd_pass(const AwPass A, cons
     if (zero && !last) return;
     if (!zero) {
         if (A.m0 == 0) {
+            // (T_q x)(h, c) (adrtcore.py:29-39): quadrants 1 and 2 lie along the image's columns, 0 and 3 along its rows
             const T* x = src + (slot >> 2) * (size_t)N * N;
             const int q = (int)(slot & 3), c0 = slice0 * C;
-            if (q == 1 || q == 2) {  // image rows along the columns
+            if (q == 1 || q == 2) {
+                const T* xc = x + c0 + lane;
 #pragma unroll 4
-                for (int e = threadIdx.x; e < RT * AW_COLS; e += AW_THREADS) {
-                    const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + r;
-                    if (c < ncols) tile[c * P + r] = (h >= 0 && h < N) ? tq_read(x, N, q, h, c0 + c) : (T)0;
+                for (int r = warp; r < RT; r += AW_THREADS / 32) {
+                    const int h = h0 + r;
+                    if (lane < ncols) aw_copy(tile + lane * P + r, xc + (ptrdiff_t)(q == 1 ? N - 1 - h : h) * N, x, h >= 0 && h < N);
                 }
             } else {
-                for (int c = warp; c < ncols; c += AW_THREADS / 32)
+                for (int c = warp; c < ncols; c += AW_THREADS / 32) {
+                    const T* xr = x + (size_t)(q == 0 ? c0 + c : N - 1 - c0 - c) * N + (N - 1);
 #pragma unroll
                     for (int i = 0; i < R; ++i) {
                         const int r = i * 32 + lane, h = h0 + r;
-                        tile[c * P + r] = (h >= 0 && h < N) ? tq_read(x, N, q, h, c0 + c) : (T)0;
+                        aw_copy(tile + c * P + r, xr - h, x, h >= 0 && h < N);
                     }
+                }
             }
         } else {
             const int P0 = N + M0 - 1;
@@ -233,11 +238,11 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_fwd_pass(const AwPass A, cons
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
                     const int r = i * 32 + lane, h = h0 + r + b * t;
-                    tile[c * P + r] = (h >= -t && h < N) ? col[h] : (T)0;
+                    aw_copy(tile + c * P + r, col + h, f, h >= -t && h < N);
                 }
             }
         }
-        __syncthreads();
+        aw_copy_wait();
         if constexpr (G >= 2) aw_step4<T, G, R, 0, true>(tile, ncols, warp, lane);
         else aw_step2<T, G, R, 0, true>(tile, ncols, warp, lane);
         __syncthreads();
@@ -250,12 +255,12 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_fwd_pass(const AwPass A, cons
         }
     }
     if (last) {
-        T* g = dst + slot * A.S + slice0 * C;
+        if (lane < ncols) {
+            T* g = dst + slot * A.S + slice0 * C + lane + (size_t)r0 * N;
+            const T* col = tile + ((lane & ~(C - 1)) | aw_rev<G>(lane & (C - 1))) * P;
+            const int rend = min(TR, HO - r0);
 #pragma unroll 4
-        for (int e = threadIdx.x; e < TR * AW_COLS; e += AW_THREADS) {
-            const int r = e / AW_COLS, c = e % AW_COLS;
-            if (c < ncols && r0 + r < HO)
-                g[(size_t)(r0 + r) * N + c] = zero ? (T)0 : tile[((c & ~(C - 1)) | aw_rev<G>(c & (C - 1))) * P + r];
+            for (int r = warp; r < rend; r += AW_THREADS / 32) g[(size_t)r * N] = zero ? (T)0 : col[r];
         }
     } else {
         const int P1 = N + M1 - 1;
@@ -293,13 +298,14 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_adj_pass(const AwPass A, cons
     for (int i = 0; i < A.nt; ++i) tmax = max(tmax, (slice0 + i) & (M0 - 1));
     if (h0 + RT - 1 < -C * tmax) return;  // no block has a row of its domain here
     if (A.m0 + G == A.n) {
-        const T* g = src + slot * A.S + slice0 * C;
+        if (lane < ncols) {
+            const T* g = src + slot * A.S + slice0 * C + lane + (size_t)(N - 1) * N;
+            T* col = tile + ((lane & ~(C - 1)) | aw_rev<G>(lane & (C - 1))) * P;
 #pragma unroll 4
-        for (int e = threadIdx.x; e < RT * AW_COLS; e += AW_THREADS) {
-            const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + r;
-            if (c < ncols)
-                tile[((c & ~(C - 1)) | aw_rev<G>(c & (C - 1))) * P + r] =
-                    (h > -N && h < N) ? g[(size_t)(h + N - 1) * N + c] : (T)0;
+            for (int r = warp; r < RT; r += AW_THREADS / 32) {
+                const int h = h0 + r;
+                aw_copy(col + r, g + (ptrdiff_t)h * N, g, h > -N && h < N);
+            }
         }
     } else {
         const int P1 = N + M1 - 1;
@@ -310,11 +316,11 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_adj_pass(const AwPass A, cons
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const int r = i * 32 + lane, h = h0 + r;
-                tile[c * P + r] = (h >= -t && h < N) ? col[h] : (T)0;
+                aw_copy(tile + c * P + r, col + h, g, h >= -t && h < N);
             }
         }
     }
-    __syncthreads();
+    aw_copy_wait();
     if constexpr (G == 4) {
         aw_step4<T, G, R, 2, false>(tile, ncols, warp, lane);
         __syncthreads();
@@ -329,10 +335,12 @@ __global__ void __launch_bounds__(AW_THREADS) adrt_adj_pass(const AwPass A, cons
     if (A.m0 == 0) {
         const int q = (int)(slot & 3), c0 = slice0 * C;
         if (q == 1 || q == 2) {
+            if (lane < ncols) {
+                const int rend = min(TR, N - h0 - HALO);
+                T* oc = o + (size_t)(h0 + HALO) * N + c0 + lane;
+                const T* col = tile + lane * P + HALO;
 #pragma unroll 4
-            for (int e = threadIdx.x; e < TR * AW_COLS; e += AW_THREADS) {
-                const int r = e / AW_COLS, c = e % AW_COLS, h = h0 + HALO + r;
-                if (c < ncols && h < N) o[(size_t)h * N + c0 + c] = tile[c * P + HALO + r];
+                for (int r = warp; r < rend; r += AW_THREADS / 32) oc[(size_t)r * N] = col[r];
             }
         } else {
             for (int c = warp; c < ncols; c += AW_THREADS / 32)
