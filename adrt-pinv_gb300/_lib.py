@@ -81,9 +81,11 @@ PROTOTYPES = {
     "adrt_rows_lanes_per_row": [_I],
     "adrt_rows_run_multi": [_P, _P, _P, _I, _P, _I, _P],
     "adrt_rows_operator": [_I, _I, _I, _I, _P, _P, _L, _P, _P],
+    "adrt_rows_operator_split_size": [_I],
     "adrt_rows_operator_split": [_I, _P, _P, _P, _P],
     "adrt_rows_operator_mma": [_I, _I, _I, _P, _P, _P, _L, _P, _P, _P],
     "adrt_twiddle_table": [_I, _I, _I, _P, _P, _P],
+    "adrt_gram_freq": [_I, _I, _I, _I, _P, _P, _P, _P, _P, _P],
     "adrt_power_rows": [_I, _I, _I, _P, _P, _I, _I, _D, _P, _P, _P],
     "adrt_cert_rowsum_dev": [_I, _I, _P, _I, _P, _P],
     "adrt_pack_fft": [_I, _I, _I, _I, _I, _P, _L, _P, _P, _I, _P],
@@ -123,7 +125,8 @@ def load(path=LIB_PATH):
     for name, args in PROTOTYPES.items():
         fn = getattr(lib, name)
         fn.argtypes = args
-        fn.restype = {"adrt_last_error": ctypes.c_char_p, "adrt_launch_count": ctypes.c_longlong}.get(name, ctypes.c_int)
+        fn.restype = {"adrt_last_error": ctypes.c_char_p, "adrt_launch_count": ctypes.c_longlong,
+                      "adrt_rows_operator_split_size": ctypes.c_longlong}.get(name, ctypes.c_int)
     _lib = lib
     return lib
 

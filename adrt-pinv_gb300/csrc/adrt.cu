@@ -19,8 +19,9 @@
 //     bytes in 4-byte types, at a time).
 //   * The adjoint runs the same passes backwards; its last pass leaves the four quadrants' images, which
 //     adrt_quadrant_sum adds (T_q^T).
-// Bounded by HBM (each pass reads and writes its level's data once). 64 int32 images at N = 256: forward 129 us, adjoint
-// 199 us (one pass per level above the fourth: 359 and 527 us); 3 FP32 images at N = 1024, adjoint: 137 us (624 us).
+// Bounded by HBM and issue (each pass reads and writes its level's data once); FP64 by its pipe (2 additions per clock
+// and SM). 64 int32 images at N = 256: forward 84 us, adjoint 107 us (one pass per level above the fourth: 359 and 527
+// us); 3 FP32 images at N = 1024, adjoint: 121 us (624 us).
 #include "common.cuh"
 #include "launch.h"
 

@@ -202,15 +202,16 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 // One Gram M = B^* B over levels 1..n (the normal operator's rows): compile-time levels, register-resident rows as in the
-// row programs. Bounded by memory and by the twiddles (about as many loads and registers as a row itself), so a group
-// keeps them for up to `per` consecutive images of its row, and two CTAs share an SM.
+// row programs, out of place or in place. Bounded by memory and by the twiddles (about as many loads and registers as a
+// row itself), so a group keeps them for up to `per` consecutive images of its row, the B-layout levels hold z^t alone
+// (z^(t+1) f = z (z^t f) forward, z^t* (g0 + z* g1) adjoint: two operations more per pair, 30 registers less, no
+// spills), and two CTAs share an SM.
 template <typename real, int n>
 __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
-    rows_gram_kernel(const adrt_row_job J, const TwSrc<real> tw, const int per, const int total) {
+    rows_gram_kernel(const adrt_row_job J, const cplx<real>* in, const TwSrc<real> tw, const int per, const int total) {
     using C = cplx<real>;
     using F = FastCfg<n>;
     using Ln = Lanes<C, n>;
-    using Ct = CtLanes<C, n>;
     constexpr int N = F::N, R = F::R, T = F::T, tb = F::tb, NB = F::NB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
@@ -228,18 +229,14 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
         C tA[R / 2 + 1];
 #pragma unroll
         for (int t = 0; t <= R / 2; ++t) tA[t] = tw.get(key, t);
-        C t0[NB ? NB : 1], t1[NB ? NB : 1];
+        C t0[NB ? NB : 1];
         if (NB) {
             const int U = tb ? (int)(__brev((unsigned)u) >> (32 - tb)) : 0;
 #pragma unroll
             for (int b = F::BLO; b < n; ++b) {
                 const int jb = b - tb;
 #pragma unroll
-                for (int vv = 0; vv < (1 << jb); ++vv) {
-                    const int t = (U << jb) + brev(vv, jb);
-                    t0[F::offB(b) + vv] = tw.get(key, t);
-                    t1[F::offB(b) + vv] = tw.get(key, t + 1);
-                }
+                for (int vv = 0; vv < (1 << jb); ++vv) t0[F::offB(b) + vv] = tw.get(key, (U << jb) + brev(vv, jb));
             }
         }
         if (F::ZT) {
@@ -248,15 +245,46 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
             for (int t = u; t < F::ZT; t += T) zt[t] = tw.get(key, t);
             Ln::gsync(gm);
         }
+        const C z = n > 1 ? tA[1] : tw.get(key, 1), zc = mk<real>(z.x, -z.y);
         const int img1 = img0 + per < J.nimg ? img0 + per : J.nimg;
         for (int img = img0; img < img1; ++img) {
-            C* ptr = reinterpret_cast<C*>(J.X) + (size_t)img * J.img_stride + (size_t)row * N;
-            C v[R], w[R];
+            const size_t at = (size_t)img * J.img_stride + (size_t)row * N;
+            C v[R];
 #pragma unroll
-            for (int j = 0; j < R; j += 2) ld2(ptr + j + R * u, v[j], v[j + 1]);
-            Ct::template gram_oop<1, n>(v, w, tA, t0, t1, buf, u, gm, zt);
+            for (int j = 0; j < R; j += 2) ld2(in + at + j + R * u, v[j], v[j + 1]);
+            Ln::fwdA(v, tA, 1, n);
+            if (n > F::r) {
+                Ln::fwdM(v, tA, 1, n, u, zt);
+                Ln::toB(v, buf, u, gm);
 #pragma unroll
-            for (int j = 0; j < R; j += 2) st2(ptr + j + R * u, w[j], w[j + 1]);
+                for (int b = F::BLO; b < n; ++b) {
+                    const int jb = b - tb;
+#pragma unroll
+                    for (int j = 0; j < R; ++j) {
+                        if (j & (1 << jb)) continue;
+                        const C f0 = v[j], p = cmul(t0[F::offB(b) + (j & ((1 << jb) - 1))], v[j | (1 << jb)]);
+                        v[j] = cadd(f0, p);
+                        v[j | (1 << jb)] = cfma(z, p, f0);
+                    }
+                }
+#pragma unroll
+                for (int b = n - 1; b >= F::BLO; --b) {
+                    const int jb = b - tb;
+#pragma unroll
+                    for (int j = 0; j < R; ++j) {
+                        if (j & (1 << jb)) continue;
+                        const C g0 = v[j], g1 = v[j | (1 << jb)];
+                        v[j] = cadd(g0, g1);
+                        v[j | (1 << jb)] = cmulc(t0[F::offB(b) + (j & ((1 << jb) - 1))], cfma(zc, g1, g0));
+                    }
+                }
+                Ln::toA(v, buf, u, gm);
+                Ln::adjM(v, tA, 1, n, u, zt);
+            }
+            Ln::adjA(v, tA, 1, n);
+            C* ptr = reinterpret_cast<C*>(J.X) + at;
+#pragma unroll
+            for (int j = 0; j < R; j += 2) st2(ptr + j + R * u, v[j], v[j + 1]);
         }
     }
 }
@@ -401,19 +429,43 @@ __global__ void __launch_bounds__(256) rows_simple_kernel(const adrt_row_job J, 
     }
 }
 
-// ------------------------------------------------------------------ twiddle table (binary powering in FP64)
-template <typename real>
-__global__ void twiddle_table_kernel(int n, int K, const double2* __restrict__ z, cplx<real>* __restrict__ tab) {
-    const int H = (1 << n) / 2 + 1;
-    const long total = (long)K * H;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int k = (int)(i / H), t = (int)(i - (long)k * H);
-        double2 base = z[k], acc = make_double2(1.0, 0.0);
-        for (int e = t; e; e >>= 1) {
-            if (e & 1) acc = cmul(base, acc);
-            base = cmul(base, base);
+// ------------------------------------------------------------------ twiddle table (FP64)
+// One warp per row: z^t = (z^32)^(t / 32) z^(t mod 32), both factors by binary powering, one of each per lane, so an entry
+// costs one FP64 complex multiply (the table is bound by the FP64 pipe: 2 FMAs per clock and SM). z comes as complex
+// values, or (OM) from offset frequencies omega, z = exp(i omega).
+__device__ __forceinline__ double2 zpow(double2 base, int e) {
+    double2 acc = make_double2(1.0, 0.0);
+    for (; e; e >>= 1) {
+        if (e & 1) acc = cmul(base, acc);
+        base = cmul(base, base);
+    }
+    return acc;
+}
+template <typename real, typename OM>
+__global__ void __launch_bounds__(256) twiddle_table_kernel(int n, int K, const double2* __restrict__ zs,
+                                                            const OM* __restrict__ omega, cplx<real>* __restrict__ tab) {
+    const int H = (1 << n) / 2 + 1, lane = threadIdx.x & 31;
+    for (int k = blockIdx.x * 8 + (threadIdx.x >> 5); k < K; k += gridDim.x * 8) {
+        double2 z;
+        if (zs) z = zs[k];
+        else sincos((double)omega[k], &z.y, &z.x);
+        const double2 lo = zpow(z, lane);
+        double2 z32 = z;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) z32 = cmul(z32, z32);
+        for (int j0 = 0; j0 * 32 < H; j0 += 32) {
+            const double2 hi = zpow(z32, j0 + lane);
+            for (int j = 0; j < 32 && (j0 + j) * 32 < H; ++j) {
+                double2 h;
+                h.x = __shfl_sync(0xffffffffu, hi.x, j);
+                h.y = __shfl_sync(0xffffffffu, hi.y, j);
+                const int t = (j0 + j) * 32 + lane;
+                if (t < H) {
+                    const double2 w = cmul(h, lo);
+                    tab[(size_t)k * H + t] = mk<real>((real)w.x, (real)w.y);
+                }
+            }
         }
-        tab[i] = mk<real>((real)acc.x, (real)acc.y);
     }
 }
 
@@ -501,7 +553,7 @@ static int launch_prog(const adrt_row_job& J, const TwSrc<real>& tw, int total, 
 
 
 template <typename real, int n>
-static int launch_gram(const adrt_row_job& J, const TwSrc<real>& tw, cudaStream_t st) {
+static int launch_gram(const adrt_row_job& J, const void* in, const TwSrc<real>& tw, cudaStream_t st) {
     using F = FastCfg<n>;
     const size_t smem = (size_t)(FAST_THREADS / F::T) * F::GS * sizeof(cplx<real>);
     auto kern = rows_gram_kernel<real, n>;
@@ -512,8 +564,33 @@ static int launch_gram(const adrt_row_job& J, const TwSrc<real>& tw, cudaStream_
     while (per < 4 && (long long)J.nsel * ((J.nimg + 2 * per - 1) / (2 * per)) >= 2ll * slots * groups) per *= 2;
     const long long total = (long long)J.nsel * ((J.nimg + per - 1) / per);
     const long long ctas = (total + groups - 1) / groups;
-    kern<<<(unsigned)(ctas < slots ? ctas : slots), FAST_THREADS, smem, st>>>(J, tw, per, (int)total);
+    kern<<<(unsigned)(ctas < slots ? ctas : slots), FAST_THREADS, smem, st>>>(J, reinterpret_cast<const cplx<real>*>(in), tw, per,
+                                                                              (int)total);
     return launch_status("rows_gram_kernel");
+}
+
+// the Gram rows of a whole op list M over levels 1..n, from `in` (same layout as J.X) to J.X; -1 where the kernel does not
+// exist (FP64 above N = 256: a row's values and twiddles outgrow the registers)
+template <typename real>
+static int gram_dispatch(const adrt_row_job& J, const void* in, const TwSrc<real>& tw, cudaStream_t st) {
+    switch (J.n) {
+        case 1: return launch_gram<real, 1>(J, in, tw, st);
+        case 2: return launch_gram<real, 2>(J, in, tw, st);
+        case 3: return launch_gram<real, 3>(J, in, tw, st);
+        case 4: return launch_gram<real, 4>(J, in, tw, st);
+        case 5: return launch_gram<real, 5>(J, in, tw, st);
+        case 6: return launch_gram<real, 6>(J, in, tw, st);
+        case 7: return launch_gram<real, 7>(J, in, tw, st);
+        case 8: return launch_gram<real, 8>(J, in, tw, st);
+    }
+    if constexpr (std::is_same<real, float>::value) {
+        switch (J.n) {
+            case 9: return launch_gram<real, 9>(J, in, tw, st);
+            case 10: return launch_gram<real, 10>(J, in, tw, st);
+            case 11: return launch_gram<real, 11>(J, in, tw, st);
+        }
+    }
+    return -1;
 }
 
 template <typename real>
@@ -554,26 +631,9 @@ static int rows_dispatch(const adrt_row_job& J, int iters, double safety, double
                 break;
         }
     }
-    if (!pout && prog_n && J.nops == 1 && J.op[0] == ADRT_OP_M && J.lo[0] == 1 && J.hi[0] == J.n) {
-        switch (J.n) {
-            case 1: return launch_gram<real, 1>(J, tw, st);
-            case 2: return launch_gram<real, 2>(J, tw, st);
-            case 3: return launch_gram<real, 3>(J, tw, st);
-            case 4: return launch_gram<real, 4>(J, tw, st);
-            case 5: return launch_gram<real, 5>(J, tw, st);
-            case 6: return launch_gram<real, 6>(J, tw, st);
-            case 7: return launch_gram<real, 7>(J, tw, st);
-            case 8: return launch_gram<real, 8>(J, tw, st);
-            case 9:
-                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 9>(J, tw, st);
-                break;
-            case 10:
-                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 10>(J, tw, st);
-                break;
-            case 11:
-                if constexpr (std::is_same<real, float>::value) return launch_gram<real, 11>(J, tw, st);
-                break;
-        }
+    if (!pout && J.nops == 1 && J.op[0] == ADRT_OP_M && J.lo[0] == 1 && J.hi[0] == J.n) {
+        const int rc = gram_dispatch<real>(J, J.X, tw, st);
+        if (rc >= 0) return rc;
     }
     if (fast_ok(J)) {
         switch (J.n) {
@@ -627,19 +687,55 @@ int rows_run(const adrt_row_job* J, int iters, double safety, double* pout, cuda
     return rows_dispatch<double>(*J, iters, safety, pout, st);
 }
 
-int twiddle_table(int dtype, int n, int K, const double* z, void* tab, cudaStream_t st) {
-    if (n < 1 || n > 11 || K < 0 || (K && (!z || !tab))) { set_error("twiddle_table: bad arguments"); return ADRT_EINVAL; }
-    if (!K) return ADRT_OK;
-    const long total = (long)K * ((1 << n) / 2 + 1);
-    int grid = (int)((total + 255) / 256);
+template <typename OM>
+static int launch_twiddles(int dtype, int n, int K, const double* z, const OM* omega, void* tab, cudaStream_t st) {
+    const double2* zs = reinterpret_cast<const double2*>(z);
+    int grid = (K + 7) / 8;
     if (grid > 4096) grid = 4096;
     if (dtype == ADRT_F32)
-        twiddle_table_kernel<float><<<grid, 256, 0, st>>>(n, K, reinterpret_cast<const double2*>(z),
-                                                           reinterpret_cast<float2*>(tab));
+        twiddle_table_kernel<float, OM><<<grid, 256, 0, st>>>(n, K, zs, omega, reinterpret_cast<float2*>(tab));
     else
-        twiddle_table_kernel<double><<<grid, 256, 0, st>>>(n, K, reinterpret_cast<const double2*>(z),
-                                                            reinterpret_cast<double2*>(tab));
+        twiddle_table_kernel<double, OM><<<grid, 256, 0, st>>>(n, K, zs, omega, reinterpret_cast<double2*>(tab));
     return launch_status("twiddle_table_kernel");
 }
 
+int twiddle_table(int dtype, int n, int K, const double* z, void* tab, cudaStream_t st) {
+    if (n < 1 || n > 11 || K < 0 || (K && (!z || !tab))) { set_error("twiddle_table: bad arguments"); return ADRT_EINVAL; }
+    if (!K) return ADRT_OK;
+    return launch_twiddles<double>(dtype, n, K, z, nullptr, tab, st);
+}
+
+// gram_freq of the adrt patch: out[b, k] = A_k^* A_k a[b, k], A_k = B_n ... B_1 at frequency omega[k] (in a's precision)
+int gram_freq(int dtype, int n, int nimg, int rows, const void* a, void* out, const void* omega, void* tab,
+              int32_t* counter, cudaStream_t st) {
+    adrt_row_job J = {};
+    J.dtype = dtype; J.n = n; J.nimg = nimg; J.nsel = rows; J.img_stride = (int64_t)rows << n; J.X = out;
+    J.freq_mod = rows; J.twtab = tab; J.counter = counter;
+    J.nops = 1; J.op[0] = ADRT_OP_M; J.lo[0] = 1; J.hi[0] = n;
+    if (int rc = validate_job(&J)) return rc;
+    if (!a || !omega || (reinterpret_cast<uintptr_t>(a) & 15) || (long long)nimg * rows > 0x7fffff00LL) {
+        set_error("gram_freq: bad arguments (null or misaligned rows, or too many)");
+        return ADRT_EINVAL;
+    }
+    if (!nimg || !rows) return ADRT_OK;
+    int rc = dtype == ADRT_F32 ? launch_twiddles(dtype, n, rows, nullptr, reinterpret_cast<const float*>(omega), tab, st)
+                               : launch_twiddles(dtype, n, rows, nullptr, reinterpret_cast<const double*>(omega), tab, st);
+    if (rc) return rc;
+    if (dtype == ADRT_F32) {
+        TwSrc<float> tw = {nullptr, reinterpret_cast<const float2*>(tab), (2 << n) - 1, (1 << n) / 2 + 1};
+        return gram_dispatch<float>(J, a, tw, st);
+    }
+    TwSrc<double> tw = {nullptr, reinterpret_cast<const double2*>(tab), (2 << n) - 1, (1 << n) / 2 + 1};
+    rc = gram_dispatch<double>(J, a, tw, st);
+    if (rc >= 0) return rc;
+    const size_t bytes = ((size_t)nimg * rows << n) * sizeof(double2);
+    if ((rc = cuda_status(cudaMemcpyAsync(out, a, bytes, cudaMemcpyDeviceToDevice, st), "gram_freq copy"))) return rc;
+    return rows_run(&J, 0, 0.0, nullptr, st);
+}
+
 }  // namespace adrt
+
+extern "C" int adrt_gram_freq(int dtype, int n, int nimg, int rows, const void* a, void* out, const void* omega, void* tab,
+                              int32_t* counter, void* stream) {
+    return adrt::gram_freq(dtype, n, nimg, rows, a, out, omega, tab, counter, adrt::as_stream(stream));
+}

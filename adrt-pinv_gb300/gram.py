@@ -8,8 +8,8 @@ reference's patch to the `adrt` package (patches/adrt-gram-freq.patch):
   lstsq_cheb(b, ...)    adrt.core.lstsq_cheb (patch, core.py): the fixed-degree Chebyshev least-squares inverse
                         x_D = c_D(R^T R) R^T b on a spectral interval [lam_min, lam_max]
 
-All three run on the library's kernels: gram_freq is the row engine's Gram op ('M', 1, n) with a per-row twiddle
-table built on the device from omega; gram and lstsq_cheb are the device pipeline of the packed passes
+All three run on the library's kernels: gram_freq is the row engine's Gram kernel with a per-row twiddle table built on
+the device from omega; gram and lstsq_cheb are the device pipeline of the packed passes
 (pack + FFT kernel, row engine, inverse FFT + unpack) with that op, and lstsq_cheb's iteration is the pipeline's
 outer Chebyshev step (FP64 iterates). Images and sinograms are in this repository's (the reference's) layout;
 R^T R does not depend on the layout. The patch's mapping between the `adrt` package's sinogram layout and this one
@@ -18,13 +18,11 @@ R^T R does not depend on the layout. The patch's mapping between the `adrt` pack
 float32 input runs the rows in FP32 (complex64), float64 in FP64; NumPy in -> NumPy out, torch in -> torch out.
 """
 
-import ctypes
-
 import numpy as np
 import torch
 
 from . import _lib as C
-from .device import OPCODE, Pipeline
+from .device import Pipeline
 from .plan import Plan
 
 _REAL = {torch.complex64: torch.float32, torch.complex128: torch.float64}
@@ -52,22 +50,14 @@ def gram_freq(a, omega):
     if n > 11:
         raise ValueError("N above 2048 is not supported")
     dev = at.device if at.is_cuda else torch.device("cuda")
-    X = at.to(dev).reshape(-1, rows, N).contiguous().clone()
-    z = torch.polar(torch.ones(rows, dtype=torch.float64, device=dev), om.to(dev, torch.float64))
-    code = C.dtype_code(_REAL[at.dtype])
-    st = C.stream_handle()
+    X = at.to(dev).resolve_conj().contiguous()
+    if X.data_ptr() % 16:
+        X = X.clone()  # rows are read in 16-byte pieces
+    out = torch.empty_like(X)
     tab = torch.empty((rows, N // 2 + 1), dtype=at.dtype, device=dev)
-    C.call("adrt_twiddle_table", code, n, rows, C.ptr(z), C.ptr(tab), st)
-    counter = torch.zeros(4, dtype=torch.int32, device=dev)
-    j = C.RowJob()
-    j.dtype, j.n, j.nimg, j.nsel, j.img_stride = code, n, X.shape[0], rows, rows * N
-    j.X, j.rows, j.freq_mod, j.roots, j.twtab = X.data_ptr(), None, rows, None, tab.data_ptr()
-    j.deg, j.coef, j.coef_stride, j.tau = None, None, 0, 0.0
-    j.nops = 1
-    j.op[0], j.lo[0], j.hi[0] = OPCODE["M"], 1, n
-    j.counter, j.grid = counter.data_ptr(), 0
-    C.call("adrt_rows_run", ctypes.byref(j), st)
-    out = X.reshape(at.shape)
+    counter = torch.empty(4, dtype=torch.int32, device=dev)
+    C.call("adrt_gram_freq", C.dtype_code(at.dtype), n, X.numel() // (rows * N), rows, C.ptr(X), C.ptr(out),
+           C.ptr(om.to(dev).contiguous()), C.ptr(tab), C.ptr(counter), C.stream_handle())
     return out if is_torch and at.is_cuda else (out.cpu() if is_torch else out.cpu().numpy())
 
 
@@ -84,10 +74,11 @@ class NormalOperator:
         self.pipe.ops = {"G": [("B", 1, n), ("BT", 1, n)], "BP": [("BT", 1, n)]}
         self.out = torch.empty((self.B, N, N), dtype=torch.float64, device=self.pipe.device)
 
-    def gram(self, x):
-        """R^T R x for x (B, N, N) real on the device; returns an FP64 buffer (valid until the next call)."""
+    def gram(self, x, out=None):
+        """R^T R x for x (B, N, N) real on the device, into out (FP32 or FP64; default: an FP64 buffer valid until the
+        next call)."""
         self.pipe.G(x)
-        return self.pipe.sum_parts(self.out)
+        return self.pipe.sum_parts(self.out if out is None else out)
 
     def lstsq_cheb(self, b, lo, hi, deg):
         """x_deg = c_deg(R^T R) R^T b for sinograms b (B, 4, 2N-1, N) FP64 on the device (FP64 result buffer)."""
@@ -118,13 +109,6 @@ def _images(a):
     return is_torch, at
 
 
-def _back(x, like, is_torch, dtype):
-    x = x.reshape(like).to(dtype)
-    if is_torch:
-        return x
-    return x.cpu().numpy()
-
-
 def gram(a, device="cuda"):
     """R^T R a for square images a (..., N, N) float32 / float64 (adrt.core.gram of the patch), same shape and
     dtype; N = 1 is the identity."""
@@ -135,9 +119,8 @@ def gram(a, device="cuda"):
     n = N.bit_length() - 1
     x = at.reshape(-1, N, N).to(device).contiguous()
     op = _operator(n, x.shape[0], "fp32" if at.dtype == torch.float32 else "fp64", device)
-    out = op.gram(x)
-    res = _back(out, at.shape, is_torch, at.dtype)
-    return res.to(at.device) if is_torch else res
+    res = op.gram(x, torch.empty_like(x)).reshape(at.shape)
+    return res.to(at.device) if is_torch else res.cpu().numpy()
 
 
 def lstsq_cheb(b, *, lam_min, lam_max=None, tol=1e-10, degree=None, device="cuda"):

@@ -133,17 +133,25 @@ int adrt_rows_run_multi(const adrt_row_job* jobs, const int32_t* code, const int
  * 6 <= n <= 9. */
 int adrt_rows_operator(int dtype, int n, int nimg, int kind, const void* T, void* Y, long long img_stride,
                        const void* roots8, void* stream);
-/* The same pass for FP32 rows on the tensor cores (n = 8, 9), the operators split once into FP16 pairs:
+/* The same pass for FP32 rows on the tensor cores (n = 7, 8, 9), the operators split once into FP16 pairs:
  * adrt_rows_operator_split turns the FP32 T above, frequency k scaled by scale[k] (a power of two; largest entry below
- * 2^14 after scaling), into Ts ((N+1) N^2 FP16 values, hi and lo tiles in the kernel's order); inv_scale[k] = 1/scale[k].
+ * 2^14 after scaling), into Ts (adrt_rows_operator_split_size(n) FP16 values, hi and lo tiles in the kernel's order);
+ * inv_scale[k] = 1/scale[k].
  * err: device int, set to a positive code if a bounded wait ran out (the rows are then not all written). */
+long long adrt_rows_operator_split_size(int n);
 int adrt_rows_operator_split(int n, const void* T, const float* scale, void* Ts, void* stream);
 int adrt_rows_operator_mma(int n, int nimg, int kind, const void* Ts, const float* inv_scale, void* Y,
                            long long img_stride, const void* roots8, int32_t* err, void* stream);
 
 /* Per-row twiddle table tab[k*(N/2+1) + t] = z_k^t (t = 0..N/2) from K complex z (FP64 in, dtype out),
- * by binary powering in FP64. */
+ * evaluated in FP64. */
 int adrt_twiddle_table(int dtype, int n, int K, const double* z, void* tab, void* stream);
+
+/* gram_freq of the reference's adrt patch: out[b, k] = A_k^* A_k a[b, k] for nimg x rows x N complex rows (dtype), A_k =
+ * B_n ... B_1 at offset frequency omega[k] (real, same precision). tab: rows x (N/2+1) complex scratch (dtype); counter:
+ * device int. out may equal a; both 16-byte aligned. */
+int adrt_gram_freq(int dtype, int n, int nimg, int rows, const void* a, void* out, const void* omega, void* tab,
+                   int32_t* counter, void* stream);
 
 /* Power iteration for Lambda_k (fastcpp.py:102-118): V (K x N, dtype) is iterated `iters` times
  * V <- M V / ||M V|| row-wise (M = B^* B over levels m_lo..n) and out[k] = safety * Re <V_k, M V_k> (FP64 out).
