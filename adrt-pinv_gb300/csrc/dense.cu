@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(TC_THREADS) dense_tc_kernel(int N, int nimg, c
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (threadIdx.x == 0) {
+        if (warp == 0 && elect_one()) {
             const uint32_t d = tmem + (uint32_t)(s * BP);
 #pragma unroll
             for (int k8 = 0; k8 < TC_KC / 8; ++k8) {
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(TC_THREADS) dense_tc_kernel(int N, int nimg, c
             promote(s);
         }
     }
-    if (!ok && threadIdx.x == 0) {
+    if (!ok && warp == 0 && elect_one()) {
         // a wait gave up while MMAs of this CTA may still be writing its TMEM columns: before the columns are freed
         // (and possibly handed to the next CTA on this SM), one more commit of every tcgen05 operation this thread
         // issued goes to the spare barrier, awaited with the same bound. Flag 1: the launch's dense rows were not
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) dense_cx_kernel(int N, int nimg
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t d = tmem + (uint32_t)(be * NACC);
                     const uint32_t a0 = smem_addr(smem_raw + s * STAGE), x0 = a0 + A_BYTES;
 #pragma unroll
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(CX_THREADS, 1) dense_cx_kernel(int N, int nimg
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (*abort_flag && threadIdx.x == 32) {
+    if (*abort_flag && warp == 1 && elect_one()) {
         // a wait gave up: before the tensor memory is freed and the CTA leaves, every MMA issued (one more commit to
         // the spare barrier) and every operator copy issued (the stages' byte counts) must have completed; the waits
         // are bounded. Flag 1: this launch's dense rows were not written; 2: even the drain ran out.

@@ -22,6 +22,15 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
     return r;
 }
 
+// one thread of a converged warp, the same one every time. MMAs are issued behind it and not behind a lane test: ptxas
+// then knows the branch to be taken by one thread and issues from uniform registers (measured with M = 128, N = 64: 60
+// clocks per tcgen05.mma against 153 behind `lane == 0`, whatever N or layout)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e != 0;
+}
+
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -59,7 +68,8 @@ __device__ __forceinline__ void mbar_expect_bulk(uint32_t mbar, uint32_t dst, co
                  : "memory");
 }
 
-// bounded wait that also gives up when another role of the CTA has set the abort flag
+// bounded wait that also gives up when another role of the CTA has set the abort flag (no suspend-time hint: with one,
+// waiters wake late; 20 us cost the row operators 3% at N = 256 and 20% at N = 512)
 __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t mbar, uint32_t parity, const volatile int* abort_flag) {
     for (long it = 0; it < (1L << 24); ++it) {
         uint32_t done;

@@ -375,7 +375,7 @@ def _rows_apply_f64(X, z_rows, ops, n, counter):
 # below, the polynomial rows are a few microseconds of latency
 ROW_OPS_MIN, ROW_OPS_MAX = 6, 9
 # batch sizes from which the FP32 row operators run on the tensor cores, by n
-ROW_OPS_MMA_BATCH = {8: 5, 9: 3}
+ROW_OPS_MMA_BATCH = {7: 4, 8: 2, 9: 2}
 
 
 def row_operators_for(plan: Plan):
@@ -390,10 +390,10 @@ def row_operators_for(plan: Plan):
 def row_operator_bytes(plan: Plan, real, batch):
     """Device bytes of a plan's row operators (G and BP) and of their phases, for a pipeline of that batch and precision."""
     N = plan.N
-    total = 2 * (N + 1) * N * N // 2 * real.itemsize + 8 * N * 2 * real.itemsize
+    phases = 8 * N * 2 * real.itemsize
     if real == torch.float32 and batch >= ROW_OPS_MMA_BATCH.get(plan.n, batch + 1):
-        total += 2 * (N + 1) * 4  # the inverse scales of the split form (its tiles take the FP32 operators' bytes)
-    return total
+        return 2 * (C.load().adrt_rows_operator_split_size(plan.n) * 2 + (N + 1) * 4) + phases  # tiles, inverse scales
+    return 2 * (N + 1) * N * N // 2 * real.itemsize + phases
 
 
 def _split_operators(n, T):
@@ -402,7 +402,7 @@ def _split_operators(n, T):
     _, e = torch.frexp(T.abs().amax(dim=(1, 2, 3)))
     one = torch.ones_like(e, dtype=torch.float32)
     scale = torch.ldexp(one, 14 - e)
-    Ts = torch.empty((T.numel(), 2), dtype=torch.float16, device=T.device)
+    Ts = torch.empty(C.load().adrt_rows_operator_split_size(n), dtype=torch.float16, device=T.device)
     C.call("adrt_rows_operator_split", n, C.ptr(T), C.ptr(scale), C.ptr(Ts), C.stream_handle())
     Ts._adrt_inv_scale = torch.ldexp(one, e - 14)
     return Ts
