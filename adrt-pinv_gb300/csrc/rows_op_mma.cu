@@ -52,7 +52,6 @@ template <int n> struct OmCfg {
     static constexpr int ODD = STACK ? (H / 8) * LBO : 2 * BT;  // from E to O in a buffer
     static constexpr int NB = n == 9 ? 1 : 2;  // B buffers, each with its group of eight loader warps
     static constexpr int THREADS = 32 * (8 + 8 * NB);
-    static constexpr int EV = NB == 2 ? 4 : 8;  // vectors per epilogue step (registers)
     static constexpr int ACC = PARS * 4 * VT;  // TMEM columns per accumulator set: product x {lo terms, hi.hi} x 2 VT
     static constexpr size_t smem = (size_t)RING * CHUNK * 2 + (size_t)NB * BBUF + 1024;
 };
@@ -108,25 +107,19 @@ __device__ __forceinline__ void store_split(unsigned char* hi, unsigned char* lo
     }
 }
 
-template <int C> __device__ __forceinline__ void tmem_ld(uint32_t addr, float (&v)[C]) {
-    uint32_t t[C];
-    if constexpr (C == 8) {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
-                     : "r"(addr));
-    } else {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3])
-                     : "r"(addr));
-    }
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, float (&v)[4]) {
+    uint32_t t[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3])
+                 : "r"(addr));
 #pragma unroll
-    for (int q = 0; q < C; ++q) v[q] = __uint_as_float(t[q]);
+    for (int q = 0; q < 4; ++q) v[q] = __uint_as_float(t[q]);
 }
 
-template <int n>
+template <int n, bool BP>
 __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
     rows_op_mma_kernel(int nimg, int tiles, const __half* __restrict__ Ts, const float* __restrict__ tinv, float2* Y,
-                       long long img_stride, const float2* __restrict__ roots, bool bp, int* __restrict__ err) {
+                       long long img_stride, const float2* __restrict__ roots, int* __restrict__ err) {
     using W = OmCfg<n>;
     constexpr int N = W::N, H = W::H, L = W::L, VT = W::VT, LPV = W::LPV, CPL = W::CPL;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -203,13 +196,14 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
     } else if (warp == 1) {  // MMAs
         // D f32 (bit 4), A and B f16, K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(2 * VT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t a0 = desc_lo(smem_addr(ring), 128);
         int ch = 0, un = 0, ac = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
             if ((u % tiles) * VT >= vectors(u / tiles)) continue;
             const int bi = un % W::NB, br = un / W::NB;
             if (!warp_wait(smem_addr(&b_full[bi]), (uint32_t)(br & 1), abort_flag)) ok = false;
-            const uint32_t b0 = smem_addr(bbuf + (size_t)bi * W::BBUF);
+            const uint32_t b0 = desc_lo(smem_addr(bbuf + (size_t)bi * W::BBUF), W::LBO);
             for (int mt = 0; ok && mt < W::MT; ++mt, ++ac) {
                 const int ai = ac & 1, ar = ac >> 1;
                 if (ar > 0 && !warp_wait(smem_addr(&acc_free[ai]), (uint32_t)((ar - 1) & 1), abort_flag)) {
@@ -226,18 +220,17 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                     if (elect_one()) {
                         *s_consumed = ch + 1;
                         const uint32_t dl = tmem + (uint32_t)(ai * W::ACC + par * 4 * VT), dh = dl + 2 * VT;
-                        const uint32_t a0 = smem_addr(ring + (size_t)s * W::CHUNK * 2);
-                        const uint32_t bt = b0 + (uint32_t)(par * 2 * W::BT);
+                        constexpr uint32_t AHI = desc_hi((W::KC / 8) * 128), BHI = desc_hi(W::SBO);
+                        // byte offsets in 16-byte units: hi to lo tile, one MMA's K
+                        constexpr uint32_t ALO = 128 * W::KC * 2 / 16, AK = 256 / 16, BLO = W::BT / 16, BK = 2 * W::LBO / 16;
+                        const uint32_t ah = a0 + (uint32_t)(s * (W::CHUNK * 2 / 16));
+                        const uint32_t bh = b0 + (uint32_t)(par * 2 * BLO + kc * (W::KC / 16) * BK);
 #pragma unroll
                         for (int ks = 0; ks < W::KC / 16; ++ks) {
-                            const int kk = kc * (W::KC / 16) + ks;
-                            const uint64_t ah = desc_kmajor(a0 + ks * 256, 128, (W::KC / 8) * 128);
-                            const uint64_t al = desc_kmajor(a0 + 128 * W::KC * 2 + ks * 256, 128, (W::KC / 8) * 128);
-                            const uint64_t bh = desc_kmajor(bt + kk * 2 * W::LBO, W::LBO, W::SBO);
-                            const uint64_t bl = desc_kmajor(bt + W::BT + kk * 2 * W::LBO, W::LBO, W::SBO);
-                            mma_f16(dl, al, bh, idesc, kk > 0 ? 1u : 0u);
-                            mma_f16(dl, ah, bl, idesc, 1u);
-                            mma_f16(dh, ah, bh, idesc, kk > 0 ? 1u : 0u);
+                            const uint32_t acc = ks > 0 || kc > 0 ? 1u : 0u;
+                            mma_f16(dl, ah + ALO + ks * AK, AHI, bh + ks * BK, BHI, idesc, acc);
+                            mma_f16(dh, ah + ks * AK, AHI, bh + ks * BK, BHI, idesc, acc);
+                            mma_f16(dl, ah + ks * AK, AHI, bh + BLO + ks * BK, BHI, idesc, 1u);
                         }
                         tc_commit(&a_free[s]);
                     }
@@ -265,8 +258,15 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
             for (int mt = 0; mt < W::MT; ++mt, ++ac) {
                 const int ai = ac & 1, o = mt * 128 + (warp & 3) * 32 + lane;
                 const int c = W::STACK && o >= H ? N - 1 - (o - H) : o;  // the output, or the first of a mirrored pair
-                const float2 pa = roots[op_phase_out<n>(k, c)];
-                const float2 pb = W::STACK ? pa : roots[op_phase_out<n>(k, N - 1 - c)];
+                // the conjugate of pa is applied; rows of -k take pa itself. The matrices' scale rides along
+                float2 pa = roots[op_phase_out<n>(k, c)], pb = W::STACK ? pa : roots[op_phase_out<n>(k, N - 1 - c)];
+                pa = cscale(ti, pa);
+                pb = cscale(ti, pb);
+                const float2 na = make_float2(pa.x, self ? pa.y : -pa.y), nb = make_float2(pb.x, self ? pb.y : -pb.y);
+                // vectors v0 + 4 i + q: rows (q & 1) of frequency k, for q >= 2 of -k (self: of the next image)
+                float2* y0 = Y + (long long)(self ? v0 / 2 : v0 / 4) * img_stride;
+                const int r0 = k * N, r1 = (L + k) * N, r2 = self ? r0 : (L - k) * N, r3 = self ? r1 : (2 * L - k) * N;
+                const long long step = (self ? 2 : 1) * img_stride, next = self ? img_stride : 0;
                 if (!warp_wait(smem_addr(&acc_full[ai]), (uint32_t)((ac >> 1) & 1), abort_flag)) {
                     if (lane == 0) *abort_flag = 1;
                     ok = false;
@@ -274,45 +274,35 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + lane_base + (uint32_t)(ai * W::ACC);
-                constexpr int EV = W::EV;
+                const int left = nv - v0;
 #pragma unroll 1
-                for (int vb = 0; vb < VT; vb += EV) {
-                    if (v0 + vb >= nv) break;
-                    float er[EV], ei[EV], t0[EV], t1[EV], orr[EV], oi[EV], t2[EV], t3[EV];
-                    tmem_ld<EV>(d + vb, er);
-                    tmem_ld<EV>(d + VT + vb, ei);
-                    tmem_ld<EV>(d + 2 * VT + vb, t0);
-                    tmem_ld<EV>(d + 3 * VT + vb, t1);
+                for (int vb = 0; vb < VT && vb < left; vb += 4, y0 += step) {
+                    float er[4], ei[4], t0[4], t1[4], orr[4], oi[4], t2[4], t3[4];
+                    tmem_ld4(d + vb, er);
+                    tmem_ld4(d + VT + vb, ei);
+                    tmem_ld4(d + 2 * VT + vb, t0);
+                    tmem_ld4(d + 3 * VT + vb, t1);
                     if constexpr (!W::STACK) {
-                        tmem_ld<EV>(d + 4 * VT + vb, orr);
-                        tmem_ld<EV>(d + 5 * VT + vb, oi);
-                        tmem_ld<EV>(d + 6 * VT + vb, t2);
-                        tmem_ld<EV>(d + 7 * VT + vb, t3);
+                        tmem_ld4(d + 4 * VT + vb, orr);
+                        tmem_ld4(d + 5 * VT + vb, oi);
+                        tmem_ld4(d + 6 * VT + vb, t2);
+                        tmem_ld4(d + 7 * VT + vb, t3);
                     }
+                    const float4 s4 = *reinterpret_cast<const float4*>(iv + vb);
+                    const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int q = 0; q < EV; ++q) {
-                        const int v = v0 + vb + q;
-                        if (v >= nv) break;
-                        const float sc = iv[vb + q] * ti;
-                        const bool neg = !self && (v & 2);
-                        const int img = self ? v >> 1 : v >> 2, row = (v & 1) * L + (neg ? L - k : k);
-                        float2* y = Y + (long long)img * img_stride + (long long)row * N;
-                        const float e_r = er[q] + t0[q], e_i = ei[q] + t1[q];
-                        if constexpr (W::STACK) {
-                            float2 z = cmulc(pa, make_float2(e_r * sc, e_i * sc));
-                            if (neg) z.y = -z.y;
-                            y[c] = z;
-                        } else {
-                            const float o_r = orr[q] + t2[q], o_i = oi[q] + t3[q];
-                            float2 za = cmulc(pa, make_float2((e_r + o_r) * sc, (e_i + o_i) * sc));
-                            float2 zb = cmulc(pb, make_float2((e_r - o_r) * sc, (e_i - o_i) * sc));
-                            if (neg) {
-                                za.y = -za.y;
-                                zb.y = -zb.y;
+                    for (int q = 0; q < 4; ++q) {
+                        if (vb + q < left) {
+                            float2* y = y0 + (q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 + next : r3 + next);
+                            const float e_r = er[q] + t0[q], e_i = ei[q] + t1[q];
+                            if constexpr (W::STACK) {
+                                y[c] = cmulc(q < 2 ? pa : na, make_float2(e_r * sc[q], e_i * sc[q]));
+                            } else {
+                                const float o_r = orr[q] + t2[q], o_i = oi[q] + t3[q];
+                                y[c] = cmulc(q < 2 ? pa : na, make_float2((e_r + o_r) * sc[q], (e_i + o_i) * sc[q]));
+                                y[N - 1 - c] = cmulc(q < 2 ? pb : nb, make_float2((e_r - o_r) * sc[q], (e_i - o_i) * sc[q]));
                             }
-                            y[c] = za;
-                            y[N - 1 - c] = zb;
                         }
                     }
                 }
@@ -341,9 +331,8 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
             auto load = [&](int vb) {
                 const int v = v0 + vb + vs;
                 if (vb < VT && v < nv) {
-                    const bool neg = !self && (v & 2);
-                    const int img = self ? v >> 1 : v >> 2, row = (v & 1) * L + (neg ? L - k : k);
-                    const float2* y = Y + (long long)img * img_stride + (long long)row * N;
+                    const int img = self ? v >> 1 : v >> 2, row = (v & 1) * L + (!self && (v & 2) ? L - k : k);
+                    const float2* y = Y + (long long)img * img_stride + row * N;
 #pragma unroll
                     for (int q = 0; q < CPL / 2; ++q) {
                         const int c = 2 * l + 2 * LPV * q;
@@ -353,13 +342,21 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                 }
             };
             load(w8 * VPW);
-            float2 pa[CPL], pb[CPL];  // phases of entries c = 2 l + 2 LPV q + r and N - 1 - c
+            // phases of entries c = 2 l + 2 LPV q + r and N - 1 - c; a lane's vectors all have the same kind (row 0 or 1 of
+            // frequency k or -k), and the rows of -k take the conjugates
+            const bool neg = !self && ((w8 * VPW + vs) & 2);
+            float2 pa[CPL], pb[CPL];
 #pragma unroll
             for (int i = 0; i < CPL; ++i) {
                 const int c = 2 * l + 2 * LPV * (i / 2) + (i & 1);
-                pa[i] = roots[op_phase_in<n>(k, c, bp)];
-                pb[i] = roots[op_phase_in<n>(k, N - 1 - c, bp)];
+                pa[i] = roots[op_phase_in<n>(k, c, BP)];
+                pb[i] = roots[op_phase_in<n>(k, N - 1 - c, BP)];
+                if (neg) {
+                    pa[i].y = -pa[i].y;
+                    pb[i].y = -pb[i].y;
+                }
             }
+            const float os = neg ? -1.f : 1.f;  // BP: O = -i (a - b), conjugated for -k
             // the buffer's previous unit must have been multiplied
             if (br > 0 && !warp_wait(smem_addr(&b_free[bi]), (uint32_t)((br - 1) & 1), abort_flag)) {
                 if (lane == 0) *abort_flag = 1;
@@ -371,16 +368,15 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                 const int vr = vb + vs, v = v0 + vr;
                 float er[CPL], ei[CPL], orr[CPL], oi[CPL], m = 0.f;
                 if (v < nv) {
-                    const float sg = !self && (v & 2) ? -1.f : 1.f;  // the row of -k enters conjugated
 #pragma unroll
                     for (int i = 0; i < CPL; ++i) {
                         const float4 p = ya[i / 2], q = yb[i / 2];
-                        const float2 a = cmul(pa[i], (i & 1) ? make_float2(p.z, sg * p.w) : make_float2(p.x, sg * p.y));
-                        const float2 b = cmul(pb[i], (i & 1) ? make_float2(q.x, sg * q.y) : make_float2(q.z, sg * q.w));
+                        const float2 a = cmul(pa[i], (i & 1) ? make_float2(p.z, p.w) : make_float2(p.x, p.y));
+                        const float2 b = cmul(pb[i], (i & 1) ? make_float2(q.x, q.y) : make_float2(q.z, q.w));
                         er[i] = a.x + b.x;
                         ei[i] = a.y + b.y;
-                        orr[i] = bp ? a.y - b.y : a.x - b.x;
-                        oi[i] = bp ? b.x - a.x : a.y - b.y;
+                        orr[i] = BP ? os * (a.y - b.y) : a.x - b.x;
+                        oi[i] = BP ? os * (b.x - a.x) : a.y - b.y;
                         m = fmaxf(m, fmaxf(fmaxf(fabsf(er[i]), fabsf(ei[i])), fmaxf(fabsf(orr[i]), fabsf(oi[i]))));
                     }
                 }
@@ -421,18 +417,18 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-template <int n>
-static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long long img_stride, const void* roots, bool bp,
-                      int* err, cudaStream_t st) {
+template <int n, bool BP>
+static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long long img_stride, const void* roots, int* err,
+                      cudaStream_t st) {
     using W = OmCfg<n>;
     static_assert(W::smem <= 227 * 1024, "shared memory");
-    auto kern = rows_op_mma_kernel<n>;
+    auto kern = rows_op_mma_kernel<n, BP>;
     if (int rc = ensure_smem((const void*)kern, W::smem)) return rc;
     const int tiles = (4 * nimg + W::VT - 1) / W::VT;
     const int total = (W::N + 1) * tiles, sms = device_sm_count();
     kern<<<total < sms ? total : sms, W::THREADS, W::smem, st>>>(
         nimg, tiles, reinterpret_cast<const __half*>(Ts), tinv, reinterpret_cast<float2*>(Y), img_stride,
-        reinterpret_cast<const float2*>(roots), bp, err);
+        reinterpret_cast<const float2*>(roots), err);
     return launch_status("rows_op_mma_kernel");
 }
 
@@ -473,7 +469,12 @@ extern "C" int adrt_rows_operator_mma(int n, int nimg, int kind, const void* Ts,
     }
     if (!nimg) return ADRT_OK;
     cudaStream_t st = as_stream(stream);
-    if (n == 7) return launch_mma<7>(nimg, Ts, inv_scale, Y, img_stride, roots8, kind == 1, err, st);
-    if (n == 8) return launch_mma<8>(nimg, Ts, inv_scale, Y, img_stride, roots8, kind == 1, err, st);
-    return launch_mma<9>(nimg, Ts, inv_scale, Y, img_stride, roots8, kind == 1, err, st);
+    switch (2 * n + kind) {
+        case 14: return launch_mma<7, false>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+        case 15: return launch_mma<7, true>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+        case 16: return launch_mma<8, false>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+        case 17: return launch_mma<8, true>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+        case 18: return launch_mma<9, false>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+        default: return launch_mma<9, true>(nimg, Ts, inv_scale, Y, img_stride, roots8, err, st);
+    }
 }
