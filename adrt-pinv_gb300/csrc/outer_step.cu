@@ -73,9 +73,11 @@ struct OuterStepArgs {
     // the same coefficients rounded to FP32 once on the host (the register-resident kernel runs no FP64 per thread):
     // the stencil's, and hi + lo splits of the outer ones
     float g1f_a0;
-    float g1f_a[OS_MAX_STEPS];
-    float g1f_1[OS_MAX_STEPS];
     float oa_hi, oa_lo, o1_hi, o1_lo, a0_hi, a0_lo;
+    // the recurrence the register-resident kernels run: with d_k = c_{k+1} - c_k = gam_k e_k, gam_k the running product of om_1,
+    // e_k = e_{k-1} + bet_k r and c_{k+1} = c_k + gam_k e_k (two multiply-adds instead of four operations)
+    float g1f_bet[OS_MAX_STEPS];
+    float g1f_gam[OS_MAX_STEPS];
 };
 
 // fill the FP32 copies of the coefficients (host)
@@ -85,9 +87,11 @@ static void fill_f32_coefficients(OuterStepArgs& A) {
         lo = (float)(v - (double)hi);
     };
     A.g1f_a0 = (float)A.g1_a0;
+    double gam = 1.0;
     for (int k = 0; k + 1 < A.g1_deg && k < OS_MAX_STEPS; ++k) {
-        A.g1f_a[k] = (float)A.g1_om_a[k];
-        A.g1f_1[k] = (float)A.g1_om_1[k];
+        gam *= A.g1_om_1[k];
+        A.g1f_gam[k] = (float)gam;
+        A.g1f_bet[k] = (float)(A.g1_om_a[k] / gam);
     }
     split(A.om_a, A.oa_hi, A.oa_lo);
     split(A.om_1, A.o1_hi, A.o1_lo);
@@ -255,6 +259,57 @@ template <int CPT> __device__ __forceinline__ void st_row(float* p, const float 
     }
 }
 
+// the float-float outer update of CPT neighbouring pixels (hi plane at gi, lo plane at gi + plane): the step
+// om_a r + om_1 (x - x_prev) in FP32 with the coefficients carried as hi + lo, added to x with an exact two-sum
+struct FfCoef { float oah, oal, o1h, o1l; };
+__device__ __forceinline__ FfCoef ff_coefficients(const OuterStepArgs& A, int img) {
+    FfCoef k = {A.oa_hi, A.oa_lo, A.o1_hi, A.o1_lo};
+    if (A.om_img) {  // per-image coefficients (slot-level serving): split here
+        const double oa = A.om_img[2 * img], o1 = A.om_img[2 * img + 1];
+        k.oah = (float)oa;
+        k.oal = (float)(oa - (double)k.oah);
+        k.o1h = (float)o1;
+        k.o1l = (float)(o1 - (double)k.o1h);
+    }
+    return k;
+}
+template <int CPT>
+__device__ __forceinline__ void ff_update_row(const OuterStepArgs& A, const FfCoef& k, const float (&rv)[CPT], size_t gi,
+                                              size_t plane) {
+    float hv[CPT], lv[CPT];
+    if (!A.xf) {
+#pragma unroll
+        for (int q = 0; q < CPT; ++q) {
+            const float h = A.a0_hi * rv[q];
+            const float l = fmaf(A.a0_hi, rv[q], -h) + A.a0_lo * rv[q];
+            hv[q] = h + l;
+            lv[q] = l - (hv[q] - h);
+        }
+    } else {
+        float xh[CPT], xl[CPT], ph[CPT], pl[CPT];
+        ld_row<CPT>(A.xf + gi, xh);
+        ld_row<CPT>(A.xf + gi + plane, xl);
+        if (A.xpf) {
+            ld_row<CPT>(A.xpf + gi, ph);
+            ld_row<CPT>(A.xpf + gi + plane, pl);
+        } else {
+#pragma unroll
+            for (int q = 0; q < CPT; ++q) ph[q] = pl[q] = 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < CPT; ++q) {
+            const float d = (xh[q] - ph[q]) + (xl[q] - pl[q]);
+            const float del = fmaf(k.oah, rv[q], fmaf(k.o1h, d, fmaf(k.oal, rv[q], k.o1l * d)));
+            const float sh = xh[q] + del, bb = sh - xh[q];
+            const float lo = ((xh[q] - (sh - bb)) + (del - bb)) + xl[q];
+            hv[q] = sh + lo;
+            lv[q] = lo - (hv[q] - sh);
+        }
+    }
+    st_row<CPT>(A.xnf + gi, hv);
+    st_row<CPT>(A.xnf + gi + plane, lv);
+}
+
 // ------------------------------------------------------------------ register-resident form (FP32 stencil and partial
 // images, 64 <= N <= 512). Warp w of a CTA owns a strip of R = 1024 / N rows spanning the whole row: lane l holds
 // columns l CPT .. l CPT + CPT - 1 (CPT = N / 32) of those rows, so its residual, both stencil iterates and its outer
@@ -333,23 +388,30 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
         }
     }
 
-    float cA[R][CPT], cB[R][CPT];
-    bool in_b = false;  // the result of the preconditioner is in cB (else in cA)
+    float c[R][CPT];
     if (A.precond == 1) {
         const float* up = rank > 0 ? cluster.map_shared_rank(bnd, rank - 1) : nullptr;
         const float* dn = rank < CL - 1 ? cluster.map_shared_rank(bnd, rank + 1) : nullptr;
-        // the strip's first and last rows of iterate v into copy b, then arrive at the cluster barrier
-        auto publish = [&](const float (&v)[R][CPT], int b) {
+        // the strip's first and last rows of the iterate into copy b, then arrive at the cluster barrier
+        auto publish = [&](int b) {
             float* f = bnd + b * HC + (w * 2) * N + j0;
 #pragma unroll
             for (int q = 0; q < CPT / 2; ++q) {
-                *reinterpret_cast<float2*>(f + 2 * q) = make_float2(v[0][2 * q], v[0][2 * q + 1]);
-                *reinterpret_cast<float2*>(f + N + 2 * q) = make_float2(v[R - 1][2 * q], v[R - 1][2 * q + 1]);
+                *reinterpret_cast<float2*>(f + 2 * q) = make_float2(c[0][2 * q], c[0][2 * q + 1]);
+                *reinterpret_cast<float2*>(f + N + 2 * q) = make_float2(c[R - 1][2 * q], c[R - 1][2 * q + 1]);
             }
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         };
-        // one Chebyshev step p <- c + om_a (s - G1 c) + om_1 (c - p); the boundary of c is in copy b
-        auto step = [&](const float (&c)[R][CPT], float (&p)[R][CPT], float om_a, float om_1, int b) {
+        float e[R][CPT];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int q = 0; q < CPT; ++q) c[r][q] = e[r][q] = A.g1f_a0 * s[r][q];
+        publish(0);
+        // Chebyshev steps e += bet (s - G1 c), c += gam e; the boundary of c is in copy (k - 1) & 1
+        for (int k = 1; k < A.g1_deg; ++k) {
+            const float bet = A.g1f_bet[k - 1], gam = A.g1f_gam[k - 1];
+            const int b = (k - 1) & 1;
 #pragma unroll
             for (int m = 0; m < R / 2; ++m) {
                 const int r0 = 2 * m, r1 = r0 + 1;
@@ -365,27 +427,29 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
                     const float t = 2.f * ((c00 + c01) + (c10 + c11));
                     float g00 = fmaf(6.f, c00, t), g01 = fmaf(6.f, c01, t);
                     float g10 = fmaf(6.f, c10, t), g11 = fmaf(6.f, c11, t);
-                    if (r0 > 0) {  // the row above the pair, pair column (the strip's first row: deferred)
-                        g00 += c[r0 - 1][bb];
-                        g01 += c[r0 - 1][a];
-                    }
-                    if (r1 < R - 1) {  // the row below
-                        g10 += c[r1 + 1][bb];
-                        g11 += c[r1 + 1][a];
-                    }
                     g00 += v > 0 ? c[r1][a - 1] : L1;  // beside the cell, on the other row of the pair
                     g10 += v > 0 ? c[r0][a - 1] : L0;
                     g01 += v < CPT / 2 - 1 ? c[r1][bb + 1] : R1;
                     g11 += v < CPT / 2 - 1 ? c[r0][bb + 1] : R0;
-                    p[r0][a] = (c00 + om_a * (s[r0][a] - g00)) + om_1 * (c00 - p[r0][a]);
-                    p[r0][bb] = (c01 + om_a * (s[r0][bb] - g01)) + om_1 * (c01 - p[r0][bb]);
-                    p[r1][a] = (c10 + om_a * (s[r1][a] - g10)) + om_1 * (c10 - p[r1][a]);
-                    p[r1][bb] = (c11 + om_a * (s[r1][bb] - g11)) + om_1 * (c11 - p[r1][bb]);
+                    e[r0][a] = fmaf(bet, s[r0][a] - g00, e[r0][a]);
+                    e[r0][bb] = fmaf(bet, s[r0][bb] - g01, e[r0][bb]);
+                    e[r1][a] = fmaf(bet, s[r1][a] - g10, e[r1][a]);
+                    e[r1][bb] = fmaf(bet, s[r1][bb] - g11, e[r1][bb]);
+                    // the row above or below the pair, pair column, always last (on the strip's first and last row:
+                    // deferred), so that a pixel's value does not depend on where the strips lie
+                    if (r0 > 0) {
+                        e[r0][a] = fmaf(-bet, c[r0 - 1][bb], e[r0][a]);
+                        e[r0][bb] = fmaf(-bet, c[r0 - 1][a], e[r0][bb]);
+                    }
+                    if (r1 < R - 1) {
+                        e[r1][a] = fmaf(-bet, c[r1 + 1][bb], e[r1][a]);
+                        e[r1][bb] = fmaf(-bet, c[r1 + 1][a], e[r1][bb]);
+                    }
                 }
             }
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             // the rows above and below the strip (zero beyond the image): G_1 c gains c(above, j^1) on the first
-            // row and c(below, j^1) on the last, so p loses om_a times those
+            // row and c(below, j^1) on the last, so e loses bet times those
             const float* fa = w > 0 ? bnd + b * HC + ((w - 1) * 2 + 1) * N
                                     : (up ? up + b * HC + ((W - 1) * 2 + 1) * N : nullptr);
             const float* fb = w < W - 1 ? bnd + b * HC + ((w + 1) * 2) * N : (dn ? dn + b * HC : nullptr);
@@ -393,32 +457,16 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
             for (int q = 0; q < CPT / 2; ++q) {
                 const float2 ta = fa ? *reinterpret_cast<const float2*>(fa + j0 + 2 * q) : make_float2(0.f, 0.f);
                 const float2 tb = fb ? *reinterpret_cast<const float2*>(fb + j0 + 2 * q) : make_float2(0.f, 0.f);
-                p[0][2 * q] = fmaf(-om_a, ta.y, p[0][2 * q]);
-                p[0][2 * q + 1] = fmaf(-om_a, ta.x, p[0][2 * q + 1]);
-                p[R - 1][2 * q] = fmaf(-om_a, tb.y, p[R - 1][2 * q]);
-                p[R - 1][2 * q + 1] = fmaf(-om_a, tb.x, p[R - 1][2 * q + 1]);
+                e[0][2 * q] = fmaf(-bet, ta.y, e[0][2 * q]);
+                e[0][2 * q + 1] = fmaf(-bet, ta.x, e[0][2 * q + 1]);
+                e[R - 1][2 * q] = fmaf(-bet, tb.y, e[R - 1][2 * q]);
+                e[R - 1][2 * q + 1] = fmaf(-bet, tb.x, e[R - 1][2 * q + 1]);
             }
-        };
-        const float a0 = A.g1f_a0;
 #pragma unroll
-        for (int r = 0; r < R; ++r)
+            for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int q = 0; q < CPT; ++q) {
-                cA[r][q] = a0 * s[r][q];
-                cB[r][q] = 0.f;
-            }
-        publish(cA, 0);
-        int k = 1;
-        for (; k + 1 < A.g1_deg; k += 2) {
-            step(cA, cB, A.g1f_a[k - 1], A.g1f_1[k - 1], (k - 1) & 1);
-            publish(cB, k & 1);
-            step(cB, cA, A.g1f_a[k], A.g1f_1[k], k & 1);
-            publish(cA, (k + 1) & 1);
-        }
-        if (k < A.g1_deg) {
-            step(cA, cB, A.g1f_a[k - 1], A.g1f_1[k - 1], (k - 1) & 1);
-            publish(cB, k & 1);
-            in_b = true;
+                for (int q = 0; q < CPT; ++q) c[r][q] = fmaf(gam, e[r][q], c[r][q]);
+            publish(k & 1);
         }
         // the last arrival's wait: no CTA leaves while a neighbour may still read its boundary rows
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -431,15 +479,15 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
                 const float mu = ((s[r0][a] + s[r0][a + 1]) + (s[r0 + 1][a] + s[r0 + 1][a + 1])) * 0.25f;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int r = r0 + (q >> 1), c = a + (q & 1);
-                    cA[r][c] = (s[r][c] - mu) * 0.25f + mu / 12.f;
+                    const int r = r0 + (q >> 1), cc = a + (q & 1);
+                    c[r][cc] = (s[r][cc] - mu) * 0.25f + mu / 12.f;
                 }
             }
     } else {
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int q = 0; q < CPT; ++q) cA[r][q] = s[r][q];
+            for (int q = 0; q < CPT; ++q) c[r][q] = s[r][q];
     }
 
     // outer update: in FP64 (FP64 state), or in float-float on the FP32 pipe (float-float state): the step
@@ -447,53 +495,11 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
     // two-sum, so the state keeps about 48 bits while no FP64 instruction runs (the FP64 pipe of this GPU is a small
     // fraction of its FP32 pipe)
     if constexpr (FF) {
-        float oah = A.oa_hi, oal = A.oa_lo, o1h = A.o1_hi, o1l = A.o1_lo;
-        if (A.om_img) {  // per-image coefficients (slot-level serving): split here
-            const double oa = A.om_img[2 * img], o1 = A.om_img[2 * img + 1];
-            oah = (float)oa;
-            oal = (float)(oa - (double)oah);
-            o1h = (float)o1;
-            o1l = (float)(o1 - (double)o1h);
-        }
-        const float a0h = A.a0_hi, a0l = A.a0_lo;
+        const FfCoef k = ff_coefficients(A, img);
         const size_t fo = gbase + (size_t)img * N * N;  // hi plane of this thread's first row; lo plane N^2 further
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const size_t gi = fo + (size_t)r * N;
-            float rv[CPT], hv[CPT], lv[CPT];
-#pragma unroll
-            for (int q = 0; q < CPT; ++q) rv[q] = in_b ? cB[r][q] : cA[r][q];
-            if (!A.xf) {
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) {
-                    const float h = a0h * rv[q];
-                    const float l = fmaf(a0h, rv[q], -h) + a0l * rv[q];
-                    hv[q] = h + l;
-                    lv[q] = l - (hv[q] - h);
-                }
-            } else {
-                float xh[CPT], xl[CPT], ph[CPT], pl[CPT];
-                ld_row<CPT>(A.xf + gi, xh);
-                ld_row<CPT>(A.xf + gi + (size_t)N * N, xl);
-                if (A.xpf) {
-                    ld_row<CPT>(A.xpf + gi, ph);
-                    ld_row<CPT>(A.xpf + gi + (size_t)N * N, pl);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) ph[q] = pl[q] = 0.f;
-                }
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) {
-                    const float d = (xh[q] - ph[q]) + (xl[q] - pl[q]);
-                    const float del = fmaf(oah, rv[q], fmaf(o1h, d, fmaf(oal, rv[q], o1l * d)));
-                    const float sh = xh[q] + del, bb = sh - xh[q];
-                    const float lo = ((xh[q] - (sh - bb)) + (del - bb)) + xl[q];
-                    hv[q] = sh + lo;
-                    lv[q] = lo - (hv[q] - sh);
-                }
-            }
-            st_row<CPT>(A.xnf + gi, hv);
-            st_row<CPT>(A.xnf + gi + (size_t)N * N, lv);
+            ff_update_row<CPT>(A, k, c[r], fo + (size_t)r * N, (size_t)N * N);
         }
         return;
     }
@@ -504,8 +510,8 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
         const size_t gi = gbase + (size_t)r * N;
 #pragma unroll
         for (int q = 0; q < CPT / 2; ++q) {
-            const double r0 = (double)(in_b ? cB[r][2 * q] : cA[r][2 * q]);
-            const double r1 = (double)(in_b ? cB[r][2 * q + 1] : cA[r][2 * q + 1]);
+            const double r0 = (double)c[r][2 * q];
+            const double r1 = (double)c[r][2 * q + 1];
             double2 out;
             if (!A.x) {
                 out = make_double2(A.a0 * r0, A.a0 * r1);
@@ -517,6 +523,129 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
             *reinterpret_cast<double2*>(A.xn + gi + 2 * q) = out;
         }
     }
+}
+
+// ------------------------------------------------------------------ tiled form (float-float state, G_1 preconditioner of
+// degree <= 16): no cluster. A CTA takes a tile of the image with a halo of 16 pixels on every side through all steps and
+// keeps the interior: the stencil reaches one pixel per step, so the halo's error never arrives there, and the only
+// synchronisation is one CTA barrier per step. LPR lanes hold a row of the region (4 columns each), a strip of R rows per
+// lane group; the strips' first and last rows meet in shared memory (two copies alternate), column neighbours by shuffle.
+// Pixels outside the image have bet = 0, so they stay zero, and strips that no later step needs are skipped. Rows and
+// columns of the halo are computed more than once, which pays where the clusters leave the SMs waiting (small batches: the
+// cluster barrier per step) or fill them badly (N = 512: strips of two rows, one CTA per SM).
+constexpr int OT_HALO = 16;
+template <int LPR, int R, int W> struct OtCfg {
+    static constexpr int CPT = 4;
+    static constexpr int COLS = LPR * CPT;             // region
+    static constexpr int STRIPS = W * (32 / LPR);
+    static constexpr int ROWS = STRIPS * R;
+    static constexpr int OUTC = COLS - 2 * OT_HALO, OUTR = ROWS - 2 * OT_HALO;
+    static_assert(OT_HALO % R == 0 && OT_HALO % CPT == 0 && OUTC > 0 && OUTR > 0, "strips and lanes lie inside or outside");
+};
+
+template <int LPR, int R, int W, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) outer_step_tile_kernel(const OuterStepArgs A, const int n, const int tx) {
+    using T = OtCfg<LPR, R, W>;
+    constexpr int CPT = T::CPT, COLS = T::COLS, STRIPS = T::STRIPS;
+    __shared__ __align__(16) float bnd[2][STRIPS][2][COLS];
+    const int N = 1 << n;
+    const int img = blockIdx.y, ty = blockIdx.x / tx;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lc = lane % LPR, strip = warp * (32 / LPR) + lane / LPR;
+    const int col = (int)(blockIdx.x - ty * tx) * T::OUTC - OT_HALO + lc * CPT;
+    const int row = ty * T::OUTR - OT_HALO + strip * R;
+    const bool inside = col >= 0 && col < N && row >= 0 && row < N;  // strips and lanes never straddle the border
+    const size_t gi = (size_t)img * N * N + (size_t)row * N + col;
+    constexpr unsigned FULL = 0xffffffffu;
+
+    float s[R][CPT], c[R][CPT], e[R][CPT];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int q = 0; q < CPT; ++q) s[r][q] = 0.f;
+        if (inside) {
+            ld_row<CPT>(A.yf + gi + (size_t)r * N, s[r]);
+            if (A.p0) {
+                float a[CPT], b[CPT], d[CPT];
+                ld_row<CPT>(reinterpret_cast<const float*>(A.p0) + gi + (size_t)r * N, a);
+                ld_row<CPT>(reinterpret_cast<const float*>(A.p1) + gi + (size_t)r * N, b);
+                ld_row<CPT>(reinterpret_cast<const float*>(A.p2) + gi + (size_t)r * N, d);
+#pragma unroll
+                for (int q = 0; q < CPT; ++q) s[r][q] -= (a[q] + b[q]) + d[q];
+            }
+        }
+    }
+    const float a0 = A.g1f_a0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < CPT; ++q) c[r][q] = e[r][q] = a0 * s[r][q];
+
+    for (int k = 1; k < A.g1_deg; ++k) {
+        // rows of the interior plus what the later steps reach (and a cell's other row)
+        const int margin = A.g1_deg - k;
+        const int top = OT_HALO - margin, bot = OT_HALO + T::OUTR - 1 + margin;
+        const bool need_src = (strip + 1) * R > top - R && strip * R <= bot + R;  // read by a computing strip
+        if (need_src) {
+            float* f = &bnd[k & 1][strip][0][lc * CPT];
+            *reinterpret_cast<float4*>(f) = make_float4(c[0][0], c[0][1], c[0][2], c[0][3]);
+            *reinterpret_cast<float4*>(f + COLS) = make_float4(c[R - 1][0], c[R - 1][1], c[R - 1][2], c[R - 1][3]);
+        }
+        __syncthreads();
+        const int wtop = warp * (32 / LPR) * R, wbot = wtop + (32 / LPR) * R - 1;  // the warp's rows
+        if (wbot < top || wtop > bot) continue;
+        const float bet = inside ? A.g1f_bet[k - 1] : 0.f, gam = A.g1f_gam[k - 1];
+        const float4 fa = strip > 0 ? *reinterpret_cast<const float4*>(&bnd[k & 1][strip > 0 ? strip - 1 : 0][1][lc * CPT])
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 fb = strip < STRIPS - 1
+                              ? *reinterpret_cast<const float4*>(&bnd[k & 1][strip < STRIPS - 1 ? strip + 1 : strip][0][lc * CPT])
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float above[CPT] = {fa.x, fa.y, fa.z, fa.w}, below[CPT] = {fb.x, fb.y, fb.z, fb.w};
+#pragma unroll
+        for (int m = 0; m < R / 2; ++m) {
+            const int r0 = 2 * m, r1 = r0 + 1;
+            // the columns beside the lane's first and last column, on both rows of the pair (a region's edge takes its own
+            // value: wrong, and outside what is kept)
+            const float L0 = __shfl_up_sync(FULL, c[r0][CPT - 1], 1, LPR), L1 = __shfl_up_sync(FULL, c[r1][CPT - 1], 1, LPR);
+            const float R0 = __shfl_down_sync(FULL, c[r0][0], 1, LPR), R1 = __shfl_down_sync(FULL, c[r1][0], 1, LPR);
+#pragma unroll
+            for (int v = 0; v < CPT / 2; ++v) {
+                const int a = 2 * v, b = a + 1;
+                const float t = 2.f * ((c[r0][a] + c[r0][b]) + (c[r1][a] + c[r1][b]));
+                const float ua = r0 > 0 ? c[r0 > 0 ? r0 - 1 : 0][b] : above[b], ub = r0 > 0 ? c[r0 > 0 ? r0 - 1 : 0][a] : above[a];
+                const float da = r1 < R - 1 ? c[r1 < R - 1 ? r1 + 1 : r1][b] : below[b];
+                const float db = r1 < R - 1 ? c[r1 < R - 1 ? r1 + 1 : r1][a] : below[a];
+                // the order of outer_step_reg_kernel, for identical results
+                const float g00 = fmaf(6.f, c[r0][a], t) + (v > 0 ? c[r1][v > 0 ? a - 1 : 0] : L1);
+                const float g01 = fmaf(6.f, c[r0][b], t) + (v < CPT / 2 - 1 ? c[r1][v < CPT / 2 - 1 ? b + 1 : b] : R1);
+                const float g10 = fmaf(6.f, c[r1][a], t) + (v > 0 ? c[r0][v > 0 ? a - 1 : 0] : L0);
+                const float g11 = fmaf(6.f, c[r1][b], t) + (v < CPT / 2 - 1 ? c[r0][v < CPT / 2 - 1 ? b + 1 : b] : R0);
+                e[r0][a] = fmaf(-bet, ua, fmaf(bet, s[r0][a] - g00, e[r0][a]));
+                e[r0][b] = fmaf(-bet, ub, fmaf(bet, s[r0][b] - g01, e[r0][b]));
+                e[r1][a] = fmaf(-bet, da, fmaf(bet, s[r1][a] - g10, e[r1][a]));
+                e[r1][b] = fmaf(-bet, db, fmaf(bet, s[r1][b] - g11, e[r1][b]));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int q = 0; q < CPT; ++q) c[r][q] = fmaf(gam, e[r][q], c[r][q]);
+    }
+    const int ir = strip * R, ic = lc * CPT;
+    if (inside && ir >= OT_HALO && ir < OT_HALO + T::OUTR && ic >= OT_HALO && ic < OT_HALO + T::OUTC) {
+        const FfCoef k = ff_coefficients(A, img);
+        const size_t fo = gi + (size_t)img * N * N;
+#pragma unroll
+        for (int r = 0; r < R; ++r) ff_update_row<CPT>(A, k, c[r], fo + (size_t)r * N, (size_t)N * N);
+    }
+}
+
+template <int LPR, int R, int W, int MINB>
+static int launch_os_tile(const OuterStepArgs& A, int n, int nimg, cudaStream_t st) {
+    using T = OtCfg<LPR, R, W>;
+    const int N = 1 << n, tx = (N + T::OUTC - 1) / T::OUTC, ty = (N + T::OUTR - 1) / T::OUTR;
+    outer_step_tile_kernel<LPR, R, W, MINB><<<dim3(tx * ty, nimg), 32 * W, 0, st>>>(A, n, tx);
+    return launch_status("outer_step_tile_kernel");
 }
 
 template <int n, int BAND, bool FF>
@@ -703,6 +832,16 @@ int outer_step_ff(int n, int nimg, const float* y, const float* p0, const float*
         }
     }
     fill_f32_coefficients(A);
+    // the tiled form where its CTAs fill the SMs at most a few times (us on 152 SMs, N, batch: tiled / clusters): small
+    // tiles up to two CTAs per SM (256, 1: 6.7 / 14.3; 256, 4: 9.2 / 14.4; 128, 8: 6.8 / 11.8; 64, 64: 9.1 / 13.1), large
+    // ones up to one per SM at N <= 128 (128, 37: 12.8 / 14.6; 128, 64: 23.7 / 14.6), two at 256 (16: 23.9 / 27.2; 32:
+    // 41.0 / 31.8) and always at 512 (6: 24.4 / 65.7; 16: 89.7 / 197.6)
+    if (band == 0 && precond == 1 && g1_deg <= OT_HALO && nimg <= 65535) {
+        const long long N = 1 << n, sms = device_sm_count();
+        const long long small = nimg * (N / 32) * (N / 32), large = nimg * ((N + 95) / 96) * ((N + 63) / 64);
+        if (small <= 2 * sms) return launch_os_tile<16, 4, 8, 2>(A, n, nimg, st);
+        if (n == 9 || large <= (n == 8 ? 2 : 1) * sms) return launch_os_tile<32, 4, 24, 1>(A, n, nimg, st);
+    }
     return dispatch_os_reg<true>(n, A, nimg, band, st);
 }
 
