@@ -2,10 +2,9 @@
 // fastops.py:209-220; Tq / TqT / iota, fastspec.py:142-174).
 //
 // One CTA handles a block of C strip columns of one image. The length-L (L = 2N) DFT of each column runs as an in-place
-// decimation-in-time transform on bit-reversed input: each thread holds E = 8 or 16 points of its column (16 where that
-// saves a pass: L = 128, 256, 1024 and up), a pass multiplies them by their twiddles (one table value per point, none in
-// the first pass) and runs a radix-E butterfly with constant rotations, and the passes exchange through a padded
-// shared-memory tile.
+// decimation-in-time transform on bit-reversed input: each thread holds E = 4 to 32 points of its column (see FftCfg), a
+// pass multiplies them by their twiddles (one table value per point, none in the first pass) and runs a radix-E butterfly
+// with constant rotations, and the passes exchange through a padded shared-memory tile.
 //
 // pack:   strips s_qa + i s_qb of each quadrant pair come from the image (Tq of the zero-padded image) or the sinogram
 //         (iota), are transformed forward and written as rows of Y. Values that lie along the columns (two of the four
@@ -24,11 +23,13 @@
 
 namespace adrt {
 
-template <typename real, int l> struct FftCfg {
+template <typename real, int l, bool SM> struct FftCfg {
     static constexpr int L = 1 << l;
-    // log2 of points per thread: in FP32 4 where that takes a pass (an exchange) less than 3; FP64 is bound by its pipe
-    // (a warp's instruction takes 16 cycles), so there more threads with fewer points each
-    static constexpr int e = l < 3 ? l : (sizeof(real) == 4 && (l + 3) / 4 < (l + 2) / 3 ? 4 : 3);
+    // log2 of points per thread: in FP32 as many as take a pass (an exchange, a twiddle multiply) less: 32 points at
+    // L = 512 and 1024 (two passes), 16 at 128, 256 and above. FP64 is bound by its pipe (half a lane per clock and SM
+    // quarter): 8. Small launches (SM) are bound by the length of a thread's chain instead: fewer points, more threads
+    static constexpr int e = l < 3 ? l : sizeof(real) == 8 ? (SM ? 2 : 3) : SM ? 3 : l == 9 || l == 10 ? 5
+                             : (l + 3) / 4 < (l + 2) / 3 ? 4 : 3;
     static constexpr int E = 1 << e;
     static constexpr int TPC = L / E;           // threads per column
     static constexpr int NPASS = (l + e - 1) / e;
@@ -59,26 +60,29 @@ template <int l> __host__ __device__ constexpr int fft_fit(int c, int elem_bytes
 template <int l> __host__ __device__ constexpr int fft_cols(int Cmax, int elem_bytes) {
     return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / imax(1, (1 << l) / 8)), (1 << l) / 2)), elem_bytes);
 }
-template <typename real, int l> __host__ __device__ constexpr int fft_cols_auto(int Cmax, int elem_bytes) {
-    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / FftCfg<real, l>::TPC), (1 << l) / 2)), elem_bytes);
+template <typename real, int l, bool SM> __host__ __device__ constexpr int fft_cols_auto(int Cmax, int elem_bytes) {
+    return fft_fit<l>(imax(1, imin(imin(Cmax, 1024 / FftCfg<real, l, SM>::TPC), (1 << l) / 2)), elem_bytes);
 }
 
-// cos and sin of 2 pi k / 16, k < 8
-template <typename real> __device__ __forceinline__ cplx<real> root16(int k) {
-    constexpr double c1 = 0.92387953251128675613, c2 = 0.70710678118654752440, c3 = 0.38268343236508977173;
-    const double re[8] = {1, c1, c2, c3, 0, -c3, -c2, -c1}, im[8] = {0, c3, c2, c1, 1, c1, c2, c3};
+// cos and sin of 2 pi k / 32, k < 16
+template <typename real> __device__ __forceinline__ cplx<real> root32(int k) {
+    constexpr double c1 = 0.98078528040323044913, c2 = 0.92387953251128675613, c3 = 0.83146961230254523708;
+    constexpr double c4 = 0.70710678118654752440, c5 = 0.55557023301960222474, c6 = 0.38268343236508977173;
+    constexpr double c7 = 0.19509032201612826785;
+    const double re[16] = {1, c1, c2, c3, c4, c5, c6, c7, 0, -c7, -c6, -c5, -c4, -c3, -c2, -c1};
+    const double im[16] = {0, c7, c6, c5, c4, c3, c2, c1, 1, c1, c2, c3, c4, c5, c6, c7};
     return mk<real>((real)re[k], (real)im[k]);
 }
-// x times exp(-+ 2 pi i k / 2^m) (INV: +), k < 2^(m-1), m <= 4, k and m constants: trivial rotations cost no multiply
+// x times exp(-+ 2 pi i k / 2^m) (INV: +), k < 2^(m-1), m <= 5, k and m constants: trivial rotations cost no multiply
 template <typename real, bool INV> __device__ __forceinline__ cplx<real> rotate(cplx<real> x, int k, int m) {
-    const int k16 = k << (4 - m);
-    if (k16 == 0) return x;
-    if (k16 == 4) return INV ? mk<real>(-x.y, x.x) : mk<real>(x.y, -x.x);
-    cplx<real> w = root16<real>(k16);
-    if (k16 == 2 || k16 == 6) {  // +-sqrt(1/2) (1 +- i)
-        const real h = root16<real>(2).x;
+    const int k32 = k << (5 - m);
+    if (k32 == 0) return x;
+    if (k32 == 8) return INV ? mk<real>(-x.y, x.x) : mk<real>(x.y, -x.x);
+    cplx<real> w = root32<real>(k32);
+    if (k32 == 4 || k32 == 12) {  // +-sqrt(1/2) (1 +- i)
+        const real h = root32<real>(4).x;
         const real a = h * (x.x - x.y), b = h * (x.x + x.y);
-        if (k16 == 2) return INV ? mk<real>(a, b) : mk<real>(b, -a);
+        if (k32 == 4) return INV ? mk<real>(a, b) : mk<real>(b, -a);
         return INV ? mk<real>(-b, a) : mk<real>(-a, -b);
     }
     if (!INV) w.y = -w.y;
@@ -87,10 +91,10 @@ template <typename real, bool INV> __device__ __forceinline__ cplx<real> rotate(
 
 // all passes of the in-place DIT transform on the registers x[] of (column c, column-thread t); the caller loads x[j]
 // with input brev(pos(0, t, j)) and finds output pos(NPASS - 1, t, j) in x[j]
-template <typename real, int l, bool INV>
-__device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<real, l>::E], const cplx<real>* __restrict__ roots,
+template <typename real, int l, bool INV, bool SM>
+__device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<real, l, SM>::E], const cplx<real>* __restrict__ roots,
                                            cplx<real>* tile, int CP, int c, int t) {
-    using F = FftCfg<real, l>;
+    using F = FftCfg<real, l, SM>;
     using C = cplx<real>;
 #pragma unroll
     for (int q = 0; q < F::NPASS; ++q) {
@@ -128,19 +132,19 @@ __device__ __forceinline__ void dit_passes(cplx<real> (&x)[FftCfg<real, l>::E], 
 }
 
 // threads of a CTA and the CTAs per SM the register budget is sized for
-template <typename real, int l, int CB> struct FftLaunch {
-    static constexpr int threads = CB * FftCfg<real, l>::TPC;
-    // threads per SM: 64 registers each for 8 points in FP32, twice that for 16 points or FP64
-    static constexpr int resident = sizeof(real) == 4 && FftCfg<real, l>::e < 4 ? 1024 : 512;
-    static constexpr int pack_min = imin(16, imax(1, (FftCfg<real, l>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads));
+template <typename real, int l, int CB, bool SM> struct FftLaunch {
+    static constexpr int threads = CB * FftCfg<real, l, SM>::TPC;
+    // threads per SM: 64 registers each for 8 points in FP32, twice that for more points or FP64
+    static constexpr int resident = sizeof(real) == 4 && FftCfg<real, l, SM>::e < 4 ? 1024 : 512;
+    static constexpr int pack_min = imin(16, imax(1, (FftCfg<real, l, SM>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads));
     static constexpr int unpack_min = imin(16, imax(1, resident / threads));
 };
 
-template <typename real, int l, int CB, typename SRC>
-__global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<real, l, CB>::pack_min)
+template <typename real, int l, int CB, bool SM, typename SRC>
+__global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch<real, l, CB, SM>::pack_min)
     pack_fft_kernel(int nimg, int src_kind, const SRC* __restrict__ src, long long src_stride, cplx<real>* __restrict__ Y,
                     const cplx<real>* __restrict__ roots_g) {
-    using F = FftCfg<real, l>;
+    using F = FftCfg<real, l, SM>;
     using C = cplx<real>;
     constexpr int L = F::L, N = L / 2;
     constexpr int CP = fft_pad(CB);
@@ -220,17 +224,17 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<rea
         }
         __syncthreads();  // roots
     }
-    dit_passes<real, l, false>(x, roots, tile, CP, c, t);
+    dit_passes<real, l, false, SM>(x, roots, tile, CP, c, t);
     C* out = Y + ((size_t)img * 2 * L + (size_t)pair * L) * N + c0 + c;
 #pragma unroll
     for (int j = 0; j < F::E; ++j) out[(size_t)F::pos(F::NPASS - 1, t, j) * N] = x[j];
 }
 
-template <typename real, int l, int CB>
-__global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<real, l, CB>::unpack_min)
+template <typename real, int l, int CB, bool SM>
+__global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch<real, l, CB, SM>::unpack_min)
     ifft_unpack_kernel(int nimg, const cplx<real>* __restrict__ Z, real* __restrict__ colpart, real* __restrict__ row0,
                        real* __restrict__ row3, const cplx<real>* __restrict__ roots_g) {
-    using F = FftCfg<real, l>;
+    using F = FftCfg<real, l, SM>;
     using C = cplx<real>;
     constexpr int L = F::L, N = L / 2, E = F::E;
     constexpr int CP = fft_pad(CB), RP = N + 1;  // row pitch of the transposed strips
@@ -256,7 +260,7 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB>::threads, FftLaunch<rea
 #pragma unroll
         for (int j = 0; j < E; ++j) x[j] = in[(size_t)(brev(j, F::e) * (L / E) + rt) * N];
         if (pair == 0) __syncthreads();  // roots
-        dit_passes<real, l, true>(x, roots, tile, CP, c, tt);
+        dit_passes<real, l, true, SM>(x, roots, tile, CP, c, tt);
         real* rows = rowt;
         if (pair == 1) {
             __syncthreads();  // the exchange tile is free
@@ -296,88 +300,111 @@ template <typename real, int l, int CB> static size_t unpack_smem() {
            (size_t)CB * ((1 << (l - 1)) + 1) * sizeof(real);
 }
 
-// columns per CTA: cols = 0 picks as many as fit, up to 16 FP32 / 8 FP64; the autotuner's choices are the widths of 8
-// points per thread and a quarter of them (narrower CTAs, more of them per SM)
-template <typename real, int l> constexpr int cols_auto() { return fft_cols_auto<real, l>(FftMax<real>::C, sizeof(cplx<real>)); }
-// the width of launches that would leave SMs idle at the others (small batches): an eighth of the widest, whole warps
-template <typename real, int l> constexpr int cols_small() {
-    return imin(cols_auto<real, l>(), imax(imax(1, cols_auto<real, l>() / 8), 32 / FftCfg<real, l>::TPC));
+// Small launches: at most two images' worth of columns at N = 256. Which form runs depends on the size and batch alone, not
+// on the columns per CTA, so every column is transformed by the same arithmetic whatever the CTA shape. Measured (pack /
+// unpack us, small against large form): FP32 N = 256, one image 3.5 / 4.6 against 4.6 / 5.9, four 4.9 / 7.1 against 4.7 /
+// 6.0; FP64 N = 64, one image 5.2 / 8.4 against 8.2 / 13.6, N = 256, eight 136 / 137 against 125 / 127.
+template <typename real, int l> constexpr bool fft_has_small() { return sizeof(real) == 8 ? l >= 4 : l == 9; }
+static bool fft_small(int l, int nimg) { return ((long long)nimg << (l - 1)) <= 512; }
+
+// columns per CTA: the autotuner's choices are the widths of 8 points per thread (as many as fit, up to 16 FP32 / 8 FP64)
+// and a quarter of them; cols = 0 picks as many as fit the form's threads, or, where those CTAs would not give every SM one,
+// fewer: FP32 small form and FP64 a quarter, L = 1024 half. (Elsewhere narrower CTAs lose more in half-used sectors and
+// table loads than idle SMs cost: N = 256, four images, pack 4.7 us with 16 columns, 7.2 with 4.)
+template <typename real, int l, bool SM> constexpr int cols_auto() {
+    return fft_cols_auto<real, l, SM>(FftMax<real>::C, sizeof(cplx<real>));
+}
+template <typename real, int l, bool SM> constexpr int cols_few() {
+    return sizeof(real) == 8 || SM ? imax(1, cols_auto<real, l, SM>() / 4)
+                                   : (l == 10 ? cols_auto<real, l, SM>() / 2 : cols_auto<real, l, SM>());
 }
 template <typename real, int l> constexpr int cols_wide() { return fft_cols<l>(FftMax<real>::C, sizeof(cplx<real>)); }
 template <typename real, int l> constexpr int cols_narrow() { return imax(1, cols_wide<real, l>() / 4); }
 
-template <typename real, int l, int CB, typename SRC>
+template <typename real, int l, int CB, bool SM, typename SRC>
 static int launch_pack_cb(int nimg, int src_kind, const void* src, long long src_stride, void* Y, const void* roots,
                           cudaStream_t st) {
     constexpr int N = 1 << (l - 1);
     const size_t smem = pack_smem<real, l, CB>();
-    auto kern = pack_fft_kernel<real, l, CB, SRC>;
+    auto kern = pack_fft_kernel<real, l, CB, SM, SRC>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, 2, nimg);
-    kern<<<grid, CB * FftCfg<real, l>::TPC, smem, st>>>(nimg, src_kind, reinterpret_cast<const SRC*>(src),
+    kern<<<grid, CB * FftCfg<real, l, SM>::TPC, smem, st>>>(nimg, src_kind, reinterpret_cast<const SRC*>(src),
                                                    src_stride ? src_stride : (long long)N * N,
                                                    reinterpret_cast<cplx<real>*>(Y),
                                                    reinterpret_cast<const cplx<real>*>(roots));
     return launch_status("pack_fft_kernel");
 }
 
-template <typename real, int l, typename SRC>
+template <typename real, int l, bool SM, typename SRC>
 static int launch_pack_src(int nimg, int src_kind, const void* src, long long src_stride, void* Y, const void* roots,
                            int cols, cudaStream_t st) {
-    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>(), SW = cols_small<real, l>();
-    constexpr int N = 1 << (l - 1);
-    if (cols == 0) {  // the widest that still gives every SM a CTA
-        const long long cta1 = 2ll * nimg * N;  // CTAs at one column each
-        const int sms = device_sm_count();
-        cols = cta1 / A >= sms ? A : (cta1 / NW >= sms ? NW : SW);
-        if (SW != A && SW != NW && cols == SW)
-            return launch_pack_cb<real, l, SW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
-    }
-    if (cols == A) return launch_pack_cb<real, l, A, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
-    if (W != A && cols == W) return launch_pack_cb<real, l, W, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
-    if (NW != W && NW != A && cols == NW) return launch_pack_cb<real, l, NW, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    constexpr int A = cols_auto<real, l, SM>(), F = cols_few<real, l, SM>(), N = 1 << (l - 1);
+    constexpr int W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
+    if (cols == 0) cols = 2ll * nimg * (N / A) >= device_sm_count() ? A : F;
+    if (cols == A) return launch_pack_cb<real, l, A, SM, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    if (F != A && cols == F) return launch_pack_cb<real, l, F, SM, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    if (W != A && W != F && cols == W) return launch_pack_cb<real, l, W, SM, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
+    if (NW != W && NW != A && NW != F && cols == NW)
+        return launch_pack_cb<real, l, NW, SM, SRC>(nimg, src_kind, src, src_stride, Y, roots, st);
     set_error("pack_fft: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
     return ADRT_EINVAL;
+}
+
+template <typename real, int l, typename SRC>
+static int launch_pack_form(int nimg, int src_kind, const void* src, long long src_stride, void* Y, const void* roots,
+                            int cols, cudaStream_t st) {
+    if constexpr (fft_has_small<real, l>()) {
+        if (fft_small(l, nimg)) return launch_pack_src<real, l, true, SRC>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
+    }
+    return launch_pack_src<real, l, false, SRC>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
 }
 
 template <typename real, int l>
 static int launch_pack(int nimg, int src_kind, int src_dtype, const void* src, long long src_stride, void* Y,
                        const void* roots, int cols, cudaStream_t st) {
     if (src_dtype == ADRT_F64)
-        return launch_pack_src<real, l, double>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
-    return launch_pack_src<real, l, float>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
+        return launch_pack_form<real, l, double>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
+    return launch_pack_form<real, l, float>(nimg, src_kind, src, src_stride, Y, roots, cols, st);
 }
 
-template <typename real, int l, int CB>
+template <typename real, int l, int CB, bool SM>
 static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots,
                             cudaStream_t st) {
     constexpr int N = 1 << (l - 1);
     const size_t smem = unpack_smem<real, l, CB>();
-    auto kern = ifft_unpack_kernel<real, l, CB>;
+    auto kern = ifft_unpack_kernel<real, l, CB, SM>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, nimg);
-    kern<<<grid, CB * FftCfg<real, l>::TPC, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z), reinterpret_cast<real*>(colpart),
-                                                   reinterpret_cast<real*>(row0), reinterpret_cast<real*>(row3),
-                                                   reinterpret_cast<const cplx<real>*>(roots));
+    kern<<<grid, CB * FftCfg<real, l, SM>::TPC, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z),
+                                                           reinterpret_cast<real*>(colpart), reinterpret_cast<real*>(row0),
+                                                           reinterpret_cast<real*>(row3),
+                                                           reinterpret_cast<const cplx<real>*>(roots));
     return launch_status("ifft_unpack_kernel");
+}
+
+template <typename real, int l, bool SM>
+static int launch_unpack_form(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots, int cols,
+                              cudaStream_t st) {
+    constexpr int A = cols_auto<real, l, SM>(), F = cols_few<real, l, SM>(), N = 1 << (l - 1);
+    constexpr int W = cols_wide<real, l>(), NW = cols_narrow<real, l>();
+    if (cols == 0) cols = (long long)nimg * (N / A) >= device_sm_count() ? A : F;
+    if (cols == A) return launch_unpack_cb<real, l, A, SM>(nimg, Z, colpart, row0, row3, roots, st);
+    if (F != A && cols == F) return launch_unpack_cb<real, l, F, SM>(nimg, Z, colpart, row0, row3, roots, st);
+    if (W != A && W != F && cols == W) return launch_unpack_cb<real, l, W, SM>(nimg, Z, colpart, row0, row3, roots, st);
+    if (NW != W && NW != A && NW != F && cols == NW)
+        return launch_unpack_cb<real, l, NW, SM>(nimg, Z, colpart, row0, row3, roots, st);
+    set_error("ifft_unpack: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
+    return ADRT_EINVAL;
 }
 
 template <typename real, int l>
 static int launch_unpack(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots, int cols,
                          cudaStream_t st) {
-    constexpr int A = cols_auto<real, l>(), W = cols_wide<real, l>(), NW = cols_narrow<real, l>(), SW = cols_small<real, l>();
-    constexpr int N = 1 << (l - 1);
-    if (cols == 0) {
-        const long long cta1 = (long long)nimg * N;
-        const int sms = device_sm_count();
-        cols = cta1 / A >= sms ? A : (cta1 / NW >= sms ? NW : SW);
-        if (SW != A && SW != NW && cols == SW) return launch_unpack_cb<real, l, SW>(nimg, Z, colpart, row0, row3, roots, st);
+    if constexpr (fft_has_small<real, l>()) {
+        if (fft_small(l, nimg)) return launch_unpack_form<real, l, true>(nimg, Z, colpart, row0, row3, roots, cols, st);
     }
-    if (cols == A) return launch_unpack_cb<real, l, A>(nimg, Z, colpart, row0, row3, roots, st);
-    if (W != A && cols == W) return launch_unpack_cb<real, l, W>(nimg, Z, colpart, row0, row3, roots, st);
-    if (NW != W && NW != A && cols == NW) return launch_unpack_cb<real, l, NW>(nimg, Z, colpart, row0, row3, roots, st);
-    set_error("ifft_unpack: %d columns per CTA unsupported (%d or %d at n=%d)", cols, W, NW, l - 1);
-    return ADRT_EINVAL;
+    return launch_unpack_form<real, l, false>(nimg, Z, colpart, row0, row3, roots, cols, st);
 }
 
 #define ADRT_FFT_CASES(F, ...)                     \
