@@ -10,7 +10,7 @@
 //
 // Persistent CTAs, one per SM, warp-specialised, over units of (frequency, 32 vectors); the units of a frequency run on
 // neighbouring CTAs, which share its matrices through L2:
-//   warps 8..   load a unit's rows (coalesced, LPV lanes per vector, the next rows in flight while the current are
+//   warps 10..  load a unit's rows (coalesced, LPV lanes per vector, the next rows in flight while the current are
 //               converted), apply the phases, fold E and O, scale, split and store both as K-major core matrices. K runs in
 //               the order the lanes hold the values (slot CPL l + 2 q + r is column 2 l + 2 LPV q + r; the matrices are
 //               stored in the same order), so each lane writes 8- or 16-byte pieces; core matrices lie 144 bytes apart,
@@ -18,10 +18,14 @@
 //               turn, so two units are loading while a third multiplies; at N = 512 one group and one buffer fit.
 //   warp 0      streams the matrices, 16 KB (128 rows x 32 columns, hi and lo) per bulk copy, through a ring of four
 //   warp 1      issues the MMAs: M = 128 outputs, N = 64 columns, K = 16
-//   warps 4-7   read the accumulators (two sets, so they overlap the next unit's MMAs), combine e and o, undo scales and
+//   warps 2-9   read the accumulators (two sets, so they overlap the next unit's MMAs), combine e and o, undo scales and
 //               phases and write the rows in place (the unit's rows were all read before its MMAs began).
 // Bounded by HBM and L2 traffic of the rows (N = 256: 16 bytes per value and pass) once the batch is large, by the
-// matrices (34 MB at N = 256, 269 MB at N = 512) when it is small; figures at the dispatch in the host code below.
+// matrices (34 MB at N = 256, 269 MB at N = 512) when it is small. Measured, us per pass: N = 128, 37 images 13.8; N = 256,
+// 64 images 72.4 (268 MB of rows: 55% of the copy rate; the roles' instruction issue and latencies are the rest); N = 512,
+// 6 images 80.8 (370 MB: 67%). With every wait and issue of warps 0 and 1 done by the whole warp, three N = 64 MMAs instead
+// of an N = 128 and an N = 64 one, and four epilogue warps: 20, 79.6 and 88. At N = 512 eight epilogue warps leave too few
+// registers for the loaders (90 against 81).
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -51,8 +55,9 @@ template <int n> struct OmCfg {
     static constexpr int BBUF = PARS * 2 * BT;
     static constexpr int ODD = STACK ? (H / 8) * LBO : 2 * BT;  // from E to O in a buffer
     static constexpr int NB = n == 9 ? 1 : 2;  // B buffers, each with its group of eight loader warps
-    static constexpr int THREADS = 32 * (8 + 8 * NB);
-    static constexpr int ACC = PARS * 4 * VT;  // TMEM columns per accumulator set: product x {lo terms, hi.hi} x 2 VT
+    static constexpr int EPI = n == 9 ? 4 : 8;  // epilogue warps: one or two for each quarter of the tensor memory's lanes
+    static constexpr int THREADS = 32 * (2 + EPI + 8 * NB);
+    static constexpr int ACC = PARS * 4 * VT;  // TMEM columns per accumulator set: product x {hi.hi, lo terms} x 2 VT
     static constexpr size_t smem = (size_t)RING * CHUNK * 2 + (size_t)NB * BBUF + 1024;
 };
 
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
             mbar_init(&b_full[q], 8);  // one arrival per loader warp
             mbar_init(&b_free[q], 1);
             mbar_init(&acc_full[q], 1);
-            mbar_init(&acc_free[q], 4);  // one per epilogue warp
+            mbar_init(&acc_free[q], W::EPI);  // one per epilogue warp
         }
         mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -171,82 +176,86 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
     // the units of this CTA: frequency and first vector; every role walks the same list
     auto vectors = [&](int k) { return nimg * ((k == 0 || k == N) ? 2 : 4); };
 
+    // Warps 0 and 1 run their whole loop on one elected thread: with the warp converged around every wait (poll, shuffle,
+    // election, __syncwarp) a chunk cost ~900 clocks of issue for ~250 of tensor work
     if (warp == 0) {  // matrices
-        int ch = 0;
-        bool ok = true;
-        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
-            const int k = u / tiles;
-            if ((u % tiles) * VT >= vectors(k)) continue;
-            const __half* src = Ts + (size_t)k * W::CHUNKS * W::CHUNK;
-            for (int q = 0; q < W::CHUNKS; ++q, ++ch) {
-                const int s = ch % W::RING, r = ch / W::RING;
-                if (r > 0 && !warp_wait(smem_addr(&a_free[s]), (uint32_t)((r - 1) & 1), abort_flag)) {
-                    if (lane == 0) *abort_flag = 1;
-                    ok = false;
-                    break;
-                }
-                if (lane == 0) {
+        if (elect_one()) {
+            int ch = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int k = u / tiles;
+                if ((u % tiles) * VT >= vectors(k)) continue;
+                const __half* src = Ts + (size_t)k * W::CHUNKS * W::CHUNK;
+                for (int q = 0; q < W::CHUNKS; ++q, ++ch) {
+                    const int s = ch % W::RING, r = ch / W::RING;
+                    if (r > 0 && !mbar_wait_or_abort(smem_addr(&a_free[s]), (uint32_t)((r - 1) & 1), abort_flag)) {
+                        ok = false;
+                        break;
+                    }
                     mbar_expect_bulk(smem_addr(&a_full[s]), smem_addr(ring + (size_t)s * W::CHUNK * 2),
                                      src + (size_t)q * W::CHUNK, W::CHUNK * 2);
                     *s_issued = ch + 1;
                 }
-                __syncwarp();
             }
+            if (!ok) *abort_flag = 1;
         }
+        __syncwarp();
     } else if (warp == 1) {  // MMAs
         // D f32 (bit 4), A and B f16, K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(2 * VT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-        const uint32_t a0 = desc_lo(smem_addr(ring), 128);
-        int ch = 0, un = 0, ac = 0;
-        bool ok = true;
-        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
-            if ((u % tiles) * VT >= vectors(u / tiles)) continue;
-            const int bi = un % W::NB, br = un / W::NB;
-            if (!warp_wait(smem_addr(&b_full[bi]), (uint32_t)(br & 1), abort_flag)) ok = false;
-            const uint32_t b0 = desc_lo(smem_addr(bbuf + (size_t)bi * W::BBUF), W::LBO);
-            for (int mt = 0; ok && mt < W::MT; ++mt, ++ac) {
-                const int ai = ac & 1, ar = ac >> 1;
-                if (ar > 0 && !warp_wait(smem_addr(&acc_free[ai]), (uint32_t)((ar - 1) & 1), abort_flag)) {
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int pk = 0; pk < W::PARS * W::NKC; ++pk, ++ch) {
-                    const int par = pk / W::NKC, kc = pk % W::NKC, s = ch % W::RING;
-                    if (!warp_wait(smem_addr(&a_full[s]), (uint32_t)((ch / W::RING) & 1), abort_flag)) {
+        // the lo tile follows the hi tile and the lo accumulator the hi one, so hi . [hi lo] is one MMA of twice the
+        // columns: it takes as long as one of 64 (65 and 60 clocks measured: both read the same 128 rows of A)
+        constexpr uint32_t idesc2 = idesc + ((uint32_t)(2 * VT >> 3) << 17);
+        static_assert(W::BT == (2 * VT / 8) * W::SBO, "hi and lo column groups are contiguous");
+        constexpr uint32_t AHI = desc_hi((W::KC / 8) * 128), BHI = desc_hi(W::SBO);
+        // byte offsets in 16-byte units: hi to lo tile, one MMA's K
+        constexpr uint32_t ALO = 128 * W::KC * 2 / 16, AK = 256 / 16, BLO = W::BT / 16, BK = 2 * W::LBO / 16;
+        if (elect_one()) {
+            const uint32_t a0 = desc_lo(smem_addr(ring), 128);
+            int ch = 0, un = 0, ac = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                if ((u % tiles) * VT >= vectors(u / tiles)) continue;
+                const int bi = un % W::NB, br = un / W::NB;
+                if (!mbar_wait_or_abort(smem_addr(&b_full[bi]), (uint32_t)(br & 1), abort_flag)) ok = false;
+                const uint32_t b0 = desc_lo(smem_addr(bbuf + (size_t)bi * W::BBUF), W::LBO);
+                for (int mt = 0; ok && mt < W::MT; ++mt, ++ac) {
+                    const int ai = ac & 1, ar = ac >> 1;
+                    if (ar > 0 && !mbar_wait_or_abort(smem_addr(&acc_free[ai]), (uint32_t)((ar - 1) & 1), abort_flag)) {
                         ok = false;
                         break;
                     }
-                    if (elect_one()) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int pk = 0; pk < W::PARS * W::NKC; ++pk, ++ch) {
+                        const int par = pk / W::NKC, kc = pk % W::NKC, s = ch % W::RING;
+                        if (!mbar_wait_or_abort(smem_addr(&a_full[s]), (uint32_t)((ch / W::RING) & 1), abort_flag)) {
+                            ok = false;
+                            break;
+                        }
                         *s_consumed = ch + 1;
-                        const uint32_t dl = tmem + (uint32_t)(ai * W::ACC + par * 4 * VT), dh = dl + 2 * VT;
-                        constexpr uint32_t AHI = desc_hi((W::KC / 8) * 128), BHI = desc_hi(W::SBO);
-                        // byte offsets in 16-byte units: hi to lo tile, one MMA's K
-                        constexpr uint32_t ALO = 128 * W::KC * 2 / 16, AK = 256 / 16, BLO = W::BT / 16, BK = 2 * W::LBO / 16;
+                        const uint32_t dh = tmem + (uint32_t)(ai * W::ACC + par * 4 * VT), dl = dh + 2 * VT;
                         const uint32_t ah = a0 + (uint32_t)(s * (W::CHUNK * 2 / 16));
                         const uint32_t bh = b0 + (uint32_t)(par * 2 * BLO + kc * (W::KC / 16) * BK);
 #pragma unroll
                         for (int ks = 0; ks < W::KC / 16; ++ks) {
-                            const uint32_t acc = ks > 0 || kc > 0 ? 1u : 0u;
-                            mma_f16(dl, ah + ALO + ks * AK, AHI, bh + ks * BK, BHI, idesc, acc);
-                            mma_f16(dh, ah + ks * AK, AHI, bh + ks * BK, BHI, idesc, acc);
-                            mma_f16(dl, ah + ks * AK, AHI, bh + BLO + ks * BK, BHI, idesc, 1u);
+                            mma_f16(dh, ah + ks * AK, AHI, bh + ks * BK, BHI, idesc2, ks > 0 || kc > 0 ? 1u : 0u);
+                            mma_f16(dl, ah + ALO + ks * AK, AHI, bh + ks * BK, BHI, idesc, 1u);
                         }
                         tc_commit(&a_free[s]);
                     }
-                    __syncwarp();
+                    if (ok) {
+                        if (mt == W::MT - 1) tc_commit(&b_free[bi]);
+                        tc_commit(&acc_full[ai]);  // last: once the epilogue has seen it, no arrival is outstanding
+                    }
                 }
-                if (ok && elect_one()) {
-                    if (mt == W::MT - 1) tc_commit(&b_free[bi]);
-                    tc_commit(&acc_full[ai]);  // last: once the epilogue has seen it, no arrival is outstanding
-                }
-                __syncwarp();
+                ++un;
             }
-            ++un;
+            if (!ok) *abort_flag = 1;
         }
-        if (!ok && lane == 0) *abort_flag = 1;
-    } else if (warp >= 4 && warp < 8) {  // epilogue: TMEM lanes 32 (warp % 4) .., one output c per lane
+        __syncwarp();
+    } else if (warp < 2 + W::EPI) {  // epilogue: TMEM lanes 32 (warp % 4) .., one output c per lane; every other 4 vectors
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+        const int eh = (warp - 2) / 4;
         int un = 0, ac = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
@@ -264,9 +273,9 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                 pb = cscale(ti, pb);
                 const float2 na = make_float2(pa.x, self ? pa.y : -pa.y), nb = make_float2(pb.x, self ? pb.y : -pb.y);
                 // vectors v0 + 4 i + q: rows (q & 1) of frequency k, for q >= 2 of -k (self: of the next image)
-                float2* y0 = Y + (long long)(self ? v0 / 2 : v0 / 4) * img_stride;
+                float2* y0 = Y + (long long)((self ? v0 / 2 + 2 * eh : v0 / 4 + eh)) * img_stride;
                 const int r0 = k * N, r1 = (L + k) * N, r2 = self ? r0 : (L - k) * N, r3 = self ? r1 : (2 * L - k) * N;
-                const long long step = (self ? 2 : 1) * img_stride, next = self ? img_stride : 0;
+                const long long step = (self ? 2 : 1) * img_stride * (W::EPI / 4), next = self ? img_stride : 0;
                 if (!warp_wait(smem_addr(&acc_full[ai]), (uint32_t)((ac >> 1) & 1), abort_flag)) {
                     if (lane == 0) *abort_flag = 1;
                     ok = false;
@@ -276,7 +285,7 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
                 const uint32_t d = tmem + lane_base + (uint32_t)(ai * W::ACC);
                 const int left = nv - v0;
 #pragma unroll 1
-                for (int vb = 0; vb < VT && vb < left; vb += 4, y0 += step) {
+                for (int vb = 4 * eh; vb < VT && vb < left; vb += W::EPI, y0 += step) {
                     float er[4], ei[4], t0[4], t1[4], orr[4], oi[4], t2[4], t3[4];
                     tmem_ld4(d + vb, er);
                     tmem_ld4(d + VT + vb, ei);
@@ -312,10 +321,10 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
             }
             ++un;
         }
-    } else if (warp >= 8) {  // rows of the unit -> E and O, split, in shared memory
+    } else {  // rows of the unit -> E and O, split, in shared memory
         constexpr int VPW = 32 / LPV;     // vectors per warp and step
         constexpr int STEP = 8 * VPW;     // vectors per step of the group
-        const int l = lane % LPV, vs = lane / LPV, grp = (warp - 8) / 8, w8 = (warp - 8) % 8;
+        const int l = lane % LPV, vs = lane / LPV, lw = warp - 2 - W::EPI, grp = lw / 8, w8 = lw % 8;
         int un = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
