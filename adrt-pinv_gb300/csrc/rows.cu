@@ -205,7 +205,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 // row programs, out of place or in place. Bounded by memory and by the twiddles (about as many loads and registers as a
 // row itself), so a group keeps them for up to `per` consecutive images of its row, the B-layout levels hold z^t alone
 // (z^(t+1) f = z (z^t f) forward, z^t* (g0 + z* g1) adjoint: two operations more per pair, 30 registers less, no
-// spills), and two CTAs share an SM.
+// spills), and two CTAs share an SM. Rows cross global memory in contiguous 16-byte pieces: the next row is copied into
+// shared memory (asynchronously) while this one is computed, the result staged in the exchange buffer. (Reading and writing
+// the A layout directly, 16 bytes per lane at a stride of R values, kept L1 88% busy with 14% of DRAM.)
 template <typename real, int n>
 __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
     rows_gram_kernel(const adrt_row_job J, const cplx<real>* in, const TwSrc<real> tw, const int per, const int total) {
@@ -222,9 +224,24 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
     const unsigned gm = (T >= 32) ? 0xffffffffu : (((1u << T) - 1u) << (giw * T));
     constexpr int GROUPS = FAST_THREADS / T;
     const int chunks = (J.nimg + per - 1) / per;
-    for (int item = blockIdx.x * GROUPS + threadIdx.x / T; item < total; item += gridDim.x * GROUPS) {
-        const int sel = item / chunks, img0 = (item - sel * chunks) * per;
-        const int row = J.rows ? J.rows[sel] : sel;
+    constexpr int EPP = 16 / (int)sizeof(C);  // values per 16-byte piece
+    C* pre = buf + F::BUF;                    // the row that is computed next, swizzled as buf is
+    auto row_of = [&](int it) { return J.rows ? J.rows[it / chunks] : it / chunks; };
+    auto img_of = [&](int it) { return it % chunks * per; };
+    auto offset = [&](int row, int img) { return (size_t)img * J.img_stride + (size_t)row * N; };
+    auto fetch = [&](size_t at) {
+#pragma unroll
+        for (int i = 0; i < R / EPP; ++i) {
+            const int p = (i * T + u) * EPP;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(pre + F::phys(p))),
+                         "l"(in + at + p)
+                         : "memory");
+        }
+    };
+    const int first = blockIdx.x * GROUPS + threadIdx.x / T;
+    if (first < total) fetch(offset(row_of(first), img_of(first)));
+    for (int item = first; item < total; item += gridDim.x * GROUPS) {
+        const int img0 = img_of(item), row = row_of(item);
         const int key = tw.roots ? row % J.freq_mod : row;
         C tA[R / 2 + 1];
 #pragma unroll
@@ -248,10 +265,16 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
         const C z = n > 1 ? tA[1] : tw.get(key, 1), zc = mk<real>(z.x, -z.y);
         const int img1 = img0 + per < J.nimg ? img0 + per : J.nimg;
         for (int img = img0; img < img1; ++img) {
-            const size_t at = (size_t)img * J.img_stride + (size_t)row * N;
+            const size_t at = offset(row, img);
             C v[R];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            Ln::gsync(gm);
 #pragma unroll
-            for (int j = 0; j < R; j += 2) ld2(in + at + j + R * u, v[j], v[j + 1]);
+            for (int j = 0; j < R; j += 2) ld2(pre + F::phys(j + R * u), v[j], v[j + 1]);
+            Ln::gsync(gm);
+            const int next = item + gridDim.x * GROUPS;
+            if (img + 1 < img1) fetch(offset(row, img + 1));
+            else if (next < total) fetch(offset(row_of(next), img_of(next)));
             Ln::fwdA(v, tA, 1, n);
             if (n > F::r) {
                 Ln::fwdM(v, tA, 1, n, u, zt);
@@ -284,7 +307,13 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
             Ln::adjA(v, tA, 1, n);
             C* ptr = reinterpret_cast<C*>(J.X) + at;
 #pragma unroll
-            for (int j = 0; j < R; j += 2) st2(ptr + j + R * u, v[j], v[j + 1]);
+            for (int j = 0; j < R; j += 2) st2(buf + F::phys(j + R * u), v[j], v[j + 1]);
+            Ln::gsync(gm);
+#pragma unroll
+            for (int i = 0; i < R / EPP; ++i) {  // the loop's first barrier keeps the next row out of buf until all have read
+                const int p = (i * T + u) * EPP;
+                *reinterpret_cast<float4*>(ptr + p) = *reinterpret_cast<const float4*>(buf + F::phys(p));
+            }
         }
     }
 }
@@ -559,9 +588,15 @@ static int launch_gram(const adrt_row_job& J, const void* in, const TwSrc<real>&
     auto kern = rows_gram_kernel<real, n>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     const int groups = FAST_THREADS / F::T, slots = (J.grid > 0 ? J.grid : num_sms()) * (sizeof(real) == 4 ? 2 : 1);
-    // images per item: as many as keep two items per resident group, up to 4
+    // images per item: an item costs its images and its twiddles (about as much as one more image), and the resident groups
+    // take ceil(items / groups) rounds. N = 256, 24 images: 39.2 us with 2 per item, 33.8 with the 6 this picks
     int per = 1;
-    while (per < 4 && (long long)J.nsel * ((J.nimg + 2 * per - 1) / (2 * per)) >= 2ll * slots * groups) per *= 2;
+    long long best = -1;
+    for (int p = 1; p <= 16 && p <= J.nimg; ++p) {
+        const long long items = (long long)J.nsel * ((J.nimg + p - 1) / p), all = (long long)slots * groups;
+        const long long cost = (items + all - 1) / all * (p + 1);
+        if (best < 0 || cost < best) { best = cost; per = p; }
+    }
     const long long total = (long long)J.nsel * ((J.nimg + per - 1) / per);
     const long long ctas = (total + groups - 1) / groups;
     kern<<<(unsigned)(ctas < slots ? ctas : slots), FAST_THREADS, smem, st>>>(J, reinterpret_cast<const cplx<real>*>(in), tw, per,
