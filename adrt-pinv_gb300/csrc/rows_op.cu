@@ -16,11 +16,12 @@
 // FMAs per Gram and d_k of them (mean degree 7 at N = 256: 100 k against 66 k), and the filter's ill-conditioned rows lose
 // nothing to the recurrence, because the matrices are evaluated in FP64 when the plan's tables are built.
 //
-// Two kernels, both in place (a CTA reads whole rows before it writes them):
-//  rows_op_small  few vectors (and FP64): bounded by reading the matrices (N^2/2 values per frequency, 34 MB in FP32
+// Three kernels, all in place (a CTA reads whole rows before it writes them):
+//  rows_op_small  few vectors (and FP64 from N = 256): bounded by reading the matrices (N^2/2 values per frequency, 34 MB in FP32
 //                 at N = 256, L2 resident) and by latency, so a CTA takes a frequency and at most 8 vectors, its
 //                 256 threads split the sum over j, every matrix value is read once per CTA straight into registers
 //                 (coalesced over c) and the partial sums meet in shared memory.
+//  rows_op_direct N = 64, and N = 128 in FP64: one output per thread, no partial sums.
 //  rows_op_tile   many vectors (FP32): bounded by the FP32 pipe; a CTA keeps E and O of 4096 / H vectors in shared
 //                 memory, streams the matrices through a cp.async ring and each thread owns an 8 x 8 tile of both
 //                 products (128 FMAs per eight 16-byte shared loads), so e_c and o_c meet in registers.
@@ -146,6 +147,75 @@ __global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __res
             y[c] = conj_if(cmulc(roots[op_phase_out<n>(k, c)], cadd(se, so)), w.neg);
             y[N - 1 - c] = conj_if(cmulc(roots[op_phase_out<n>(k, N - 1 - c)], csub(se, so)), w.neg);
         }
+    }
+}
+
+// ------------------------------------------------------------------ rows of 64, and of 128 in FP64
+// A thread per real output (c, parity, vector, re / im) and the whole sum over j: where the FP64 pipe (half a lane per clock
+// and SM quarter) is the bound, the partial sums of rows_op_small's slices would cost as many additions as the products at
+// H = 32. Every value computed once, by as many warps as it takes to reach all four quarters; the thread's matrix column
+// is in flight before the rows are.
+template <typename real, int n>
+__global__ void __launch_bounds__(256) rows_op_direct(int nimg, const real* __restrict__ T, cplx<real>* Y, long long img_stride,
+                                                      const cplx<real>* __restrict__ roots, bool bp) {
+    using C = cplx<real>;
+    constexpr int N = OpCfg<n>::N, H = OpCfg<n>::H, VT = 64 / H, PF = 16;
+    static_assert(VT * H * 4 == 256 && H % PF == 0 && H % 32 == 0, "one output per thread, one combination per warp");
+    __shared__ __align__(16) real as[2][VT * N];   // phased rows, re and im
+    __shared__ __align__(16) real X[VT * 4 * H];   // E and O: [parity][vector][re, im][j]; then e and o over c
+    const int k = blockIdx.y, v0 = blockIdx.x * VT;
+    const bool self = k == 0 || k == N;
+    const int nv = nimg * (self ? 2 : 4);
+    if (v0 >= nv) return;
+    const int c = threadIdx.x % H, combo = threadIdx.x / H, ri = combo & 1, v = combo / 2 % VT, par = combo / (2 * VT);
+    const real* Tc = T + ((size_t)k * 2 + par) * H * H + c;
+    real t[2][PF];
+#pragma unroll
+    for (int q = 0; q < 2 * PF; ++q) t[q / PF][q % PF] = Tc[(size_t)q * H];
+    // one component of one phased value per thread
+    const int es = threadIdx.x >> 1, ec = threadIdx.x & 1, ev = es / N, col = es % N;
+    const bool live = v0 + ev < nv;
+    const OpVec w = op_vec<n>(k, v0 + ev);
+    C* y = Y + (long long)w.img * img_stride + (long long)w.row * N + col;
+    real part = 0;
+    if (live) {
+        const C a = conj_if(*y, w.neg), r = roots[op_phase_in<n>(k, col, bp)];
+        part = ec ? fma(r.x, a.y, r.y * a.x) : fma(r.x, a.x, -(r.y * a.y));
+    }
+    as[ec][es] = part;
+    C ro = mk<real>(0, 0);
+    if (live && ec == 0) ro = roots[op_phase_out<n>(k, col)];
+    __syncthreads();
+    {
+        // O = a - b, or -i (a - b) for the back-projections
+        const int src = par && bp ? 1 - ri : ri;
+        const real a = as[src][v * N + c], b = as[src][v * N + N - 1 - c];
+        X[threadIdx.x] = par ? (bp && ri ? b - a : a - b) : a + b;
+    }
+    __syncthreads();
+    const real* x = X + combo * H;
+    real s0 = 0, s1 = 0;
+#pragma unroll
+    for (int ch = 0; ch < H / PF; ++ch) {
+#pragma unroll
+        for (int q = 0; q < PF; q += 2) {
+            s0 = fma(t[ch & 1][q], x[ch * PF + q], s0);
+            s1 = fma(t[ch & 1][q + 1], x[ch * PF + q + 1], s1);
+        }
+        if (ch + 2 < H / PF) {
+#pragma unroll
+            for (int q = 0; q < PF; ++q) t[ch & 1][q] = Tc[(size_t)((ch + 2) * PF + q) * H];
+        }
+    }
+    __syncthreads();
+    X[threadIdx.x] = s0 + s1;
+    __syncthreads();
+    if (live && ec == 0) {
+        const int o = col < H ? col : N - 1 - col;
+        const real* e = X + 2 * ev * H + o;
+        const real* d = e + 2 * VT * H;
+        const C z = col < H ? mk<real>(e[0] + d[0], e[H] + d[H]) : mk<real>(e[0] - d[0], e[H] - d[H]);
+        *y = conj_if(cmulc(ro, z), w.neg);
     }
 }
 
@@ -279,6 +349,15 @@ static int launch_small(int nimg, const void* T, void* Y, long long img_stride, 
     return launch_status("rows_op_small");
 }
 
+template <typename real, int n>
+static int launch_direct(int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp, cudaStream_t st) {
+    constexpr int N = OpCfg<n>::N, VT = 128 / N;
+    rows_op_direct<real, n><<<dim3((4 * nimg + VT - 1) / VT, N + 1), 256, 0, st>>>(
+        nimg, reinterpret_cast<const real*>(T), reinterpret_cast<cplx<real>*>(Y), img_stride,
+        reinterpret_cast<const cplx<real>*>(roots), bp);
+    return launch_status("rows_op_direct");
+}
+
 template <int n>
 static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp, cudaStream_t st) {
     using W = OpTile<n>;
@@ -293,12 +372,21 @@ static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, c
 template <int n>
 static int rows_operator_n(int dtype, int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp,
                            cudaStream_t st) {
-    if (dtype == ADRT_F64) {
-        if (nimg == 1) return launch_small<double, n, 2>(nimg, T, Y, img_stride, roots, bp, st);
-        return launch_small<double, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
+    // Measured, us per pass. FP64, one image, small / direct: N = 64 10.4 / 5.2 (32 images 184 / 89), N = 128 25.4 / 22.9 (16
+    // images 353 / 283). FP32 N = 64, direct / small or tile: one image 2.3 / 3.0, 16 7.1 / 12.4, 32 11.9 / 16.8, 48 16.8 /
+    // 16.4. FP32 N = 128, small / direct: one image 3.9 / 4.1
+    if constexpr (n == 6) {
+        if (dtype == ADRT_F64) return launch_direct<double, n>(nimg, T, Y, img_stride, roots, bp, st);
+        if (nimg <= 40) return launch_direct<float, n>(nimg, T, Y, img_stride, roots, bp, st);
+    } else {
+        if (dtype == ADRT_F64) {
+            if constexpr (n == 7) return launch_direct<double, n>(nimg, T, Y, img_stride, roots, bp, st);
+            else if (nimg == 1) return launch_small<double, n, 2>(nimg, T, Y, img_stride, roots, bp, st);
+            else return launch_small<double, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
+        }
+        if (nimg == 1) return launch_small<float, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
+        if (4 * nimg <= OpTile<n>::VT / 2) return launch_small<float, n, 8>(nimg, T, Y, img_stride, roots, bp, st);
     }
-    if (nimg == 1) return launch_small<float, n, 4>(nimg, T, Y, img_stride, roots, bp, st);
-    if (4 * nimg <= OpTile<n>::VT / 2) return launch_small<float, n, 8>(nimg, T, Y, img_stride, roots, bp, st);
     return launch_tile<n>(nimg, T, Y, img_stride, roots, bp, st);
 }
 
