@@ -15,7 +15,8 @@
 //         butterfly is never computed), and the four quadrant strips go with TqT and cropped into three image-space
 //         partial sums: colpart (quadrants II+III: out columns), rowpart0 (quadrant I: out rows), rowpart3 (quadrant
 //         IV). Pair (0,1) runs with the threads of a column in reverse order, so that the offsets i of quadrant III and
-//         N-1-i of quadrant II meet in one thread; the row quadrants are transposed through shared memory.
+//         N-1-i of quadrant II meet in one thread; the row quadrants are transposed through shared memory. Small
+//         launches transform both pairs at once, half of the threads each, and quadrant II crosses shared memory.
 #include <type_traits>
 
 #include "common.cuh"
@@ -27,8 +28,10 @@ template <typename real, int l, bool SM> struct FftCfg {
     static constexpr int L = 1 << l;
     // log2 of points per thread: in FP32 as many as take a pass (an exchange, a twiddle multiply) less: 32 points at
     // L = 512 and 1024 (two passes), 16 at 128, 256 and above. FP64 is bound by its pipe (half a lane per clock and SM
-    // quarter): 8. Small launches (SM) are bound by the length of a thread's chain instead: fewer points, more threads
-    static constexpr int e = l < 3 ? l : sizeof(real) == 8 ? (SM ? 2 : 3) : SM ? 3 : l == 9 || l == 10 ? 5
+    // quarter): 8. Small launches (SM) are bound by the length of a thread's chain instead: fewer points, more threads (an
+    // FP64 instruction holds a warp's quarter for 64 clocks: 2 points up to L = 128, where 4 take 5.2 / 8.4 us against 4.3 /
+    // 6.0; at L = 256 the exchanges cost more than that saves, 6.8 / 11.2 against 6.2 / 9.3)
+    static constexpr int e = l < 3 ? l : sizeof(real) == 8 ? (SM ? (l <= 7 ? 1 : 2) : 3) : SM ? 3 : l == 9 || l == 10 ? 5
                              : (l + 3) / 4 < (l + 2) / 3 ? 4 : 3;
     static constexpr int E = 1 << e;
     static constexpr int TPC = L / E;           // threads per column
@@ -137,7 +140,9 @@ template <typename real, int l, int CB, bool SM> struct FftLaunch {
     // threads per SM: 64 registers each for 8 points in FP32, twice that for more points or FP64
     static constexpr int resident = sizeof(real) == 4 && FftCfg<real, l, SM>::e < 4 ? 1024 : 512;
     static constexpr int pack_min = imin(16, imax(1, (FftCfg<real, l, SM>::e < 4 && sizeof(real) == 4 ? 2048 : resident) / threads));
-    static constexpr int unpack_min = imin(16, imax(1, resident / threads));
+    static constexpr bool both = SM && 2 * threads <= 1024;  // unpack transforms its two pairs at once
+    static constexpr int unpack_threads = both ? 2 * threads : threads;
+    static constexpr int unpack_min = imin(16, imax(1, resident / unpack_threads));
 };
 
 template <typename real, int l, int CB, bool SM, typename SRC>
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch
 }
 
 template <typename real, int l, int CB, bool SM>
-__global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch<real, l, CB, SM>::unpack_min)
+__global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::unpack_threads, FftLaunch<real, l, CB, SM>::unpack_min)
     ifft_unpack_kernel(int nimg, const cplx<real>* __restrict__ Z, real* __restrict__ colpart, real* __restrict__ row0,
                        real* __restrict__ row3, const cplx<real>* __restrict__ roots_g) {
     using F = FftCfg<real, l, SM>;
@@ -240,51 +245,85 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch
     constexpr int CP = fft_pad(CB), RP = N + 1;  // row pitch of the transposed strips
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* roots = reinterpret_cast<C*>(smem_raw);
-    C* tile = roots + L;                              // L x CP exchange tile
-    real* rowt = reinterpret_cast<real*>(tile + L * CP);  // CB x RP: quadrant I transposed (pair (2,3) uses the tile)
+    C* tile = roots + L;                              // L x CP exchange tile (both: one per pair)
+    constexpr bool BOTH = FftLaunch<real, l, CB, SM>::both;
+    real* rowt = reinterpret_cast<real*>(tile + (BOTH ? 2 : 1) * L * CP);  // CB x RP: quadrant I transposed
     const int c0 = blockIdx.x * CB;
     const int img = blockIdx.y;
-    const int nthr = CB * F::TPC;
+    constexpr int nthr = FftLaunch<real, l, CB, SM>::unpack_threads;
     for (int i = threadIdx.x; i < L; i += nthr) roots[i] = roots_g[i];
-    const int c = threadIdx.x % CB, t = threadIdx.x / CB;
+    const int tid = BOTH ? threadIdx.x % (nthr / 2) : threadIdx.x;
+    const int c = tid % CB, t = tid / CB;
     const real scale = (real)1 / (real)L;
     const size_t ib = (size_t)img * N * N;
-    real im0[E];
-#pragma unroll
-    for (int pair = 0; pair < 2; ++pair) {
-        // pair (0,1) with the column's threads reversed: output p of thread t is then N-1-p of pair (2,3)'s
-        const int tt = pair == 0 ? F::TPC - 1 - t : t;
+    constexpr int bl = F::nb(F::NPASS - 1), top = 1 << (bl - 1);  // register bit of the offset's top bit
+    auto load = [&](int pair, int tt, C (&x)[E]) {
         const int rt = F::TPC > 1 ? (int)(__brev((unsigned)tt) >> (32 - (F::TPC > 1 ? l - F::e : 1))) : 0;
         const C* in = Z + ((size_t)img * 2 * L + (size_t)pair * L) * N + c0 + c;
-        C x[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) x[j] = in[(size_t)(brev(j, F::e) * (L / E) + rt) * N];
-        if (pair == 0) __syncthreads();  // roots
-        dit_passes<real, l, true, SM>(x, roots, tile, CP, c, tt);
-        real* rows = rowt;
-        if (pair == 1) {
-            __syncthreads();  // the exchange tile is free
-            rows = reinterpret_cast<real*>(tile);
-        }
-        constexpr int bl = F::nb(F::NPASS - 1), top = 1 << (bl - 1);  // register bit of the offset's top bit
+    };
+    real* r3 = reinterpret_cast<real*>(tile);  // quadrant IV transposed, over the exchange tile
+    if constexpr (BOTH) {
+        // one half of the threads per pair; quadrant II crosses to quadrant III's threads through pair 0's tile
+        const int pair = threadIdx.x / (nthr / 2);
+        C x[E];
+        load(pair, t, x);
+        __syncthreads();  // roots
+        dit_passes<real, l, true, SM>(x, roots, tile + pair * L * CP, CP, c, t);
+        __syncthreads();  // the exchange tiles are free
+        real* im = reinterpret_cast<real*>(tile);
+        r3 = reinterpret_cast<real*>(tile + L * CP);
+        real* rows = pair == 0 ? rowt : r3;
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             if (j & top) continue;  // offsets >= N
-            const int p = F::pos(F::NPASS - 1, tt, j);
-            if (pair == 0) {
-                rows[c * RP + (N - 1 - p)] = scale * x[j].x;
-                im0[j] = scale * x[j].y;
-            } else {
-                rows[c * RP + (N - 1 - p)] = scale * x[j].y;
-                // colpart[i][c0+c] = S_III[i][c] + S_II[N-1-i][c]: the register of the complementary offset
-                const int jc = (E - 1 - j) & ~top;
-                colpart[ib + (size_t)p * N + c0 + c] = scale * x[j].x + im0[jc];
+            const int p = F::pos(F::NPASS - 1, t, j);
+            rows[c * RP + (N - 1 - p)] = scale * (pair == 0 ? x[j].x : x[j].y);
+            if (pair == 0) im[(N - 1 - p) * CP + c] = scale * x[j].y;
+        }
+        __syncthreads();
+        if (pair == 1) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                if (j & top) continue;
+                const int p = F::pos(F::NPASS - 1, t, j);
+                colpart[ib + (size_t)p * N + c0 + c] = scale * x[j].x + im[p * CP + c];
             }
         }
+    } else {
+        real im0[E];
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+            // pair (0,1) with the column's threads reversed: output p of thread t is then N-1-p of pair (2,3)'s
+            const int tt = pair == 0 ? F::TPC - 1 - t : t;
+            C x[E];
+            load(pair, tt, x);
+            if (pair == 0) __syncthreads();  // roots
+            dit_passes<real, l, true, SM>(x, roots, tile, CP, c, tt);
+            real* rows = rowt;
+            if (pair == 1) {
+                __syncthreads();  // the exchange tile is free
+                rows = r3;
+            }
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                if (j & top) continue;  // offsets >= N
+                const int p = F::pos(F::NPASS - 1, tt, j);
+                if (pair == 0) {
+                    rows[c * RP + (N - 1 - p)] = scale * x[j].x;
+                    im0[j] = scale * x[j].y;
+                } else {
+                    rows[c * RP + (N - 1 - p)] = scale * x[j].y;
+                    // colpart[i][c0+c] = S_III[i][c] + S_II[N-1-i][c]: the register of the complementary offset
+                    const int jc = (E - 1 - j) & ~top;
+                    colpart[ib + (size_t)p * N + c0 + c] = scale * x[j].x + im0[jc];
+                }
+            }
+        }
+        __syncthreads();
     }
-    __syncthreads();
     // rowpart0[c0+c][N-1-r] = S_I[r][c] ; rowpart3[N-1-c0-c][N-1-r] = S_IV[r][c]
-    const real* r3 = reinterpret_cast<const real*>(tile);
     for (int e = threadIdx.x; e < N * CB; e += nthr) {
         const int r = e % N, cc = e / N;
         row0[ib + (size_t)(c0 + cc) * N + r] = rowt[cc * RP + r];
@@ -295,15 +334,16 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch
 template <typename real, int l, int CB> static size_t pack_smem() {
     return ((size_t)(1 << l) + (size_t)(1 << l) * fft_pad(CB)) * sizeof(cplx<real>);
 }
-template <typename real, int l, int CB> static size_t unpack_smem() {
-    return ((size_t)(1 << l) + (size_t)(1 << l) * fft_pad(CB)) * sizeof(cplx<real>) +
+template <typename real, int l, int CB, bool SM> static size_t unpack_smem() {
+    return ((size_t)(1 << l) + (size_t)(1 << l) * fft_pad(CB) * (FftLaunch<real, l, CB, SM>::both ? 2 : 1)) * sizeof(cplx<real>) +
            (size_t)CB * ((1 << (l - 1)) + 1) * sizeof(real);
 }
 
 // Small launches: at most two images' worth of columns at N = 256. Which form runs depends on the size and batch alone, not
 // on the columns per CTA, so every column is transformed by the same arithmetic whatever the CTA shape. Measured (pack /
-// unpack us, small against large form): FP32 N = 256, one image 3.5 / 4.6 against 4.6 / 5.9, four 4.9 / 7.1 against 4.7 /
-// 6.0; FP64 N = 64, one image 5.2 / 8.4 against 8.2 / 13.6, N = 256, eight 136 / 137 against 125 / 127.
+// unpack us, small against large form): FP32 N = 256, one image 3.5 / 4.2 against 4.6 / 5.9 (four, without both pairs at
+// once: 4.9 / 7.1 against 4.7 / 6.0); FP64 N = 64, one image 4.3 / 6.0 against 8.2 / 13.6, eight 9.5 / 9.4 against 9.2 /
+// 13.9; N = 128, four 16.5 / 17.1 against 16.6 / 17.0; N = 256, two 36 / 36 against 34 / 33, eight 136 / 137 against 125 / 127.
 template <typename real, int l> constexpr bool fft_has_small() { return sizeof(real) == 8 ? l >= 4 : l == 9; }
 static bool fft_small(int l, int nimg) { return ((long long)nimg << (l - 1)) <= 512; }
 
@@ -372,11 +412,11 @@ template <typename real, int l, int CB, bool SM>
 static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, void* row3, const void* roots,
                             cudaStream_t st) {
     constexpr int N = 1 << (l - 1);
-    const size_t smem = unpack_smem<real, l, CB>();
+    const size_t smem = unpack_smem<real, l, CB, SM>();
     auto kern = ifft_unpack_kernel<real, l, CB, SM>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, nimg);
-    kern<<<grid, CB * FftCfg<real, l, SM>::TPC, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z),
+    kern<<<grid, FftLaunch<real, l, CB, SM>::unpack_threads, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z),
                                                            reinterpret_cast<real*>(colpart), reinterpret_cast<real*>(row0),
                                                            reinterpret_cast<real*>(row3),
                                                            reinterpret_cast<const cplx<real>*>(roots));
