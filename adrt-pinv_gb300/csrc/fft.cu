@@ -160,6 +160,9 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::threads, FftLaunch
     const int c0 = blockIdx.x * CB;
     const int pair = blockIdx.y;
     const int img = blockIdx.z;
+    chain_wait();
+    src = after_wait(src);
+    roots_g = after_wait(roots_g);
     constexpr int nthr = CB * F::TPC;
     for (int i = threadIdx.x; i < L; i += nthr) roots[i] = roots_g[i];
     const int c = threadIdx.x % CB, t = threadIdx.x / CB;
@@ -250,6 +253,9 @@ __global__ void __launch_bounds__(FftLaunch<real, l, CB, SM>::unpack_threads, Ff
     real* rowt = reinterpret_cast<real*>(tile + (BOTH ? 2 : 1) * L * CP);  // CB x RP: quadrant I transposed
     const int c0 = blockIdx.x * CB;
     const int img = blockIdx.y;
+    chain_wait();
+    Z = after_wait(Z);
+    roots_g = after_wait(roots_g);
     constexpr int nthr = FftLaunch<real, l, CB, SM>::unpack_threads;
     for (int i = threadIdx.x; i < L; i += nthr) roots[i] = roots_g[i];
     const int tid = BOTH ? threadIdx.x % (nthr / 2) : threadIdx.x;
@@ -369,11 +375,9 @@ static int launch_pack_cb(int nimg, int src_kind, const void* src, long long src
     auto kern = pack_fft_kernel<real, l, CB, SM, SRC>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, 2, nimg);
-    kern<<<grid, CB * FftCfg<real, l, SM>::TPC, smem, st>>>(nimg, src_kind, reinterpret_cast<const SRC*>(src),
-                                                   src_stride ? src_stride : (long long)N * N,
-                                                   reinterpret_cast<cplx<real>*>(Y),
-                                                   reinterpret_cast<const cplx<real>*>(roots));
-    return launch_status("pack_fft_kernel");
+    return launch_chained("pack_fft_kernel", kern, grid, CB * FftCfg<real, l, SM>::TPC, smem, st, nimg, src_kind,
+                          reinterpret_cast<const SRC*>(src), src_stride ? src_stride : (long long)N * N,
+                          reinterpret_cast<cplx<real>*>(Y), reinterpret_cast<const cplx<real>*>(roots));
 }
 
 template <typename real, int l, bool SM, typename SRC>
@@ -416,11 +420,10 @@ static int launch_unpack_cb(int nimg, const void* Z, void* colpart, void* row0, 
     auto kern = ifft_unpack_kernel<real, l, CB, SM>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     dim3 grid(N / CB, nimg);
-    kern<<<grid, FftLaunch<real, l, CB, SM>::unpack_threads, smem, st>>>(nimg, reinterpret_cast<const cplx<real>*>(Z),
-                                                           reinterpret_cast<real*>(colpart), reinterpret_cast<real*>(row0),
-                                                           reinterpret_cast<real*>(row3),
-                                                           reinterpret_cast<const cplx<real>*>(roots));
-    return launch_status("ifft_unpack_kernel");
+    return launch_chained("ifft_unpack_kernel", kern, grid, FftLaunch<real, l, CB, SM>::unpack_threads, smem, st, nimg,
+                          reinterpret_cast<const cplx<real>*>(Z), reinterpret_cast<real*>(colpart),
+                          reinterpret_cast<real*>(row0), reinterpret_cast<real*>(row3),
+                          reinterpret_cast<const cplx<real>*>(roots));
 }
 
 template <typename real, int l, bool SM>

@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(OS_THREADS) outer_step_kernel(const OuterStepA
     const TP* p0 = reinterpret_cast<const TP*>(A.p0);
     const TP* p1 = reinterpret_cast<const TP*>(A.p1);
     const TP* p2 = reinterpret_cast<const TP*>(A.p2);
+    chain_wait();
 
     // residual into shared memory (the partial images summed in their own precision, the difference in FP64); two
     // neighbouring elements per thread and load (E and the image offsets are even)
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(32 * (BAND / (1024 >> n)), (1 << n) <= 256 ? 2
     const int j0 = lane * CPT;
     const size_t gbase = (size_t)img * N * N + (size_t)(rank * BAND + w * R) * N + j0;
     constexpr unsigned FULL = 0xffffffffu;
+    chain_wait();
 
     // residual: the partial images summed in FP32, the difference in FP64 rounded to FP32 (FP64 y), or in FP32 (FP32
     // y: the same value, since the exact difference of two FP32 numbers is rounded once either way)
@@ -557,6 +559,7 @@ __global__ void __launch_bounds__(32 * W, MINB) outer_step_tile_kernel(const Out
     const bool inside = col >= 0 && col < N && row >= 0 && row < N;  // strips and lanes never straddle the border
     const size_t gi = (size_t)img * N * N + (size_t)row * N + col;
     constexpr unsigned FULL = 0xffffffffu;
+    chain_wait();
 
     float s[R][CPT], c[R][CPT], e[R][CPT];
 #pragma unroll
@@ -644,8 +647,8 @@ template <int LPR, int R, int W, int MINB>
 static int launch_os_tile(const OuterStepArgs& A, int n, int nimg, cudaStream_t st) {
     using T = OtCfg<LPR, R, W>;
     const int N = 1 << n, tx = (N + T::OUTC - 1) / T::OUTC, ty = (N + T::OUTR - 1) / T::OUTR;
-    outer_step_tile_kernel<LPR, R, W, MINB><<<dim3(tx * ty, nimg), 32 * W, 0, st>>>(A, n, tx);
-    return launch_status("outer_step_tile_kernel");
+    return launch_chained("outer_step_tile_kernel", outer_step_tile_kernel<LPR, R, W, MINB>, dim3(tx * ty, nimg), 32 * W, 0, st,
+                          A, n, tx);
 }
 
 template <int n, int BAND, bool FF>
@@ -666,13 +669,15 @@ static int launch_os_reg(const OuterStepArgs& A, int nimg, cudaStream_t st) {
     cfg.blockDim = dim3(32 * W);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CL;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     return launch_ex_status(cudaLaunchKernelEx(&cfg, kern, A), "outer_step_reg_kernel");
 }
 
@@ -693,13 +698,15 @@ static int launch_os_band(const OuterStepArgs& A, int nimg, cudaStream_t st) {
     cfg.blockDim = dim3(OS_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CL;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     return launch_ex_status(cudaLaunchKernelEx(&cfg, kern, A), "outer_step_kernel");
 }
 

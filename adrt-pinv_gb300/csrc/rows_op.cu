@@ -95,6 +95,9 @@ __global__ void __launch_bounds__(256) rows_op_small(int nimg, const real* __res
     const int k = blockIdx.y, v0 = blockIdx.x * VT;
     const int nv = nimg * ((k == 0 || k == N) ? 2 : 4);
     if (v0 >= nv) return;
+    chain_wait();
+    T = after_wait(T);
+    roots = after_wait(roots);
     op_load<real, n, VT, 256, VT>(Y, img_stride, roots, bp, k, v0, nv, E, O);
     __syncthreads();
 
@@ -167,6 +170,9 @@ __global__ void __launch_bounds__(256) rows_op_direct(int nimg, const real* __re
     const bool self = k == 0 || k == N;
     const int nv = nimg * (self ? 2 : 4);
     if (v0 >= nv) return;
+    chain_wait();
+    T = after_wait(T);
+    roots = after_wait(roots);
     const int c = threadIdx.x % H, combo = threadIdx.x / H, ri = combo & 1, v = combo / 2 % VT, par = combo / (2 * VT);
     const real* Tc = T + ((size_t)k * 2 + par) * H * H + c;
     real t[2][PF];
@@ -252,6 +258,9 @@ __global__ void __launch_bounds__(OpTile<n>::THREADS, 2)
     const int k = blockIdx.y, v0 = blockIdx.x * VT;
     const int nv = nimg * ((k == 0 || k == N) ? 2 : 4);
     if (v0 >= nv) return;
+    chain_wait();
+    T = after_wait(T);
+    roots = after_wait(roots);
     const float* Tk = T + (size_t)k * 2 * H * H;
     auto fetch = [&](int ch) {
         if (ch < NCH) {
@@ -343,19 +352,17 @@ static int launch_small(int nimg, const void* T, void* Y, long long img_stride, 
     const size_t smem = (size_t)(2 * H * VT + KS * 2 * VB * H) * sizeof(cplx<real>);
     auto kern = rows_op_small<real, n, VT>;
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
-    kern<<<dim3((4 * nimg + VT - 1) / VT, N + 1), 256, smem, st>>>(nimg, reinterpret_cast<const real*>(T),
-                                                                   reinterpret_cast<cplx<real>*>(Y), img_stride,
-                                                                   reinterpret_cast<const cplx<real>*>(roots), bp);
-    return launch_status("rows_op_small");
+    return launch_chained("rows_op_small", kern, dim3((4 * nimg + VT - 1) / VT, N + 1), 256, smem, st, nimg,
+                          reinterpret_cast<const real*>(T), reinterpret_cast<cplx<real>*>(Y), img_stride,
+                          reinterpret_cast<const cplx<real>*>(roots), bp);
 }
 
 template <typename real, int n>
 static int launch_direct(int nimg, const void* T, void* Y, long long img_stride, const void* roots, bool bp, cudaStream_t st) {
     constexpr int N = OpCfg<n>::N, VT = 128 / N;
-    rows_op_direct<real, n><<<dim3((4 * nimg + VT - 1) / VT, N + 1), 256, 0, st>>>(
-        nimg, reinterpret_cast<const real*>(T), reinterpret_cast<cplx<real>*>(Y), img_stride,
-        reinterpret_cast<const cplx<real>*>(roots), bp);
-    return launch_status("rows_op_direct");
+    return launch_chained("rows_op_direct", rows_op_direct<real, n>, dim3((4 * nimg + VT - 1) / VT, N + 1), 256, 0, st, nimg,
+                          reinterpret_cast<const real*>(T), reinterpret_cast<cplx<real>*>(Y), img_stride,
+                          reinterpret_cast<const cplx<real>*>(roots), bp);
 }
 
 template <int n>
@@ -363,10 +370,9 @@ static int launch_tile(int nimg, const void* T, void* Y, long long img_stride, c
     using W = OpTile<n>;
     auto kern = rows_op_tile<n>;
     if (int rc = ensure_smem((const void*)kern, W::smem)) return rc;
-    kern<<<dim3((4 * nimg + W::VT - 1) / W::VT, W::H * 2 + 1), W::THREADS, W::smem, st>>>(
-        nimg, reinterpret_cast<const float*>(T), reinterpret_cast<float2*>(Y), img_stride,
-        reinterpret_cast<const float2*>(roots), bp);
-    return launch_status("rows_op_tile");
+    return launch_chained("rows_op_tile", kern, dim3((4 * nimg + W::VT - 1) / W::VT, W::H * 2 + 1), W::THREADS, W::smem, st,
+                          nimg, reinterpret_cast<const float*>(T), reinterpret_cast<float2*>(Y), img_stride,
+                          reinterpret_cast<const float2*>(roots), bp);
 }
 
 template <int n>

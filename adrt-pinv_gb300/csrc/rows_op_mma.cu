@@ -172,6 +172,10 @@ __global__ void __launch_bounds__(OmCfg<n>::THREADS, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
+    Ts = after_wait(Ts);
+    tinv = after_wait(tinv);
+    roots = after_wait(roots);
 
     // the units of this CTA: frequency and first vector; every role walks the same list
     auto vectors = [&](int k) { return nimg * ((k == 0 || k == N) ? 2 : 4); };
@@ -435,10 +439,9 @@ static int launch_mma(int nimg, const void* Ts, const float* tinv, void* Y, long
     if (int rc = ensure_smem((const void*)kern, W::smem)) return rc;
     const int tiles = (4 * nimg + W::VT - 1) / W::VT;
     const int total = (W::N + 1) * tiles, sms = device_sm_count();
-    kern<<<total < sms ? total : sms, W::THREADS, W::smem, st>>>(
-        nimg, tiles, reinterpret_cast<const __half*>(Ts), tinv, reinterpret_cast<float2*>(Y), img_stride,
-        reinterpret_cast<const float2*>(roots), err);
-    return launch_status("rows_op_mma_kernel");
+    return launch_chained("rows_op_mma_kernel", kern, total < sms ? total : sms, W::THREADS, W::smem, st, nimg, tiles,
+                          reinterpret_cast<const __half*>(Ts), tinv, reinterpret_cast<float2*>(Y), img_stride,
+                          reinterpret_cast<const float2*>(roots), err);
 }
 
 }  // namespace adrt
