@@ -5,10 +5,10 @@
 // that a batch returns, image by image, the iterate the reference's loop returns. All arithmetic is FP64; vector
 // updates are written as separately rounded products and sums (no fused multiply-add), as NumPy evaluates them.
 //
-// Per iteration (CGLS): q = R p (n level passes), <q,q>, alpha; x += alpha p, r -= alpha q; s = R^T r (n passes),
+// Per iteration (CGLS): q = R p (passes of up to four levels), <q,q>, alpha; x += alpha p, r -= alpha q; s = R^T r,
 // <s,s>, the convergence test and beta; p = s + beta p. Inner products are per-image partial sums over fixed
 // segments (one CTA each) summed in a fixed order by one thread per image, so results do not depend on timing.
-// Nothing here waits on the host: the host launches blocks of iterations (or records them in a CUDA graph) and
+// Nothing here waits on the host: the host launches blocks of iterations (directly, or, after many, as a CUDA graph) and
 // reads the per-image active flags between blocks.
 #include "common.cuh"
 #include "launch.h"

@@ -374,7 +374,8 @@ def _rows_apply_f64(X, z_rows, ops, n, counter):
 # sizes whose packed passes run as row operators: above, the operators outgrow what a lane should hold (17 GB at N = 2048);
 # below, the polynomial rows are a few microseconds of latency
 ROW_OPS_MIN, ROW_OPS_MAX = 6, 9
-# batch sizes from which the FP32 row operators run on the tensor cores, by n
+# batch sizes from which the FP32 row operators run on the tensor cores, by n. Measured, us per pass, tensor cores / CUDA cores:
+# N = 128, two images 6.1 / 5.8, four 6.4 / 9.7; N = 256, one 10.1 / 8.7, two 10.9 / 16.3; N = 512, one 62.3 / 62.4, two 65.7 / 143
 ROW_OPS_MMA_BATCH = {7: 4, 8: 2, 9: 2}
 
 

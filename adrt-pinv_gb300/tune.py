@@ -52,8 +52,9 @@ def tile_dimensions(pipe, cfg):
 
 
 def fft_cols_default(N, real):
-    """The offset FFTs' default strip columns per CTA (csrc/fft.cu fft_cols): up to 16 (FP32) / 8 (FP64), at most
-    1024 threads (8 points each along the 2N-long axis), at most N/2, and within 227 KB of shared memory."""
+    """The widest strip of columns per CTA that can be asked of the offset FFTs at every size (csrc/fft.cu fft_cols): up to
+    16 (FP32) / 8 (FP64), at most 1024 threads of 8 points each along the 2N-long axis, at most N/2, and within 227 KB of
+    shared memory. (0 picks the width by size and batch.)"""
     L = 2 * N
     elem = 8 if real == torch.float32 else 16
     tpc = L // 8 if L >= 8 else 1  # threads per column: 8 points each

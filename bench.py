@@ -11,9 +11,11 @@ stencil and FP64 with the others. Metric: whole-job reconstructions per second. 
           an instrumented eager pass before it gives the per-kernel timings, the launch count and `eager`.
   e2e   : the public API FastHybridGpu.apply on pinned host sinograms into a pinned host result every step (H2D + D2H
           inside the timed region; consecutive calls overlap a batch's copy with the previous batch's graph).
-  roofline : the row engine's G_h launch, the dominant kernel, timed live with CUDA events on its stream; algorithmic
-          FLOPs = 2 N^2 per packed row (row operators) or level-rows x 8N (polynomial rows, the reference's cost unit,
-          fastops.py:166); peak = FP32 FMA throughput measured in this run by the library's probe kernel.
+  roofline : the row engine's G_h launch, the dominant kernel, timed live with CUDA events on its stream. Row operators
+          on the tensor cores: the rows read and written once and the matrices read once, against the measured copy
+          bandwidth. On the CUDA cores: algorithmic FLOPs = 2 N^2 per packed row (row operators) or level-rows x 8N
+          (polynomial rows, the reference's cost unit, fastops.py:166), against the FP32 FMA throughput measured in this
+          run by the library's probe kernel.
   cpu_baseline : the reference's C++-engine path (FastHybridCpp semantics: C row kernels + NumPy) timed on this
           host's cores on one image of the same workload, same plan.
   extras (one-GPU runs, --no-extras to skip): preconditioner_ff / _fp32 (the other preconditioner precision),
@@ -415,11 +417,18 @@ def run_ours(args):
             "e2e": {"value": e2e_value, "unit": "recon/s", "h2d_bytes_per_step": int(b_host.numel() * 8),
                     "d2h_bytes_per_step": int(out_host.numel() * 8)}}
     line["roofline_hbm"] = hbm_rooflines(ktimer, pipe)
-    if rows_launch_ms:
+    if rows_launch_ms and operators and pipe.tables.uses_mma(B):
+        # on the tensor cores: the rows read and written once and the FP16 hi / lo matrices read once
+        nbytes = 2 * B * 4 * N * N * 8 + C.load().adrt_rows_operator_split_size(n) * 2
+        gbs, (hbm, src) = nbytes / (rows_launch_ms * 1e-3) / 1e9, measured_hbm_peak()
+        line["roofline"] = {"bound": "hbm", "kernel": "rows_op_mma_kernel (G_h as one real operator per frequency)",
+                            "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm, "peak_source": src,
+                            "bytes_per_launch": nbytes, "flop_per_launch": flops_per_launch, "launch_ms": rows_launch_ms}
+    elif rows_launch_ms:
         achieved = flops_per_launch / (rows_launch_ms * 1e-3) / 1e12
         tr = traffic_per_launch()  # captured at N=256, batch 64; rows scale with the batch
         tr = tr * B / 64 if tr is not None and n == 8 and not operators else None
-        line["roofline"] = {"bound": "fp32", "kernel": "rows_op_tile (G_h as one real operator per frequency)" if operators
+        line["roofline"] = {"bound": "fp32", "kernel": "row operators (G_h as one real operator per frequency)" if operators
                             else "rows_prog_kernel (G_h op list, polynomial rows)",
                             "achieved": achieved, "peak": peak / 1e12, "unit": "TFLOP/s", "frac": achieved * 1e12 / peak,
                             "peak_source": "measured in this run: FP32 FMA probe kernel",
@@ -455,10 +464,10 @@ def run_ours(args):
 
 def adrt_int32_timing(pkg, n, B, steps, torch):
     """The spatial ADRT forward and transpose on B int32 images with values in [0, 255] (bit-exact integer sums),
-    each timed with CUDA events; HBM roofline per call from the bytes every level pass moves (level m reads the
-    level-(m-1) data and writes level m; the transpose mirrors it; the first forward level reads the image, the last
-    transpose level writes it), against the measured copy bandwidth; checked bit-exact against the oracle on one
-    image."""
+    each timed with CUDA events; HBM roofline per call from the bytes its passes of up to four levels move (each reads
+    the data of the level below it and writes its last level's; the first forward pass reads the image; the transpose
+    mirrors it, ending in four quadrant images that one more pass adds), against the measured copy bandwidth; checked
+    bit-exact against the oracle on one image."""
     from oracle import adrt_np as A
 
     N = 1 << n
@@ -478,7 +487,11 @@ def adrt_int32_timing(pkg, n, B, steps, torch):
         C.call("adrt_transpose", C.I32, n, B, C.ptr(b), C.ptr(xt), C.ptr(scratch), st)
 
     lvl = lambda m: 4 * (N + (1 << m) - 1) * N * 4  # bytes of level-m data, four quadrants, int32
-    fwd_bytes = B * (N * N * 4 + sum(lvl(m) for m in range(1, n + 1)) + sum(lvl(m) for m in range(1, n)))
+    np_ = (n + 3) // 4  # passes; the levels between them are written and read
+    mids = [sum(n // np_ + (q < n % np_) for q in range(p + 1)) for p in range(np_ - 1)]
+    img = N * N * 4
+    passes = lvl(n) + sum(2 * lvl(m) for m in mids)
+    nbytes = {"forward": B * (img + passes), "transpose": B * (passes + 2 * 4 * img + img)}
     peak, _ = measured_hbm_peak()
     out = {}
     for name, fn in (("forward", fwd), ("transpose", adj)):
@@ -491,8 +504,8 @@ def adrt_int32_timing(pkg, n, B, steps, torch):
         e1.record()
         torch.cuda.synchronize()
         ms = e0.elapsed_time(e1) / steps
-        gbs = fwd_bytes / (ms * 1e-3) / 1e9
-        out[name] = {"ms": ms, "images_per_s": B / (ms * 1e-3), "bytes_per_call": fwd_bytes, "achieved_gbs": gbs,
+        gbs = nbytes[name] / (ms * 1e-3) / 1e9
+        out[name] = {"ms": ms, "images_per_s": B / (ms * 1e-3), "bytes_per_call": nbytes[name], "achieved_gbs": gbs,
                      "peak_gbs": peak, "frac": gbs / peak}
     x0 = x[0].cpu().numpy()
     out["bit_exact_forward"] = bool(np.array_equal(b[0].cpu().numpy(), A.adrt(n, x0, dtype=np.int64)))
