@@ -203,9 +203,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 // One Gram M = B^* B over levels 1..n (the normal operator's rows): compile-time levels, register-resident rows as in the
 // row programs, out of place or in place. Bounded by memory and by the twiddles (about as many loads and registers as a
-// row itself), so a group keeps them for up to `per` consecutive images of its row, the B-layout levels hold z^t alone
-// (z^(t+1) f = z (z^t f) forward, z^t* (g0 + z* g1) adjoint: two operations more per pair, 30 registers less, no
-// spills), and two CTAs share an SM. Rows cross global memory in contiguous 16-byte pieces: the next row is copied into
+// row itself), so a group keeps them for up to `per` consecutive images of its row, the B-layout levels hold z^t and one
+// z^(t+1) per level (the others are z^t of another slot: 22 registers less than both tables; z z^t would take none, at one
+// more rounding: 1.2e-7 against 1.1e-7 for complex64 rows of 512),
+// and two CTAs share an SM. Rows cross global memory in contiguous 16-byte pieces: the next row is copied into
 // shared memory (asynchronously) while this one is computed, the result staged in the exchange buffer. (Reading and writing
 // the A layout directly, 16 bytes per lane at a stride of R values, kept L1 88% busy with 14% of DRAM.)
 template <typename real, int n>
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
         C tA[R / 2 + 1];
 #pragma unroll
         for (int t = 0; t <= R / 2; ++t) tA[t] = tw.get(key, t);
-        C t0[NB ? NB : 1];
+        C t0[NB ? NB : 1], tn[n > F::BLO ? n - F::BLO : 1];
         if (NB) {
             const int U = tb ? (int)(__brev((unsigned)u) >> (32 - tb)) : 0;
 #pragma unroll
@@ -254,15 +255,20 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
                 const int jb = b - tb;
 #pragma unroll
                 for (int vv = 0; vv < (1 << jb); ++vv) t0[F::offB(b) + vv] = tw.get(key, (U << jb) + brev(vv, jb));
+                tn[b - F::BLO] = tw.get(key, (U + 1) << jb);
             }
         }
+        // z^(t+1) of slot vv of level b: the next exponent's z^t, or the first one of the next lane's
+        auto t1 = [&](int b, int vv) {
+            const int jb = b - tb, r = brev(vv, jb) + 1;
+            return r < (1 << jb) ? t0[F::offB(b) + brev(r & ((1 << jb) - 1), jb)] : tn[b - F::BLO];
+        };
         if (F::ZT) {
             Ln::gsync(gm);  // the previous item's table is no longer read
 #pragma unroll 1
             for (int t = u; t < F::ZT; t += T) zt[t] = tw.get(key, t);
             Ln::gsync(gm);
         }
-        const C z = n > 1 ? tA[1] : tw.get(key, 1), zc = mk<real>(z.x, -z.y);
         const int img1 = img0 + per < J.nimg ? img0 + per : J.nimg;
         for (int img = img0; img < img1; ++img) {
             const size_t at = offset(row, img);
@@ -285,9 +291,10 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
 #pragma unroll
                     for (int j = 0; j < R; ++j) {
                         if (j & (1 << jb)) continue;
-                        const C f0 = v[j], p = cmul(t0[F::offB(b) + (j & ((1 << jb) - 1))], v[j | (1 << jb)]);
-                        v[j] = cadd(f0, p);
-                        v[j | (1 << jb)] = cfma(z, p, f0);
+                        const int vv = j & ((1 << jb) - 1);
+                        const C f0 = v[j], f1 = v[j | (1 << jb)];
+                        v[j] = cfma(t0[F::offB(b) + vv], f1, f0);
+                        v[j | (1 << jb)] = cfma(t1(b, vv), f1, f0);
                     }
                 }
 #pragma unroll
@@ -298,7 +305,8 @@ __global__ void __launch_bounds__(FAST_THREADS, sizeof(real) == 4 ? 2 : 1)
                         if (j & (1 << jb)) continue;
                         const C g0 = v[j], g1 = v[j | (1 << jb)];
                         v[j] = cadd(g0, g1);
-                        v[j | (1 << jb)] = cmulc(t0[F::offB(b) + (j & ((1 << jb) - 1))], cfma(zc, g1, g0));
+                        const int vv = j & ((1 << jb) - 1);
+                        v[j | (1 << jb)] = cdot2c(t0[F::offB(b) + vv], g0, t1(b, vv), g1);
                     }
                 }
                 Ln::toA(v, buf, u, gm);
