@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 // row programs, out of place or in place. Bounded by memory and by the twiddles (about as many loads and registers as a
 // row itself), so a group keeps them for up to `per` consecutive images of its row, the B-layout levels hold z^t and one
 // z^(t+1) per level (the others are z^t of another slot: 22 registers less than both tables; z z^t would take none, at one
-// more rounding: 1.2e-7 against 1.1e-7 for complex64 rows of 512),
-// and two CTAs share an SM. Rows cross global memory in contiguous 16-byte pieces: the next row is copied into
+// more rounding: 1.2e-7 against 1.1e-7 for complex64 rows of 512), and two CTAs share an SM. Rows cross global memory in contiguous 16-byte pieces: the next row is copied into
 // shared memory (asynchronously) while this one is computed, the result staged in the exchange buffer. (Reading and writing
 // the A layout directly, 16 bytes per lane at a stride of R values, kept L1 88% busy with 14% of DRAM.)
 template <typename real, int n>
@@ -597,7 +596,7 @@ static int launch_gram(const adrt_row_job& J, const void* in, const TwSrc<real>&
     if (int rc = ensure_smem((const void*)kern, smem)) return rc;
     const int groups = FAST_THREADS / F::T, slots = (J.grid > 0 ? J.grid : num_sms()) * (sizeof(real) == 4 ? 2 : 1);
     // images per item: an item costs its images and its twiddles (about as much as one more image), and the resident groups
-    // take ceil(items / groups) rounds. N = 256, 24 images: 39.2 us with 2 per item, 33.8 with the 6 this picks
+    // take ceil(items / groups) rounds. N = 256, 24 images: 2 per item take 16% longer than the 6 this picks (35.4 us)
     int per = 1;
     long long best = -1;
     for (int p = 1; p <= 16 && p <= J.nimg; ++p) {
